@@ -62,6 +62,13 @@ int hb_attention_generic(void* out, const void* q, const void* kv, int dtype, co
                          const int32_t* kv_len, int rows, int tokens, int heads, int kv_heads, int head_dim,
                          int pages, int page_size, float scale, int window, const float* sinks, hb_stream stream);
 
+// The same in float32 for head sizes up to 256 that are multiples of 4, out, q and kv on 16-byte boundaries: rows
+// 0 .. n_decode - 1 bring one token each; `tiles` is at least the tiles of 64 queries of the others.
+int hb_attention_f32(float* out, const float* q, const float* kv, const int32_t* block_table, int table_stride,
+                     const int32_t* row_slot, const int32_t* query_start, const int32_t* kv_len, int n_decode, int rows,
+                     int tiles, int heads, int kv_heads, int head_dim, int pages, int page_size, float scale, int window,
+                     const float* sinks, hb_stream stream);
+
 // bfloat16 attention on tensor cores for rows that bring one token each (rows 0 .. rows - 1 of the batch). The keys of
 // a row are cut into `splits` parts that run side by side; with more than one split, `scratch` must hold
 // hb_attention_decode_scratch_floats(...) floats: the parts' partial results, merged by a second kernel.

@@ -482,12 +482,22 @@ class CudaKernels:
             raise KernelError("paged_attention: out and q [tokens, heads, head_dim], kv [pages, 2, kv_heads, page_size, "
                               "head_dim], one dtype")
         fast = q.dtype == torch.bfloat16 and head_dim % 16 == 0 and head_dim <= 256 and self.attention_bf16 == "fast"
-        if not fast:
+        # (sizes, offsets and row lengths that the float32 kernels' 16-byte reads do not fit stay with the generic one)
+        wide = q.dtype == torch.float32 and head_dim % 4 == 0 and head_dim <= 256 \
+            and not (q.data_ptr() | out.data_ptr() | kv.data_ptr()) % 16
+        if not fast and not wide:
             return self._attention_generic(out, q, kv, block_table, rows, scale, window, sinks)
         kv_heads = kv.shape[2]
         common = (self._i32(block_table, "block_table"), block_table.shape[1], self._i32(rows.row_slot, "row_slot"),
                   self._i32(rows.query_start, "query_start"), self._i32(rows.kv_len, "kv_len"))
         sizes = (heads, kv_heads, head_dim, kv.shape[0], kv.shape[3], ctypes.c_float(scale), int(window))
+        if wide:
+            tiles = 0
+            if rows.n_rows > rows.n_decode:              # (without the host's row starts: the most that there can be)
+                tiles = self._query_tiles(rows, 64) if rows.host_query_start is not None or 64 in rows.plan \
+                    else rows.n_tokens // 64 + rows.n_rows
+            return self._call("hb_attention_f32", self._p(out), self._p(q), self._p(kv), *common, rows.n_decode,
+                              rows.n_rows, tiles, *sizes, self._p(sinks))
         if rows.n_decode:
             splits = self.decode_splits(rows.n_decode, heads, kv_heads, rows.max_kv)
             mode = self._decode_mode_of(rows)

@@ -1,14 +1,17 @@
-"""The float32 engine's products where their forms meet: rows around the limit between the kernel for few rows and the
-tiles, k around its segments, tiles that a cluster shares."""
+"""The float32 engine's products and attention where their forms meet: rows around the limit between the kernel for few
+rows and the tiles, k around its segments, tiles that a cluster shares; head sizes around the padded ones, rows of one
+token beside rows of many."""
 import math
 
 import pytest
 import torch
 
-from test_gpu_kernels import rand
+import ref_kernels
+from test_gpu_kernels import on_device, paged_case, rand
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
+REF = ref_kernels.RefKernels()
 
 
 @pytest.fixture(scope="module")
@@ -46,3 +49,56 @@ def test_products_per_head_on_views(K, m, heads, n, k):
     want = torch.einsum("thk,hnk->thn", x[..., :k].double(), w.double())
     assert (wide[..., :n].cpu() - want).abs().max().item() <= 6e-8 * 8 * k
     assert (wide[..., n:] == 7.0).all()
+
+
+# (heads, kv heads, head size, page): padded sizes and their neighbours, groups of 1 to 7, one size of the generic kernel
+GEOMETRIES = [(3, 3, 4, 5), (4, 2, 64, 16), (7, 1, 68, 64), (5, 5, 128, 7), (8, 2, 128, 64), (2, 1, 132, 16), (4, 4, 256, 8), (6, 2, 30, 16)]
+SPEC = [(0, 1), (31, 1), (300, 1), (0, 63), (0, 64), (5, 65), (200, 2), (70, 129)]
+
+
+@pytest.mark.parametrize("geometry", GEOMETRIES)
+@pytest.mark.parametrize("window", [0, 1, 33, 100])
+@pytest.mark.parametrize("sink", [False, True])
+def test_attention_float32(K, geometry, window, sink):
+    heads, kv_heads, head_dim, page = geometry
+    q, kv, table, rows = paged_case(heads, kv_heads, head_dim, page, SPEC, torch.float32, seed=head_dim + window)
+    sinks = rand(heads, seed=9, scale=2.0) if sink else None
+    scale = 1 / math.sqrt(head_dim)
+    want = torch.empty_like(q, dtype=torch.float64)
+    REF.paged_attention(want, q, kv, table, rows, scale, window, sinks)
+    out = torch.full_like(q, float("nan"), device=DEV)
+    K.paged_attention(out, q.to(DEV), kv.to(DEV), table.to(DEV), on_device(rows), scale, window, sinks.to(DEV) if sink else None)
+    assert (out.cpu() - want).abs().max().item() <= 2e-5
+
+
+@pytest.mark.parametrize("window", [0, 50])
+def test_attention_float32_does_not_depend_on_the_cut(K, window):
+    """The last 70 of 230 tokens computed at once, behind 160 and behind 193 others: the same bits for the tokens they share."""
+    heads, kv_heads, head_dim, page = 4, 2, 128, 16
+    q, kv, table, rows = paged_case(heads, kv_heads, head_dim, page, [(160, 70)], torch.float32, seed=3)
+    outs = []
+    for skip in (0, 33):
+        from holon_b200.engine.batch import Rows
+        n = 70 - skip
+        qs = torch.tensor([0, n], dtype=torch.int32)
+        part = Rows(rows.row_slot, qs, rows.kv_len, 1, n, 0, n, 230)
+        out = torch.empty(n, heads, head_dim, device=DEV)
+        K.paged_attention(out, q[skip:].contiguous().to(DEV), kv.to(DEV), table.to(DEV), on_device(part), 0.09, window)
+        outs.append(out)
+    assert torch.equal(outs[0][33:], outs[1])
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_attention_float32_leaves_out_what_is_not_seen(K, bad):
+    """Values of the last key that are no numbers reach the query that sees it and none before it."""
+    heads, kv_heads, head_dim, page = 4, 2, 64, 16
+    q, kv, table, rows = paged_case(heads, kv_heads, head_dim, page, [(20, 90), (0, 40)], torch.float32, seed=5)
+    out = []
+    for plant in (False, True):
+        if plant:
+            kv[table[rows.row_slot[0], 109 // page], 1, :, 109 % page] = bad
+        o = torch.empty_like(q, device=DEV)
+        K.paged_attention(o, q.to(DEV), kv.to(DEV), table.to(DEV), on_device(rows), 0.125, 0)
+        out.append(o)
+    assert torch.equal(out[0][:89], out[1][:89]) and torch.equal(out[0][90:], out[1][90:])
+    assert not out[1][89].isfinite().any()
