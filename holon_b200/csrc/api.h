@@ -162,6 +162,15 @@ int hb_latent_attention_generic(void* out, const void* qa, const void* cache, in
                                 int table_stride, const int32_t* row_slot, const int32_t* query_start,
                                 const int32_t* kv_len, int rows, int tokens, int heads, int rank, int rot, int pages,
                                 int page_size, float scale, int window, const float* sinks, hb_stream stream);
+// bfloat16 prompt portions on tcgen05 tensor cores: rows row0 .. rows - 1, which bring `portion` of the step's `tokens`
+// tokens; for sizes that hb_latent_tcgen05_takes answers with 1 and a positive scale. hb_latent_tcgen05_status
+// synchronises the device and returns (and clears) the kernel's bounded-wait status word.
+int hb_latent_attention_tcgen05(void* out, const void* qa, const void* cache, const int32_t* block_table, int table_stride,
+                                const int32_t* row_slot, const int32_t* query_start, const int32_t* kv_len, int row0,
+                                int rows, int tokens, int portion, int heads, int rank, int rot, int pages, int page_size,
+                                float scale, int window, const float* sinks, hb_stream stream);
+int hb_latent_tcgen05_takes(int heads, int rank, int rot, int pages, int page_size);
+int hb_latent_tcgen05_status(unsigned int* status);
 
 // The same on tensor cores in bfloat16 (csrc/latent_bf16.cu) for rows row0 .. row1 - 1 of the batch, which bring `tokens`
 // tokens in all, the first of them token `first_token` of the step; rank and rot multiples of 16, rank up to 512.

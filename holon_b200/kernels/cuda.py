@@ -842,7 +842,8 @@ class CudaKernels:
         up their barrier and flags are put back to zero, so that the next launch starts clean."""
         out = 0
         for name in ("hb_gemm_tcgen05_status", "hb_gemm_tcgen05_pair_status", "hb_attention_tcgen05_status",
-                     "hb_gemm_chain_status", "hb_gemm_tickets_status", "hb_gemm_mid_status", "hb_experts_tcgen05_status", "hb_attention_maps_status"):
+                     "hb_gemm_chain_status", "hb_gemm_tickets_status", "hb_gemm_mid_status", "hb_experts_tcgen05_status", "hb_attention_maps_status",
+                     "hb_latent_tcgen05_status"):
             status = ctypes.c_uint(0)
             if getattr(self.lib, name)(ctypes.byref(status)):
                 raise KernelError(self.lib.hb_last_error().decode())
@@ -977,8 +978,20 @@ class CudaKernels:
             self._call("hb_latent_attention_bf16", self._p(out), self._p(scratch), self._p(qa), self._p(cache), *common,
                        0, ones, 0, ones, *sizes, splits, self._p(sinks))
         if rows.n_rows > ones:
+            # prompt portions: on tcgen05 wherever it takes the sizes (2,048 tokens of 16 heads, rank 512 + 64: 730 us on
+            # mma.sync, 234 us on tcgen05; a tile step of either costs the same for few queries as for many)
+            if self.prefill_attention == "tcgen05" and scale > 0 and (t - ones) * heads // 128 + rows.n_rows <= 65535 \
+                    and self._latent_tcgen05_takes(heads, rank, rot, cache.shape[0], cache.shape[1]):
+                return self._call("hb_latent_attention_tcgen05", self._p(out), self._p(qa), self._p(cache), *common, ones,
+                                  rows.n_rows, t, t - ones, *sizes, self._p(sinks))
             self._call("hb_latent_attention_bf16", self._p(out), None, self._p(qa), self._p(cache), *common, ones,
                        rows.n_rows, ones, t - ones, *sizes, 1, self._p(sinks))
+
+    def _latent_tcgen05_takes(self, *sizes: int) -> bool:
+        key = ("latent", *sizes)
+        if key not in self._splits:
+            self._splits[key] = int(self.lib.hb_latent_tcgen05_takes(*map(int, sizes)))
+        return bool(self._splits[key])
 
     def latent_splits(self, rows: int, heads: int, rank: int, max_kv: int) -> int:
         """Parts the keys of one-token rows are cut into for the latent attention kernel: enough that two CTAs an SM
