@@ -460,6 +460,11 @@ size_t hb_state_space_prompt_scratch_floats(int tiles, int heads, int groups, in
 int hb_state_space_prompt(float* y, const float* cb, const float* x, const float* dt, const float* rate_log, const float* skip,
                           float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0, int rows,
                           int tiles, int heads, int groups, int n, int vdim, hb_stream stream);
+// hb_recurrent_scan for rows row0 .. rows - 1 in the same chunks, with one decay per head (head_decay [heads]) or per head and token
+// (token_decay [tokens, heads]), without beta, rate, take and skip; tiles and scratch as above (groups = kv_heads, n = dim).
+int hb_recurrent_chunks(float* out, const float* qk, const float* v, const float* head_decay, const float* token_decay, float* state,
+                        float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0, int rows, int tiles, int heads,
+                        int kv_heads, int dim, int vdim, hb_stream stream);
 
 // ---- the matrix memory with exponential gates (csrc/mlstm.cu): the kernels around hb_recurrent_scan with token_decay.
 // pre [tokens, ld] 32-bit: the input gate's pre-activations of the heads, then the forget gate's; bias [2 heads] likewise.

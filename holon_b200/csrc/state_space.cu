@@ -1,10 +1,15 @@
-// The state-space recurrence for rows of several tokens, in chunks of 64 (the form of Dao and Gu, Transformers are SSMs: Generalized
+// The state-space recurrence, and those of recurrent.cu whose decay is one number per head or per head and token and that have no
+// delta rule, for rows of several tokens, in chunks of 64 (the form of Dao and Gu, Transformers are SSMs: Generalized
 // Models and Efficient Algorithms Through Structured State Space Duality), everything in 32-bit on CUDA cores:
 //     S_t = g_t S_(t-1) + dt_t B_t x_t^T,  y_t = S_t^T C_t + skip x_t,  g_t = exp(-exp(rate_log) dt_t)
 // With L_i the sum of the logarithms of g over a chunk's tokens up to i (kept as a pair of float32 whose sum is exact to double
 // precision: what the weights need are differences of such sums), a chunk with the state S_in before it gives
 //     y_i = sum_(j <= i) (C_i . B_j) exp(L_i - L_j) dt_j x_j + exp(L_i) S_in^T C_i + skip x_i
 //     S_out = exp(L_last) S_in + sum_j exp(L_last - L_j) dt_j B_j x_j^T.
+// With a decay given as itself (FIXED: one per head, TOKEN: per head and token) dt = 1, there is no skip, and L sums the logarithms of
+// its magnitude in double precision, a zero counting as -10^4 (below which an exponential is zero); signs are kept beside it. A value that is no finite
+// number reaches the outputs from its token on and no earlier one.
+// 2,048 tokens of 16 heads of 128 by 128 with a decay per head: 154 us in chunks, 422 us token by token (recurrent.cu).
 // Four kernels: the chunks' products C_i . B_j, per group; the chunks' own contributions to the state, per head; the walk over a
 // row's chunks, an element of the state a thread, which leaves every chunk's S_in behind and writes the row's state back; the
 // chunks' outputs, per head. Only the third is sequential, one multiply-add a chunk. Blocks find their (row, chunk) in the step's
@@ -35,20 +40,29 @@ __device__ __forceinline__ Chunk find_chunk(const int32_t* __restrict__ query_st
 // permuted by k / 4, so that stores of four k's of one i by eight neighbouring lanes, and of four i's by four, hit different banks.
 __device__ __forceinline__ int group_at(int k, int g) { return k * (SS_T / 4) + (g ^ ((k >> 2) & 7)); }
 
-// acc += a^T b over a slice.
-__device__ __forceinline__ void tile_step(float (&acc)[8][4], const float* a, const float* b, int depth) {
+// total += a^T b over a slice, 16 steps of k to a sum of their own: one sum over all steps loses twice as much (an output's error
+// against 64 bits 2.5e-7 in place of 1.3e-7, the token-by-token scan's 1.0 to 2.1e-7 for decays of 0.875 to 0.984).
+__device__ __forceinline__ void tile_step(float (&total)[8][4], const float* a, const float* b, int depth) {
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const float4* a4 = (const float4*)a;
     const float4* b4 = (const float4*)b;
+    for (int k0 = 0; k0 < depth; k0 += 16) {
+        float acc[8][4] = {};
+        const int end = min(depth, k0 + 16);
 #pragma unroll 8
-    for (int k = 0; k < depth; ++k) {
-        const float4 r0 = a4[group_at(k, ty * 2)], r1 = a4[group_at(k, ty * 2 + 1)], c = b4[group_at(k, tx)];
-        const float r[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+        for (int k = k0; k < end; ++k) {
+            const float4 r0 = a4[group_at(k, ty * 2)], r1 = a4[group_at(k, ty * 2 + 1)], c = b4[group_at(k, tx)];
+            const float r[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            acc[i][0] = fmaf(r[i], c.x, acc[i][0]); acc[i][1] = fmaf(r[i], c.y, acc[i][1]);
-            acc[i][2] = fmaf(r[i], c.z, acc[i][2]); acc[i][3] = fmaf(r[i], c.w, acc[i][3]);
+            for (int i = 0; i < 8; ++i) {
+                acc[i][0] = fmaf(r[i], c.x, acc[i][0]); acc[i][1] = fmaf(r[i], c.y, acc[i][1]);
+                acc[i][2] = fmaf(r[i], c.z, acc[i][2]); acc[i][3] = fmaf(r[i], c.w, acc[i][3]);
+            }
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) total[i][j] += acc[i][j];
     }
 }
 
@@ -86,14 +100,38 @@ __device__ __forceinline__ void store_across(float* a, const Quads& q) {
 }
 __device__ __forceinline__ void scale_quad(float4& v, float f) { v.x *= f; v.y *= f; v.z *= f; v.w *= f; }
 
-// L_i of a chunk's tokens for one head, by warp 0: hi + lo in two floats; tokens past the chunk repeat the last.
-__device__ __forceinline__ void log_decays(float* hi, float* lo, float* steps, const float* __restrict__ dt, const Chunk& c, int heads,
-                                           int h, float rate) {
+enum Form { STATE_SPACE, FIXED, TOKEN };                   // where decays come from: dt and rate_log; head_decay in rate_log's place; token_decay in dt's
+
+// L_i of a chunk's tokens for one head, by warp 0: hi + lo in two floats; tokens past the chunk repeat the last. sign: of the decays'
+// product up to i (not for STATE_SPACE).
+template <int FORM>
+__device__ __forceinline__ void log_decays(float* hi, float* lo, float* steps, float* sign, const float* __restrict__ dt, const Chunk& c,
+                                           int heads, int h, const float* __restrict__ rate_log) {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
-        const float d0 = 2 * lane < c.n ? dt[(size_t)(c.t0 + 2 * lane) * heads + h] : 0.f;
-        const float d1 = 2 * lane + 1 < c.n ? dt[(size_t)(c.t0 + 2 * lane + 1) * heads + h] : 0.f;
-        const double a0 = -(double)rate * d0, a1 = -(double)rate * d1;
+        const bool in0 = 2 * lane < c.n, in1 = 2 * lane + 1 < c.n;
+        float d0 = in0 ? 1.f : 0.f, d1 = in1 ? 1.f : 0.f;
+        if (FORM != FIXED) {
+            d0 = in0 ? dt[(size_t)(c.t0 + 2 * lane) * heads + h] : 0.f;
+            d1 = in1 ? dt[(size_t)(c.t0 + 2 * lane + 1) * heads + h] : 0.f;
+        }
+        double a0, a1;
+        if (FORM == STATE_SPACE) {
+            const float rate = expf(rate_log[h]);
+            a0 = -(double)rate * d0; a1 = -(double)rate * d1;
+        } else {
+            const float g0 = FORM == FIXED ? rate_log[h] : d0, g1 = FORM == FIXED ? rate_log[h] : d1;
+            auto logarithm = [](float g) -> double {
+                const double a = g == 0.f ? -1e4 : log(fabs((double)g));
+                return a > 1e4 ? 1e4 : a;
+            };
+            a0 = in0 ? logarithm(g0) : 0.0; a1 = in1 ? logarithm(g1) : 0.0;
+            const unsigned n0 = __ballot_sync(0xffffffffu, in0 && g0 < 0.f), n1 = __ballot_sync(0xffffffffu, in1 && g1 < 0.f);
+            const unsigned before = (1u << lane) - 1, here = __popc(n0 & before) + __popc(n1 & before) + ((n0 >> lane) & 1);
+            sign[2 * lane] = here & 1 ? -1.f : 1.f;
+            sign[2 * lane + 1] = (here + ((n1 >> lane) & 1)) & 1 ? -1.f : 1.f;
+            d0 = in0 ? 1.f : 0.f; d1 = in1 ? 1.f : 0.f;
+        }
         double s = a0 + a1;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -108,7 +146,7 @@ __device__ __forceinline__ void log_decays(float* hi, float* lo, float* steps, c
 }
 
 // ---- products[tile][group][i][j] = C_i . B_j, [64][64] each. grid (tiles, groups)
-__global__ void __launch_bounds__(SS_THREADS, 4) ss_products_kernel(float* __restrict__ products, const float* __restrict__ cb,
+__global__ void __launch_bounds__(SS_THREADS, 3) ss_products_kernel(float* __restrict__ products, const float* __restrict__ cb,
                                                                  const int32_t* __restrict__ query_start, int row0, int rows, int groups, int n) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
     const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
@@ -140,12 +178,13 @@ __global__ void __launch_bounds__(SS_THREADS, 4) ss_products_kernel(float* __res
 
 // ---- own[tile][head][p][n] = sum_j exp(L_last - L_j) dt_j x_j[p] B_j[n]; last[tile][head] = exp(L_last). grid (tiles, heads, tiles of
 // p times tiles of n)
-__global__ void __launch_bounds__(SS_THREADS, 4) ss_own_kernel(float* __restrict__ own, float* __restrict__ last, const float* __restrict__ cb,
+template <int FORM>
+__global__ void __launch_bounds__(SS_THREADS, 3) ss_own_kernel(float* __restrict__ own, float* __restrict__ last, const float* __restrict__ cb,
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const int32_t* __restrict__ query_start,
                                                             int row0, int rows, int heads, int groups, int n, int vdim, int n_tiles) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
-    __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q];
+    __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q], sign[FORM == STATE_SPACE ? 1 : SS_Q];
     const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
     if (c.row < 0) return;
     const int h = blockIdx.y, g = h / (heads / groups);
@@ -157,12 +196,14 @@ __global__ void __launch_bounds__(SS_THREADS, 4) ss_own_kernel(float* __restrict
     const bool vx = (vdim & 3) == 0, vb = (n & 3) == 0;
     fetch_across(qa, xp, xs, vdim - p0, c.n, vx);                   // (on its way while the decays are added up)
     fetch_across(qb, bp, bs, n - n0, c.n, vb);
-    log_decays(hi, lo, steps, dt, c, heads, h, expf(rate_log[h]));
+    log_decays<FORM>(hi, lo, steps, sign, dt, c, heads, h, rate_log);
     __syncthreads();
     if (threadIdx.x < SS_Q) {
         const int j = threadIdx.x;
-        w[j] = expf((hi[SS_Q - 1] - hi[j]) + (lo[SS_Q - 1] - lo[j])) * steps[j];
-        if (j == 0 && blockIdx.z == 0) last[(size_t)blockIdx.x * heads + h] = expf(hi[SS_Q - 1] + lo[SS_Q - 1]);
+        float f = 1.f, all = 1.f;
+        if (FORM != STATE_SPACE) { all = sign[SS_Q - 1]; f = all * sign[j]; }
+        w[j] = f * expf((hi[SS_Q - 1] - hi[j]) + (lo[SS_Q - 1] - lo[j])) * steps[j];
+        if (j == 0 && blockIdx.z == 0) last[(size_t)blockIdx.x * heads + h] = all * expf(hi[SS_Q - 1] + lo[SS_Q - 1]);
     }
     __syncthreads();
     float acc[8][4] = {};
@@ -230,14 +271,16 @@ __global__ void ss_walk_kernel(float* __restrict__ own, const float* __restrict_
 }
 
 // ---- y_i[p] of a chunk: the products' part over its own tokens, the state's part over n, the skip. grid (tiles, heads, tiles of p)
-__global__ void __launch_bounds__(SS_THREADS, 4) ss_out_kernel(float* __restrict__ y, const float* __restrict__ products,
+template <int FORM>
+__global__ void __launch_bounds__(SS_THREADS, 3) ss_out_kernel(float* __restrict__ y, const float* __restrict__ products,
                                                             const float* __restrict__ before, const float* __restrict__ cb,
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const float* __restrict__ skip,
                                                             const int32_t* __restrict__ query_start, int row0, int rows, int heads,
                                                             int groups, int n, int vdim) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
-    __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q];
+    __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q], sign[FORM == STATE_SPACE ? 1 : SS_Q];
+    __shared__ int bad[SS_T];                                       // per column: the first token whose value is no finite number
     const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
     if (c.row < 0) return;
     const int h = blockIdx.y, g = h / (heads / groups), p0 = (int)blockIdx.z * SS_T;
@@ -261,9 +304,13 @@ __global__ void __launch_bounds__(SS_THREADS, 4) ss_out_kernel(float* __restrict
         }
     };
     fetch(0);                                                       // (on its way while the decays are added up)
-    log_decays(hi, lo, steps, dt, c, heads, h, expf(rate_log[h]));
+    log_decays<FORM>(hi, lo, steps, sign, dt, c, heads, h, rate_log);
     __syncthreads();
-    if (threadIdx.x < SS_Q) w[threadIdx.x] = expf(hi[threadIdx.x] + lo[threadIdx.x]);
+    if (threadIdx.x < SS_Q) {
+        const int i = threadIdx.x;
+        w[i] = (FORM == STATE_SPACE ? 1.f : sign[i]) * expf(hi[i] + lo[i]);
+        bad[i] = SS_Q;
+    }
     __syncthreads();
     float acc[8][4] = {};
     for (int s = 0; s < slices; ++s) {
@@ -273,9 +320,20 @@ __global__ void __launch_bounds__(SS_THREADS, 4) ss_out_kernel(float* __restrict
             for (int r = 0; r < 4; ++r) {
                 const int row = ((int)threadIdx.x >> 3) + 16 * r;
                 const float hr = hi[row], lr = lo[row];
-                auto weight = [&](int jj, float v) -> float { return jj <= row && jj < c.n ? v * expf((hr - hi[jj]) + (lr - lo[jj])) * steps[jj] : 0.f; };
+                auto weight = [&](int jj, float v) -> float {
+                    if (jj > row || jj >= c.n) return 0.f;
+                    const float f = FORM == STATE_SPACE ? v : v * (sign[row] * sign[jj]);
+                    return f * expf((hr - hi[jj]) + (lr - lo[jj])) * steps[jj];
+                };
                 qa.v[r].x = weight(j, qa.v[r].x); qa.v[r].y = weight(j + 1, qa.v[r].y);
                 qa.v[r].z = weight(j + 2, qa.v[r].z); qa.v[r].w = weight(j + 3, qa.v[r].w);
+                float* x4 = &qb.v[r].x;                             // (a weight of zero would make a NaN of an infinity in an earlier row)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (!isfinite(x4[e])) {
+                        atomicMin(&bad[((int)threadIdx.x & 15) * 4 + e], s * SS_K + ((int)threadIdx.x >> 4) + 8 * r);
+                        x4[e] = 0.f;
+                    }
             }
         } else {
 #pragma unroll
@@ -290,14 +348,18 @@ __global__ void __launch_bounds__(SS_THREADS, 4) ss_out_kernel(float* __restrict
         __syncthreads();
     }
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const float d = skip[h];
+    const float d = skip ? skip[h] : 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int r = ty * 8 + i;
         if (r >= c.n) break;
         const size_t at = ((size_t)(c.t0 + r) * heads + h) * vdim + p0 + tx * 4;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) if (p0 + tx * 4 + k < vdim) y[at + k] = fmaf(d, x[at + k], acc[i][k]);
+        for (int k = 0; k < 4; ++k)
+            if (p0 + tx * 4 + k < vdim) {
+                const float v = r >= bad[tx * 4 + k] ? NAN : acc[i][k];
+                y[at + k] = skip ? fmaf(d, x[at + k], v) : v;
+            }
     }
 }
 
@@ -305,14 +367,15 @@ extern "C" size_t hb_state_space_prompt_scratch_floats(int tiles, int heads, int
     return (size_t)tiles * ((size_t)heads * vdim * n + (size_t)groups * SS_Q * SS_Q + heads);
 }
 
-extern "C" int hb_state_space_prompt(float* y, const float* cb, const float* x, const float* dt, const float* rate_log, const float* skip,
+template <int FORM>
+static int run_chunks(const char* what, float* y, const float* cb, const float* x, const float* dt, const float* rate_log, const float* skip,
                                      float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
                                      int rows, int tiles, int heads, int groups, int n, int vdim, hb_stream stream) {
     if (rows <= row0 || tiles == 0) return 0;
-    if (groups < 1 || heads % groups || n < 1 || vdim < 1) HB_REFUSE("state_space_prompt: %d heads of %d, %d groups of %d", heads, vdim, groups, n);
-    if (!scratch || ((uintptr_t)scratch & 15) || ((uintptr_t)state & 15)) HB_REFUSE("state_space_prompt: scratch and state must lie on 16-byte boundaries");
+    if (groups < 1 || heads % groups || n < 1 || vdim < 1) HB_REFUSE("%s: %d heads of %d, %d groups of %d", what, heads, vdim, groups, n);
+    if (!scratch || ((uintptr_t)scratch & 15) || ((uintptr_t)state & 15)) HB_REFUSE("%s: scratch and state must lie on 16-byte boundaries", what);
     const int p_tiles = (vdim + SS_T - 1) / SS_T, n_tiles = (n + SS_T - 1) / SS_T;
-    if (heads > 65535 || (long)p_tiles * n_tiles > 65535) HB_REFUSE("state_space_prompt: %d heads of %d x %d", heads, vdim, n);
+    if (heads > 65535 || (long)p_tiles * n_tiles > 65535) HB_REFUSE("%s: %d heads of %d x %d", what, heads, vdim, n);
     const int size = vdim * n;
     float* products = scratch;                                     // [tiles][groups][64][64]
     float* own = products + (size_t)tiles * groups * SS_Q * SS_Q;  // [tiles][heads][vdim][n]
@@ -320,17 +383,38 @@ extern "C" int hb_state_space_prompt(float* y, const float* cb, const float* x, 
     cudaStream_t s = (cudaStream_t)stream;
     ss_products_kernel<<<dim3(tiles, groups), SS_THREADS, 0, s>>>(products, cb, query_start, row0, rows, groups, n);
     HB_LAUNCH_CHECK("state_space_products");
-    ss_own_kernel<<<dim3(tiles, heads, p_tiles * n_tiles), SS_THREADS, 0, s>>>(own, last, cb, x, dt, rate_log, query_start, row0, rows, heads,
+    ss_own_kernel<FORM><<<dim3(tiles, heads, p_tiles * n_tiles), SS_THREADS, 0, s>>>(own, last, cb, x, dt, rate_log, query_start, row0, rows, heads,
                                                                                groups, n, vdim, n_tiles);
     HB_LAUNCH_CHECK("state_space_own");
     const bool vec = size % 4 == 0;
     const int elements = vec ? size / 4 : size, slices = (elements + 127) / 128;
-    if (slices > 65535) HB_REFUSE("state_space_prompt: states of %d numbers", size);
+    if (slices > 65535) HB_REFUSE("%s: states of %d numbers", what, size);
     if (vec) ss_walk_kernel<true><<<dim3(rows - row0, heads, slices), 128, 0, s>>>(own, last, state, query_start, row_slot, row0, heads, size);
     else ss_walk_kernel<false><<<dim3(rows - row0, heads, slices), 128, 0, s>>>(own, last, state, query_start, row_slot, row0, heads, size);
     HB_LAUNCH_CHECK("state_space_walk");
-    ss_out_kernel<<<dim3(tiles, heads, p_tiles), SS_THREADS, 0, s>>>(y, products, own, cb, x, dt, rate_log, skip, query_start, row0, rows, heads,
+    ss_out_kernel<FORM><<<dim3(tiles, heads, p_tiles), SS_THREADS, 0, s>>>(y, products, own, cb, x, dt, rate_log, skip, query_start, row0, rows, heads,
                                                                      groups, n, vdim);
     HB_LAUNCH_CHECK("state_space_out");
     return 0;
+}
+
+extern "C" int hb_state_space_prompt(float* y, const float* cb, const float* x, const float* dt, const float* rate_log, const float* skip,
+                                     float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
+                                     int rows, int tiles, int heads, int groups, int n, int vdim, hb_stream stream) {
+    return run_chunks<STATE_SPACE>("state_space_prompt", y, cb, x, dt, rate_log, skip, state, scratch, query_start, row_slot, row0, rows, tiles,
+                                   heads, groups, n, vdim, stream);
+}
+
+// hb_recurrent_scan for rows row0 .. rows - 1 with one decay per head (head_decay) or per head and token (token_decay) and no delta rule:
+// qk [tokens, 2, kv_heads, dim]. tiles and scratch as above, with kv_heads and dim in the places of groups and n.
+extern "C" int hb_recurrent_chunks(float* out, const float* qk, const float* v, const float* head_decay, const float* token_decay,
+                                   float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
+                                   int rows, int tiles, int heads, int kv_heads, int dim, int vdim, hb_stream stream) {
+    if ((head_decay != nullptr) == (token_decay != nullptr)) HB_REFUSE("recurrent_chunks: one decay per head, or one per head and token");
+    if ((uintptr_t)qk & 15) HB_REFUSE("recurrent_chunks: qk must lie on a 16-byte boundary");
+    if (token_decay)
+        return run_chunks<TOKEN>("recurrent_chunks", out, qk, v, token_decay, nullptr, nullptr, state, scratch, query_start, row_slot, row0,
+                                 rows, tiles, heads, kv_heads, dim, vdim, stream);
+    return run_chunks<FIXED>("recurrent_chunks", out, qk, v, nullptr, head_decay, nullptr, state, scratch, query_start, row_slot, row0, rows,
+                             tiles, heads, kv_heads, dim, vdim, stream);
 }

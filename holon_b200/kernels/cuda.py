@@ -177,6 +177,7 @@ class CudaKernels:
         # Two mixers that read the same input run as two branches of a step's graph (HOLON_B200_BRANCHES=0: one after the other).
         self.branches = os.environ.get("HOLON_B200_BRANCHES", "1") != "0"
         self._side = None
+        self.scan_parts = True                # rows of many tokens through csrc/state_space.cu (tests: False)
         # One word of page-locked host memory that a kernel's bounded wait writes when it gives up (csrc/status.cu)
         word = ctypes.POINTER(ctypes.c_uint)()
         with torch.cuda.device(self.device):
@@ -1197,6 +1198,10 @@ class CudaKernels:
             if t is not None and t.dtype != torch.float32:
                 raise KernelError(f"{what}: 32-bit tensors expected, got {t.dtype}")
 
+    # Tokens a row on average from which the scan goes in chunks of 64 (four launches: 16 heads of 128 by 128, one row of 128 tokens
+    # 33 us token by token and 43 in chunks, 256 tokens 60 and 49, 2,048 tokens 422 and 154; eight rows of 100 96 and 106).
+    CHUNK_TOKENS = 192
+
     def recurrent_scan(self, out, qk, v, decay, head_decay, beta, state, rows, token_decay=None, rate=None, take=None,
                        skip=None) -> None:
         """The token-by-token update of a matrix state per head (csrc/api.h: hb_recurrent_scan). `rate` (float32 [tokens,
@@ -1216,11 +1221,23 @@ class CudaKernels:
                 or (take is not None and take.shape != (t, heads)) or (skip is not None and skip.shape != (heads,)):
             raise KernelError("recurrent_scan: qk [tokens, 2, kv_heads, dim], v and out [tokens, heads, vdim], state "
                               "[slots, heads, vdim, dim], decay [tokens, heads, dim] or head_decay [heads], beta [tokens, heads]")
-        self._call("hb_recurrent_scan", self._p(out), self._p(qk), self._p(v), self._p(decay), self._p(head_decay),
-                   self._p(token_decay), self._p(beta), self._p(rate), self._p(take), self._p(skip), self._p(state),
-                   self._i32(rows.query_start, "query_start"),
-                   self._i32(rows.row_slot, "row_slot"), rows.n_rows, heads, kv_heads, dim, vdim,
-                   int(getattr(rows, "max_q", 0) or 0))
+        # Rows of many tokens: in chunks of 64 where the decay is one number per head. What the launches depend on are counts of
+        # rows and tokens, so that they can be captured.
+        scanned, ones, portions = rows.n_rows, rows.n_decode, rows.n_rows - rows.n_decode
+        more = t - ones
+        ends = (self._i32(rows.query_start, "query_start"), self._i32(rows.row_slot, "row_slot"), ones, rows.n_rows)
+        if self.scan_parts and portions and take is None and decay is None and beta is None and more >= self.CHUNK_TOKENS * portions \
+                and not (qk.data_ptr() | state.data_ptr()) % 16:
+            scanned, tiles = ones, more // 64 + portions                               # (the most that any cut into those rows has)
+            scratch = torch.empty(tiles * (heads * vdim * dim + kv_heads * 64 * 64 + heads), dtype=torch.float32, device=self.device)
+            self._call("hb_recurrent_chunks", self._p(out), self._p(qk), self._p(v), self._p(head_decay), self._p(token_decay),
+                       self._p(state), self._p(scratch), *ends, tiles, heads, kv_heads, dim, vdim)
+        if scanned:
+            self._call("hb_recurrent_scan", self._p(out), self._p(qk), self._p(v), self._p(decay), self._p(head_decay),
+                       self._p(token_decay), self._p(beta), self._p(rate), self._p(take), self._p(skip), self._p(state),
+                       self._i32(rows.query_start, "query_start"),
+                       self._i32(rows.row_slot, "row_slot"), scanned, heads, kv_heads, dim, vdim,
+                       int(getattr(rows, "max_q", 0) or 0))
 
     def delta_prepare(self, qk, v, beta, decay, gate, first, conv, conv_state, low2, dt_bias, rate_log, rows, q_scale,
                       unit_eps, carry=False) -> None:

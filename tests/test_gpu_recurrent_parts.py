@@ -1,0 +1,107 @@
+"""The recurrences in parts of several tokens against the token-by-token formula in 64 bits and against the token-by-token
+kernel: rows whose last part is short, one-token rows beside them, every form of decay, decays of zero and below, value sizes
+that leave a tile of columns half empty."""
+import pytest
+import torch
+
+from holon_b200.engine.batch import Rows
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+FORMS = ["fixed", "token"]
+
+
+@pytest.fixture(scope="module")
+def K():
+    from holon_b200.kernels import load_kernels
+    return load_kernels(torch.device(DEV))
+
+
+def plain(qk, v, state, counts, slots, decay, beta, rate):
+    """decay [tokens, heads, dim] in 64 bits; state [slots, heads, vdim, dim]."""
+    qk, v, state, decay = (x.double() for x in (qk, v, state, decay))
+    group, out, t = v.shape[1] // qk.shape[2], torch.empty_like(v), 0
+    for n, slot in zip(counts, slots):
+        s = state[slot].transpose(1, 2).clone()                                       # [head, key, value]
+        for t in range(t, t + n):
+            q, k = (qk[t, i].repeat_interleave(group, 0) for i in (0, 1))
+            a = torch.einsum("hkv,hk->hv", s if rate is not None else s * decay[t][..., None], k)
+            u = v[t] if beta is None else beta[t].double()[:, None] * (v[t] - a)
+            s = s * decay[t][..., None] + k[..., None] * u[:, None]
+            if rate is not None:
+                s = s - (rate[t].double() * k)[..., None] * a[:, None]
+            out[t] = torch.einsum("hkv,hk->hv", s, q)
+        t += 1
+        state[slot] = s.transpose(1, 2)
+    return out, state
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 64, 64), (3, 3, 128, 129), (5, 5, 256, 20), (6, 2, 128, 128), (2, 1, 64, 7),
+                                                     (40, 8, 64, 70), (3, 1, 36, 10)])
+def test_against_the_formula(K, form, heads, kv_heads, dim, vdim, monkeypatch):
+    for name in ("CHUNK_TOKENS", "BLOCK_TOKENS"):                                      # (short rows too)
+        monkeypatch.setattr(type(K), name, 2, raising=False)
+    g = torch.Generator().manual_seed(dim + vdim)
+    counts, slots = [1, 1, 8, 3, 200, 9, 7, 64, 65, 127], [6, 0, 3, 1, 2, 8, 5, 7, 9, 10]
+    t = sum(counts)
+    qk = torch.nn.functional.normalize(torch.randn(t, 2, kv_heads, dim, generator=g), dim=-1)
+    v, state = torch.randn(t, heads, vdim, generator=g), torch.randn(11, heads, vdim, dim, generator=g) * 0.2
+    decay = 1 - torch.rand(t, heads, dim, generator=g) ** 3 * 0.3
+    decay[5:40:7] = 0.0                                                               # what went before is gone
+    decay[60:64, :, ::3] = 1e-30
+    decay[70:74] *= -1
+    beta = torch.rand(t, heads, generator=g) if "delta" in form else None
+    rate = torch.rand(t, heads, dim, generator=g) if form == "general" else None
+    head = 1 - 2.0 ** -(3 + torch.arange(heads, dtype=torch.float32)) if "fixed" in form else None
+    if head is not None:
+        head[-1] *= -1
+    token = decay[:, :, 0].contiguous() if form == "token" else None
+    if head is not None:
+        decay = head[None, :, None].expand(t, heads, dim)
+    if token is not None:
+        decay = token[:, :, None].expand(t, heads, dim)
+    want, want_state = plain(qk, v, state, counts, slots, decay, beta, rate)
+    starts = torch.tensor([0] + counts, dtype=torch.int32).cumsum(0).to(torch.int32)
+    rows = Rows(torch.tensor(slots, dtype=torch.int32, device=DEV), starts.to(DEV), starts[1:].to(DEV), len(counts), t, 2, max(counts), 0)
+    dev = lambda x: None if x is None else x.contiguous().to(DEV)                     # noqa: E731
+    errors = {}
+    for parts in (False, True):
+        monkeypatch.setattr(K, "scan_parts", parts)
+        s, out = dev(state), torch.full((t, heads, vdim), float("nan"), device=DEV)
+        before = K.launches
+        K.recurrent_scan(out, dev(qk), dev(v), dev(decay) if head is None and token is None else None, dev(head), dev(beta), s, rows,
+                         token_decay=dev(token), rate=dev(rate))
+        assert K.launches - before == (2 if parts and not ("delta" in form or form == "general") or parts and dim in (64, 128, 256) else 1)
+        errors[parts] = [float(torch.linalg.norm(x.cpu() - w) / torch.linalg.norm(w)) for x, w in ((out, want), (s, want_state))]
+        # 32-bit sums over up to 256 channels, and over the tokens that a decay near one lets through
+        assert max(errors[parts]) < 2e-6, errors
+        assert torch.equal(s[4].cpu(), state[4])                                      # a slot of no row
+    assert errors[True][0] < 1.25 * errors[False][0] + 1e-8 and errors[True][1] < 2 * errors[False][1], errors
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_what_is_no_number_reaches_no_earlier_token(K, form):
+    """An infinity among token 37's values, and then among its keys: the outputs before it keep their bits, those from it on are no numbers."""
+    t, heads, dim, vdim = 220, 2, 64, 64
+    g = torch.Generator().manual_seed(1)
+    qk = torch.nn.functional.normalize(torch.randn(t, 2, heads, dim, generator=g), dim=-1).to(DEV)
+    v, decay = torch.randn(t, heads, vdim, generator=g).to(DEV), (1 - torch.rand(t, heads, dim, generator=g) * 0.1).to(DEV)
+    beta, rate = torch.rand(t, heads, generator=g).to(DEV), torch.rand(t, heads, dim, generator=g).to(DEV)
+    rows = Rows(torch.zeros(1, dtype=torch.int32, device=DEV), torch.tensor([0, t], dtype=torch.int32, device=DEV),
+                torch.tensor([t], dtype=torch.int32, device=DEV), 1, t, 0, t, t)
+
+    def run(qk, v):
+        out, state = torch.empty_like(v), torch.zeros(2, heads, vdim, dim, device=DEV)
+        K.recurrent_scan(out, qk, v, decay if form in ("delta", "general") else None, decay[0, :, 0].contiguous() if form == "fixed" else None,
+                         beta if form == "delta" else None, state, rows, token_decay=decay[:, :, 0].contiguous() if form == "token" else None,
+                         rate=rate if form == "general" else None)
+        return out, state
+
+    clean, _ = run(qk, v)
+    bad_v, bad_k = v.clone(), qk.clone()
+    bad_v[37, 1, 5] = float("inf")
+    bad_k[37, 1, 1, 7] = float("inf")
+    for out, state, where in ((*run(qk, bad_v), (slice(37, None), 1, 5)), (*run(bad_k, v), (slice(38, None), 1))):
+        assert torch.equal(out[:37], clean[:37]) and torch.equal(out[:, 0], clean[:, 0])
+        assert not out[where].isfinite().any() and not state[0, 1].isfinite().all()
