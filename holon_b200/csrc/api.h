@@ -413,6 +413,13 @@ int hb_softcap(float* x, long count, float cap, hb_stream stream);
 int hb_recurrent_scan(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
                       const float* token_decay, const float* beta, const float* rate, const float* take, const float* skip,
                       float* state, const int32_t* query_start, const int32_t* row_slot, int rows, int heads, int kv_heads, int dim, int vdim, int most, hb_stream stream);
+// The same with beta or rate for rows row0 .. rows - 1, eight tokens at a time (csrc/recurrent_blocks.cu), key sizes 64, 128 and 256.
+// blocks: at least the sum over the rows of ceil(tokens / 8); scratch: blocks * heads * hb_recurrent_blocks_floats(rate given, dim)
+// floats (0: a key size that is not taken) on a 16-byte boundary.
+int hb_recurrent_blocks(float* out, const float* qk, const float* v, const float* decay, const float* head_decay, const float* beta,
+                        const float* rate, float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
+                        int rows, int blocks, int heads, int kv_heads, int dim, int vdim, hb_stream stream);
+int hb_recurrent_blocks_floats(int general, int dim);
 // The generalized delta rule's inputs from its first product, rows [r | k | v | g | a] of `dtype` (each heads dim wide,
 // `ld` apart) and the low-rank decay projection's output `pre` [tokens, heads dim] in 32-bit: qk = (r, k), v,
 // decay = exp(-decay_scale sigmoid(pre + decay_bias)), rate = sigmoid(a + rate_bias) / (sum_head k^2 + unit_eps); with

@@ -177,7 +177,7 @@ class CudaKernels:
         # Two mixers that read the same input run as two branches of a step's graph (HOLON_B200_BRANCHES=0: one after the other).
         self.branches = os.environ.get("HOLON_B200_BRANCHES", "1") != "0"
         self._side = None
-        self.scan_parts = True                # rows of many tokens through csrc/state_space.cu (tests: False)
+        self.scan_parts = True                # rows of many tokens through csrc/state_space.cu, recurrent_blocks.cu (tests: False)
         # One word of page-locked host memory that a kernel's bounded wait writes when it gives up (csrc/status.cu)
         word = ctypes.POINTER(ctypes.c_uint)()
         with torch.cuda.device(self.device):
@@ -1201,6 +1201,9 @@ class CudaKernels:
     # Tokens a row on average from which the scan goes in chunks of 64 (four launches: 16 heads of 128 by 128, one row of 128 tokens
     # 33 us token by token and 43 in chunks, 256 tokens 60 and 49, 2,048 tokens 422 and 154; eight rows of 100 96 and 106).
     CHUNK_TOKENS = 192
+    # And eight tokens at a time (two launches: the delta rule with 32 tokens 17 us token by token and 24 in blocks, 48 tokens 21 and
+    # 21, 64 tokens 25 and 23, 2,048 tokens 574 and 367; eight rows of 40 70 and 35; the generalized rule alike).
+    BLOCK_TOKENS = 48
 
     def recurrent_scan(self, out, qk, v, decay, head_decay, beta, state, rows, token_decay=None, rate=None, take=None,
                        skip=None) -> None:
@@ -1221,8 +1224,8 @@ class CudaKernels:
                 or (take is not None and take.shape != (t, heads)) or (skip is not None and skip.shape != (heads,)):
             raise KernelError("recurrent_scan: qk [tokens, 2, kv_heads, dim], v and out [tokens, heads, vdim], state "
                               "[slots, heads, vdim, dim], decay [tokens, heads, dim] or head_decay [heads], beta [tokens, heads]")
-        # Rows of many tokens: in chunks of 64 where the decay is one number per head. What the launches depend on are counts of
-        # rows and tokens, so that they can be captured.
+        # Rows of many tokens: in chunks of 64 where the decay is one number per head, with a delta rule eight tokens at a time.
+        # What the launches depend on are counts of rows and tokens, so that they can be captured.
         scanned, ones, portions = rows.n_rows, rows.n_decode, rows.n_rows - rows.n_decode
         more = t - ones
         ends = (self._i32(rows.query_start, "query_start"), self._i32(rows.row_slot, "row_slot"), ones, rows.n_rows)
@@ -1232,6 +1235,14 @@ class CudaKernels:
             scratch = torch.empty(tiles * (heads * vdim * dim + kv_heads * 64 * 64 + heads), dtype=torch.float32, device=self.device)
             self._call("hb_recurrent_chunks", self._p(out), self._p(qk), self._p(v), self._p(head_decay), self._p(token_decay),
                        self._p(state), self._p(scratch), *ends, tiles, heads, kv_heads, dim, vdim)
+        elif self.scan_parts and portions and (beta is not None) != (rate is not None) and token_decay is None \
+                and more >= self.BLOCK_TOKENS * portions and not state.data_ptr() % 16:
+            floats = self.lib.hb_recurrent_blocks_floats(int(rate is not None), dim)   # (0: a key size that is not taken)
+            if floats:
+                scanned, blocks = ones, more // 8 + portions
+                scratch = torch.empty(blocks * heads * floats, dtype=torch.float32, device=self.device)
+                self._call("hb_recurrent_blocks", self._p(out), self._p(qk), self._p(v), self._p(decay), self._p(head_decay),
+                           self._p(beta), self._p(rate), self._p(state), self._p(scratch), *ends, blocks, heads, kv_heads, dim, vdim)
         if scanned:
             self._call("hb_recurrent_scan", self._p(out), self._p(qk), self._p(v), self._p(decay), self._p(head_decay),
                        self._p(token_decay), self._p(beta), self._p(rate), self._p(take), self._p(skip), self._p(state),
