@@ -451,6 +451,92 @@ __global__ void delta_prepare_kernel(float* __restrict__ qk, float* __restrict__
     if (e < nv) gate[(size_t)t * nv + e] = sigmoid_f(z[heads * dim + e]);
 }
 
+// The same for steps of many tokens, four neighbouring numbers a thread over `run` tokens in turn: the convolution's weights and inputs wait in
+// registers from token to token, each head of q and k is dim / 4 neighbouring lanes (a power of two up to 32), whose inputs are read once. grid
+// (runs of tokens, blocks of the quads of q, k and v | of beta's heads | of the decays' quads | of the gate's). Bound by memory: 2,048 tokens,
+// 16 heads of 128 by 128 over 4 key heads move 105 MB in 35 us (3.0 TB/s); an element a thread and token took 113 us.
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(128) delta_prepare_wide_kernel(
+        float* __restrict__ qk, float* __restrict__ v, float* __restrict__ beta, float* __restrict__ decay, float* __restrict__ gate,
+        const T* __restrict__ first, int ld, const T* __restrict__ conv, T* conv_state, const float* __restrict__ low2,
+        const float* __restrict__ dt_bias, const float* __restrict__ rate_log, const int32_t* __restrict__ query_start,
+        const int32_t* __restrict__ row_slot, int rows, int tokens, int run, int heads, int kv_heads, int dim, int vdim, float q_scale,
+        float unit_eps, int carry, int conv_blocks, int beta_blocks, int decay_blocks) {
+    const int nq = kv_heads * dim, nv = heads * vdim, nd = heads * dim, C = 2 * nq + nv;
+    const int begin = blockIdx.x * run, end = min(begin + run, tokens);
+    int seg = blockIdx.y;
+    if (seg < conv_blocks) {
+        const int quad = seg * 128 + threadIdx.x;
+        const bool live = quad < C / 4;
+        const int c = live ? quad * 4 : 0, lanes = dim / 4;
+        constexpr int KEEP = TAPS > 1 ? TAPS - 1 : 1;
+        float w[TAPS][4], before[KEEP][4];                               // before: the inputs ahead of the token, oldest first
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[j][i] = to_f32(conv[(size_t)(c + i) * TAPS + j]);
+        int b = row_of_token(query_start, rows, begin);
+        for (int t = begin; t < end; ++t) {
+            while (t >= query_start[b + 1]) ++b;
+            const int t0 = query_start[b];
+            T* st = TAPS > 1 ? conv_state + (size_t)row_slot[b] * (TAPS - 1) * C + c : nullptr;
+            auto input = [&](int from, float (&x)[4]) {                  // the inputs of token `from` of this row
+                Vec4<T>::load(from >= t0 ? first + (size_t)from * ld + c : st + (size_t)(TAPS - 1 + (from - t0)) * C, x);
+            };
+            if (t == begin || t == t0) {
+#pragma unroll
+                for (int j = 0; j + 1 < TAPS; ++j) input(t - (TAPS - 1) + j, before[j]);
+            }
+            float x[4], acc[4] = {0.f, 0.f, 0.f, 0.f};
+            input(t, x);
+#pragma unroll
+            for (int j = 0; j + 1 < TAPS; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] = fmaf(w[j][i], before[j][i], acc[i]);
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc[i] = silu_f(fmaf(w[TAPS - 1][i], x[i], acc[i]));
+                ss = fmaf(acc[i], acc[i], ss);
+#pragma unroll
+                for (int j = 0; j + 2 < TAPS; ++j) before[j][i] = before[j + 1][i];
+                before[KEEP - 1][i] = x[i];
+            }
+            if (carry && live && TAPS > 1 && query_start[b + 1] - t0 == 1) {     // a row of one token: its carried inputs move on
+#pragma unroll
+                for (int j = 0; j + 1 < TAPS; ++j) Vec4<T>::store(st + (size_t)j * C, before[j]);
+            }
+            for (int o = 1; o < lanes; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);   // (a warp of v's quads sums for nothing)
+            const float f = c >= 2 * nq ? 1.f : rsqrtf(ss + unit_eps) * (c < nq ? q_scale : 1.f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] *= f;
+            if (live) Vec4<float>::store(c < 2 * nq ? qk + (size_t)t * 2 * nq + c : v + (size_t)t * nv + (c - 2 * nq), acc);
+        }
+        return;
+    }
+    seg -= conv_blocks;
+    if (seg < beta_blocks) {
+        const int h = seg * 128 + threadIdx.x;
+        if (h < heads)
+            for (int t = begin; t < end; ++t) beta[(size_t)t * heads + h] = sigmoid_f(to_f32(first[(size_t)t * ld + C + h]));
+        return;
+    }
+    seg -= beta_blocks;
+    const bool decays = seg < decay_blocks;
+    const int e = ((decays ? seg : seg - decay_blocks) * 128 + threadIdx.x) * 4;
+    if (e >= (decays ? nd : nv)) return;
+    const float rate = decays ? -expf(rate_log[e / dim]) : 0.f;
+    float bias[4] = {0.f, 0.f, 0.f, 0.f};
+    if (decays) Vec4<float>::load(dt_bias + e, bias);
+    for (int t = begin; t < end; ++t) {
+        float z[4];
+        Vec4<float>::load(low2 + (size_t)t * (nd + nv) + (decays ? e : nd + e), z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] = decays ? expf(rate * softplus_f(z[i] + bias[i])) : sigmoid_f(z[i]);
+        Vec4<float>::store(decays ? decay + (size_t)t * nd + e : gate + (size_t)t * nv + e, z);
+    }
+}
+
 extern "C" int hb_delta_prepare(float* qk, float* v, float* beta, float* decay, float* gate, const void* first, int dtype,
                                 int ld, const void* conv, int taps, void* conv_state, const float* low2,
                                 const float* dt_bias, const float* rate_log, const int32_t* query_start,
@@ -463,6 +549,30 @@ extern "C" int hb_delta_prepare(float* qk, float* v, float* beta, float* decay, 
     if (segments > 65535) HB_REFUSE("delta_prepare: %ld segments a token are above 65535", segments);
     dim3 grid(tokens, (unsigned)segments);
     cudaStream_t s = (cudaStream_t)stream;
+    // From 64 tokens on, with two to four taps and rows that 16-byte (bfloat16: 8-byte) reads fit (16 heads of 128 by 128 over 4 key heads,
+    // bfloat16, 2,048 tokens: 35 us, an element a thread 113).
+    const size_t four = dtype == HB_F32 ? 16 : 8;
+    const int lanes = dim / 4;
+    if (tokens >= 64 && taps >= 2 && taps <= 4 && dim % 4 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && vdim % 4 == 0 && ld % 4 == 0
+        && (((uintptr_t)qk | (uintptr_t)v | (uintptr_t)decay | (uintptr_t)gate | (uintptr_t)low2 | (uintptr_t)dt_bias) & 15) == 0
+        && (((uintptr_t)first | (uintptr_t)conv_state) % four) == 0 && (dtype == HB_F32 || dtype == HB_BF16)) {
+        const int nd = heads * dim, nv = heads * vdim, C = 2 * kv_heads * dim + nv;
+        const int conv_blocks = (C / 4 + 127) / 128, beta_blocks = (heads + 127) / 128, decay_blocks = (nd / 4 + 127) / 128;
+        const int run = tokens >= 1024 ? 8 : tokens >= 256 ? 4 : 2;
+        const long segs = (long)conv_blocks + beta_blocks + decay_blocks + (nv / 4 + 127) / 128;
+        if (segs <= 65535) {
+            const dim3 wide((tokens + run - 1) / run, (unsigned)segs);
+#define HB_WIDE(T, N) delta_prepare_wide_kernel<T, N><<<wide, 128, 0, s>>>(qk, v, beta, decay, gate, (const T*)first, ld, (const T*)conv, \
+    (T*)conv_state, low2, dt_bias, rate_log, query_start, row_slot, rows, tokens, run, heads, kv_heads, dim, vdim, q_scale, unit_eps, carry, \
+    conv_blocks, beta_blocks, decay_blocks)
+#define HB_TAPS(T) do { if (taps == 4) HB_WIDE(T, 4); else if (taps == 3) HB_WIDE(T, 3); else HB_WIDE(T, 2); } while (0)
+            if (dtype == HB_F32) HB_TAPS(float); else HB_TAPS(bf16);
+#undef HB_TAPS
+#undef HB_WIDE
+            HB_LAUNCH_CHECK("delta_prepare");
+            return 0;
+        }
+    }
 #define HB_ARGS(T) (const T*)first, ld, (const T*)conv, taps, (T*)conv_state, low2, dt_bias, rate_log, \
     query_start, row_slot, rows, heads, kv_heads, dim, vdim, q_scale, unit_eps, carry
     if (dtype == HB_F32) delta_prepare_kernel<float><<<grid, 256, 0, s>>>(qk, v, beta, decay, gate, HB_ARGS(float));
@@ -647,6 +757,59 @@ __global__ void retention_prepare_kernel(float* __restrict__ qk, float* __restri
     if (e < heads * vdim) v[t * heads * vdim + e] = in(2 * nq + e);
 }
 
+// The same with four neighbouring numbers a thread, and of rotated channels the four they turn with. A head of q or k is half / 4 units that turn
+// and (dim - rot_dims) / 4 that do not. Bound by memory (2,048 tokens of 16 heads of 128 by 128: 75 MB in 13 us; an element a thread took 52 us).
+template <typename T>
+__global__ void __launch_bounds__(256) retention_prepare_wide_kernel(float* __restrict__ qk, float* __restrict__ v, const T* __restrict__ first,
+                                                                     int ld, const int32_t* __restrict__ positions,
+                                                                     const float* __restrict__ table, int rot_dims, int max_positions, int heads,
+                                                                     int dim, int vdim, float k_scale, int silu) {
+    const size_t t = blockIdx.x;
+    const T* row = first + t * ld;
+    const int half = rot_dims >> 1, nq = heads * dim, turning = half >> 2, units = turning + ((dim - rot_dims) >> 2);
+    auto load = [&](int i, float (&x)[4]) {
+        Vec4<T>::load(row + i, x);
+        if (silu)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[k] = silu_f(x[k]);
+    };
+    int u = blockIdx.y * 256 + threadIdx.x;
+    if (u < 2 * heads * units) {
+        const int h = u / units, i = u - h * units;                      // (q's heads, then k's)
+        const float f = h >= heads ? k_scale : 1.f;
+        float x[4];
+        if (i >= turning) {
+            const int e = h * dim + rot_dims + (i - turning) * 4;
+            load(e, x);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[k] *= f;
+            Vec4<float>::store(qk + t * 2 * nq + e, x);
+            return;
+        }
+        const int pos = min(max(positions[t], 0), max_positions > 0 ? max_positions - 1 : 0), e = h * dim + i * 4;
+        const float* cs = table + (size_t)pos * rot_dims + i * 4;
+        float y[4], c[4], n[4], a[4], b[4];
+        load(e, x);
+        load(e + half, y);
+        Vec4<float>::load(cs, c);
+        Vec4<float>::load(cs + half, n);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            a[k] = (x[k] * c[k] - y[k] * n[k]) * f;
+            b[k] = (y[k] * c[k] + x[k] * n[k]) * f;
+        }
+        Vec4<float>::store(qk + t * 2 * nq + e, a);
+        Vec4<float>::store(qk + t * 2 * nq + e + half, b);
+        return;
+    }
+    u -= 2 * heads * units;
+    if (u < heads * vdim / 4) {
+        float x[4];
+        load(2 * nq + u * 4, x);
+        Vec4<float>::store(v + t * heads * vdim + u * 4, x);
+    }
+}
+
 extern "C" int hb_retention_prepare(float* qk, float* v, const void* first, int dtype, int ld, const int32_t* positions,
                                     const float* table, int rot_dims, int max_positions, int tokens, int heads, int dim,
                                     int vdim, float k_scale, int silu, hb_stream stream) {
@@ -656,6 +819,15 @@ extern "C" int hb_retention_prepare(float* qk, float* v, const void* first, int 
     cudaStream_t s = (cudaStream_t)stream;
     const long segments = (2L * heads * dim + (long)heads * vdim + 255) / 256;
     if (segments > 65535) HB_REFUSE("retention_prepare: %ld segments a token are above 65535", segments);
+    if (dim % 4 == 0 && vdim % 4 == 0 && rot_dims % 8 == 0 && ld % 4 == 0 && (((uintptr_t)qk | (uintptr_t)v | (uintptr_t)table) & 15) == 0
+        && (uintptr_t)first % (dtype == HB_F32 ? 16 : 8) == 0 && (dtype == HB_F32 || dtype == HB_BF16)) {
+        const int units = 2 * heads * (rot_dims / 8 + (dim - rot_dims) / 4) + heads * vdim / 4;
+        const dim3 wide(tokens, (units + 255) / 256);
+        if (dtype == HB_F32) retention_prepare_wide_kernel<float><<<wide, 256, 0, s>>>(qk, v, (const float*)first, ld, positions, table, rot_dims, max_positions, heads, dim, vdim, k_scale, silu);
+        else retention_prepare_wide_kernel<bf16><<<wide, 256, 0, s>>>(qk, v, (const bf16*)first, ld, positions, table, rot_dims, max_positions, heads, dim, vdim, k_scale, silu);
+        HB_LAUNCH_CHECK("retention_prepare");
+        return 0;
+    }
     const dim3 tokens_by_segments(tokens, (unsigned)segments);
     if (dtype == HB_F32) retention_prepare_kernel<float><<<tokens_by_segments, 256, 0, s>>>(qk, v, (const float*)first, ld, positions, table, rot_dims, max_positions, heads, dim, vdim, k_scale, silu);
     else if (dtype == HB_BF16) retention_prepare_kernel<bf16><<<tokens_by_segments, 256, 0, s>>>(qk, v, (const bf16*)first, ld, positions, table, rot_dims, max_positions, heads, dim, vdim, k_scale, silu);

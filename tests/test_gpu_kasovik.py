@@ -459,3 +459,44 @@ def test_generate_on_the_command_line(tmp_path, capsys):
             logits = plain.forward(weights, config, ids)[-1]
             assert float(logits.max() - logits[token]) <= 1e-3 * float(logits.std()), (len(ids), token)
             ids.append(token)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps", [(4, 2, 64, 32, 4), (6, 3, 128, 36, 3), (5, 5, 4, 12, 2), (3, 1, 96, 32, 4), (2, 1, 64, 32, 1)])
+@pytest.mark.parametrize("counts", [[1, 70], [1, 1, 300, 2], [1, 64, 1023, 5]])
+def test_delta_prepare_of_many_tokens(K, dtype, heads, kv_heads, dim, vdim, taps, counts):
+    """Four channels a thread over runs of two, four and eight tokens (and sizes that stay with the other kernel): runs that
+    cross rows, rows that end inside a run, one-token rows whose carried inputs the kernel itself moves on."""
+    t, nv = sum(counts), heads * vdim
+    c = 2 * kv_heads * dim + nv
+    slots = list(range(len(counts)))[::-1]
+    first, conv = rand(t, c + heads, dtype=dtype, seed=t), rand(c, taps, dtype=dtype, seed=1, scale=0.6)
+    low2, dt_bias, rate_log = rand(t, heads * dim + nv, seed=2, scale=2.0), rand(heads * dim, seed=4), rand(heads, seed=5) - 1.0
+    cw = rand(len(counts) + 1, taps - 1, c, dtype=dtype, seed=6) if taps > 1 else None
+    cg = cw.to(DEV) if taps > 1 else None
+    shapes = [(t, 2, kv_heads, dim), (t, heads, vdim), (t, heads), (t, heads, dim), (t, nv)]
+    got, want = [torch.full(s, float("nan"), device=DEV) for s in shapes], [torch.zeros(s) for s in shapes]
+    K.delta_prepare(*got, first.to(DEV), conv.to(DEV), cg, low2.to(DEV), dt_bias.to(DEV), rate_log.to(DEV), rows_of(counts, slots),
+                    dim ** -0.5, 1e-6, carry=True)
+    K.conv_carry(cg, first.to(DEV), c, taps, rows_of(counts, slots), least=2)
+    REF.delta_prepare(*want, first, conv, cw, low2, dt_bias, rate_log, rows_of(counts, slots, device="cpu"), dim ** -0.5, 1e-6)
+    REF.conv_carry(cw, first, c, taps, rows_of(counts, slots, device="cpu"))
+    for g, w in zip(got, want):
+        close(g, w, torch.float32, scale=8.0)
+    if taps > 1:
+        assert torch.equal(cg.cpu(), cw)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim,vdim,rot_dims", [(128, 128, 128), (64, 20, 16), (16, 4, 8), (24, 12, 0)])
+def test_retention_prepare_four_numbers_a_thread(K, dtype, dim, vdim, rot_dims):
+    t, heads = 70, 5
+    first, positions = rand(t, 2 * heads * dim + heads * vdim + 4, dtype=dtype, seed=1), torch.arange(t, dtype=torch.int32) * 3 % 200
+    table = rand(200, rot_dims, seed=3) if rot_dims else None
+    for silu in (False, True):
+        got = [torch.full(s, float("nan"), device=DEV) for s in ((t, 2, heads, dim), (t, heads, vdim))]
+        want = [torch.zeros(*g.shape) for g in got]
+        K.retention_prepare(*got, first.to(DEV), positions.to(DEV), table.to(DEV) if rot_dims else None, rot_dims, 0.3, silu=silu)
+        REF.retention_prepare(*want, first, positions, table, rot_dims, 0.3, silu=silu)
+        for g, w in zip(got, want):
+            close(g, w, torch.float32)
