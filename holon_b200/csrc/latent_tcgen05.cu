@@ -5,20 +5,20 @@
 // side of one problem: its folded queries qa are contiguous rows of rank + rot. A CTA owns 128 of them and walks the
 // 64-row tiles of the cache that some of them see:
 //   S = Q K^T    tcgen05.mma 128 x 64 x 16 over rank + rot, both operands in shared memory (TMA, 128-byte swizzle, blocks
-//                of 64 columns), S in one of two 64-column tensor-memory buffers;
-//   softmax      four warps, one row per thread, the running maximum lagging by up to 2^8 (as in attention_tcgen05.cu);
-//                the weights go back to tensor memory as bfloat16 pairs, over the S they came from;
+//                of 64 columns), in two sums: over the blocks that hold output columns of this CTA and over the others, each
+//                issued by a warp of its own into 64 columns of tensor memory, two buffers of each;
+//   softmax      four warps, one row per thread, which adds the two sums, the running maximum lagging by up to 2^8 (as in attention_tcgen05.cu);
+//                the weights go back to tensor memory as bfloat16 pairs, over the first of the sums they came from;
 //   O += P C     tcgen05.mma 128 x (rank / VS) x 16, four per tile, P from tensor memory, the same cache rows in shared
 //                memory as an MN-major operand.
 // An output of 128 x 512 alone would fill tensor memory, so above rank 256 two CTAs (VS = 2, neighbours in the grid) take
 // half of the output's columns each and both compute the scores: 1.5 times the multiply-adds, 40 tensor instructions a
 // tile and CTA. At rank 512 + 64 the queries take 144 KB of shared memory and leave room for one tile of the cache (72 KB): its
-// blocks that hold none of this CTA's output columns are free, and are refilled, as soon as the scores are done, and the
-// next tile's scores begin with them; the others follow when the weights have been applied. Smaller ranks hold up to
-// three tiles.
-// Bound at rank 512 by the 36 score instructions of a tile, of which one thread issues one in about 100 ns, and by the
-// chain weights applied -> half of the next tile loaded -> its scores -> softmax. 2,048 tokens, 16 heads, rank 512 + 64:
-// 234 us (mma.sync, latent_bf16.cu: 730 us); two prompts of 1,500 and 938 tokens, 16 heads, a window of 1,024: 187 us (519 us).
+// blocks that hold none of this CTA's output columns are free, and are refilled, as soon as their sum is done, and the
+// next tile's begins; the others follow when the weights have been applied. Smaller ranks hold up to three tiles.
+// Bound at rank 512 by the chain weights applied -> half of the next tile loaded -> its scores -> softmax, which one tile in shared
+// memory does not let overlap. 2,048 tokens, 16 heads, rank 512 + 64: 219 us (one warp for both sums: 234; mma.sync, latent_bf16.cu: 730);
+// two prompts of 1,500 and 938 tokens, 16 heads, a window of 1,024: 188 us (187; 519).
 // Cache rows past a request's length are zeroed in shared memory before they are used.
 // Every mbarrier wait is bounded (tcgen05.cuh).
 #include "tcgen05.cuh"
@@ -29,8 +29,9 @@
 #define LT_STAGES 3
 #define LT_Q_BLOCK (LT_BM * 128)                  // bytes of a [128 x 64] block of queries
 #define LT_K_BLOCK (LT_BN * 128)
-#define LT_THREADS 224
-#define LT_TMEM_COLS 512                          // S0 [0, 64), S1 [64, 128), O [128, 128 + rank / VS)
+#define LT_THREADS 256
+#define LT_TMEM_COLS 512                          // buffer i: sums [128 i, 128 i + 64) and [128 i + 64, 128 i + 128); O [256, 256 + rank / VS)
+#define LT_O 256
 #define LT_RESCALE 8.0f
 #define LT_SMEM_MAX 232448
 
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tcgen05_kernel(
             mbar_init(a_full0 + 8 * s, 1); mbar_init(a_empty0 + 8 * s, 1);
             mbar_init(v_full0 + 8 * s, 1); mbar_init(v_empty0 + 8 * s, 1);
         }
-        for (int i = 0; i < 2; ++i) { mbar_init(s_full0 + 8 * i, 1); mbar_init(p_full0 + 8 * i, 4); mbar_init(p_empty0 + 8 * i, 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(s_full0 + 8 * i, 2); mbar_init(p_full0 + 8 * i, 4); mbar_init(p_empty0 + 8 * i, 1); }
         mbar_init(o_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -114,55 +115,54 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tcgen05_kernel(
                 for (int i = v0; i < v0 + nv; ++i) tma_load_2d(dst + i * LT_K_BLOCK, &map_kv, v_full0 + 8 * s, i * 64, row);
             }
         }
-    } else if (b >= 0 && warp == 1) {
+    } else if (b >= 0 && (warp == 1 || warp == 7)) {                          // the scores: blocks without values, blocks with
         // kind::f16, D float32, A and B bfloat16; N / 8 at bit 17, M / 16 at bit 24
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(LT_BN >> 3) << 17) | ((uint32_t)(LT_BM >> 4) << 24);
+        const bool values = warp == 7;
+        const uint32_t full0 = values ? v_full0 : a_full0;
         // (all lanes wait, and agree on how a wait ended: they zero rows together)
         bool ok = tiles > 0 && __all_sync(0xffffffffu, mbar_wait(q_full, 0, 3));
-        for (int j = 0; j < tiles; ++j) {
+        for (int j = 0; j < tiles && ok; ++j) {
             const int s = j % stages;
-            const uint32_t parity = (j / stages) & 1, src = kv_s + s * stage_bytes, s_t = tmem + (j & 1) * LT_BN;
+            const uint32_t src = kv_s + s * stage_bytes, s_t = tmem + (j & 1) * 2 * LT_BN + (values ? LT_BN : 0);
             const int past = n - (tile_lo + j) * LT_BN;                       // rows of the tile from here on lie past the request's end
-            uint32_t some = 0;
-            // S_j overwrites S and the weights of tile j - 2: wait until those have been applied
-            if (ok && j >= 2) ok = __all_sync(0xffffffffu, mbar_wait(p_empty0 + 8 * (j & 1), ((j - 2) >> 1) & 1, 4));
-            for (int half = 0; half < 2 && ok; ++half) {                      // the score-only blocks, then the value blocks
-                ok = __all_sync(0xffffffffu, mbar_wait((half ? v_full0 : a_full0) + 8 * s, parity, 5));
-                if (!ok) break;
-                if (past < LT_BN) {
-                    for (int i = 0; i < blocks; ++i)
-                        if ((i >= v0 && i < v0 + nv) == (half == 1))
-                            for (int at = past * 128 + lane * 16; at < LT_K_BLOCK; at += 512)   // (the swizzle stays within a row's 128 bytes)
-                                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(src + i * LT_K_BLOCK + at), "r"(0) : "memory");
-                    fence_async_smem();
-                    __syncwarp();
-                }
-                if (lane == 0) {
-                    tc_fence_after();
-                    for (int i = 0; i < blocks; ++i) {
-                        if ((i >= v0 && i < v0 + nv) != (half == 1)) continue;
-                        const int steps = min(4, (dk - i * 64) >> 4);
-                        const uint64_t da = tc_smem_desc(q_s + i * LT_Q_BLOCK), db = tc_smem_desc(src + i * LT_K_BLOCK);
-                        for (int kk = 0; kk < steps; ++kk) { tc_mma(s_t, da + 2 * kk, db + 2 * kk, idesc, some); some = 1; }
-                    }
-                    if (half == 0) tc_commit(a_empty0 + 8 * s);               // these blocks have been read
-                    else tc_commit(s_full0 + 8 * (j & 1));
-                }
+            // S_j overwrites the sums and the weights of tile j - 2: wait until those have been applied
+            if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait(p_empty0 + 8 * (j & 1), ((j - 2) >> 1) & 1, 4));
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (j / stages) & 1, 5));
+            if (!ok) break;
+            if (past < LT_BN) {
+                for (int i = 0; i < blocks; ++i)
+                    if ((i >= v0 && i < v0 + nv) == values)
+                        for (int at = past * 128 + lane * 16; at < LT_K_BLOCK; at += 512)   // (the swizzle stays within a row's 128 bytes)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(src + i * LT_K_BLOCK + at), "r"(0) : "memory");
+                fence_async_smem();
                 __syncwarp();
             }
-            if (!ok) break;
+            if (lane == 0) {
+                tc_fence_after();
+                uint32_t some = 0;
+                for (int i = 0; i < blocks; ++i) {
+                    if ((i >= v0 && i < v0 + nv) != values) continue;
+                    const int steps = min(4, (dk - i * 64) >> 4);
+                    const uint64_t da = tc_smem_desc(q_s + i * LT_Q_BLOCK), db = tc_smem_desc(src + i * LT_K_BLOCK);
+                    for (int kk = 0; kk < steps; ++kk) { tc_mma(s_t, da + 2 * kk, db + 2 * kk, idesc, some); some = 1; }
+                }
+                if (!values) tc_commit(a_empty0 + 8 * s);                     // these blocks have been read
+                tc_commit(s_full0 + 8 * (j & 1));
+            }
+            __syncwarp();
         }
     } else if (b >= 0 && warp == 6) {
         if (lane == 0) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(nv << 3) << 17) | ((uint32_t)(LT_BM >> 4) << 24);
-            const uint32_t o_t = tmem + 2 * LT_BN;
+            const uint32_t o_t = tmem + LT_O;
             bool ok = true;
             for (int j = 0; j < tiles && ok; ++j) {                           // O += P_j C_j
                 const int s = j % stages;
                 ok = mbar_wait(p_full0 + 8 * (j & 1), (j >> 1) & 1, 6);       // (its scores read the same blocks: they are there)
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t src = kv_s + s * stage_bytes + v0 * LT_K_BLOCK, p_t = tmem + (j & 1) * LT_BN;
+                const uint32_t src = kv_s + s * stage_bytes + v0 * LT_K_BLOCK, p_t = tmem + (j & 1) * 2 * LT_BN;
 #pragma unroll
                 for (int kk = 0; kk < LT_BN / 16; ++kk)                       // 16 rows a step: 8 columns along P
                     tc_mma_f16_ts(o_t, p_t + kk * 8, tc_smem_desc_mn(src + kk * 16 * 128, LT_K_BLOCK), idesc, (j | kk) != 0);
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tcgen05_kernel(
         const int q = warp & 3, r = q * 32 + lane;                            // this warp's quarter of the TMEM lanes; this thread's row
         const int pos = pos0 + (flat0 + r) / heads;
         const int first_pos = pos0 + flat0 / heads;                           // the tile's first query
-        const uint32_t lane_t = tmem + ((uint32_t)(q * 32) << 16), o_t = lane_t + 2 * LT_BN;
+        const uint32_t lane_t = tmem + ((uint32_t)(q * 32) << 16), o_t = lane_t + LT_O;
         float m_used = -INFINITY, l = 0.f;                                    // in log2 units; the maximum may lag by LT_RESCALE
         bool ok = true;
         for (int j = 0; j < tiles && ok; ++j) {
@@ -184,9 +184,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tcgen05_kernel(
             if (!ok) break;
             tc_fence_after();
             uint32_t sr[2][32];
-            tc_ld32_nowait(lane_t + (j & 1) * LT_BN, sr[0]);
-            tc_ld32_nowait(lane_t + (j & 1) * LT_BN + 32, sr[1]);
-            tc_ld_wait();
+            const uint32_t s_t = lane_t + (j & 1) * 2 * LT_BN;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {                                     // the two sums of 32 scores
+                uint32_t other[32];
+                tc_ld32_nowait(s_t + 32 * c, sr[c]);
+                tc_ld32_nowait(s_t + LT_BN + 32 * c, other);
+                tc_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) sr[c][i] = __float_as_uint(__uint_as_float(sr[c][i]) + __uint_as_float(other[i]));
+            }
             const int key0 = (tile_lo + j) * LT_BN;
             if (key0 + LT_BN - 1 > first_pos || window > 0) {
 #pragma unroll
@@ -243,7 +250,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tcgen05_kernel(
             unpack2(add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3])), lo, hi);
             l += lo + hi;
             if (!ok) break;
-            tc_st32(lane_t + (j & 1) * LT_BN, pk);                            // P over the S it came from
+            tc_st32(s_t, pk);                                                 // P over the first of the sums it came from
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full0 + 8 * (j & 1));
