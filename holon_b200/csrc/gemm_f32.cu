@@ -40,8 +40,9 @@ __device__ __forceinline__ float2 halves(uint64_t v) {
 // that the registers hold one set of sums. Where there are too few tiles for the chip, the blocks of a cluster of SPLIT
 // share a tile's segments and add them through distributed shared memory.
 // Measured with a 28-layer model of width 1,024 in one pass over 541 rows: its 112 products of 4,096 and 6,144 columns by
-// 1,024 take 157 us on average (36 TFLOP/s), those of 1,024 columns by 2,048 and 3,072 122 us. With 64 x 64 tiles and 4 x 4
-// outputs a thread this pass and four steps of two rows took 78.7 ms in products, now 20.3.
+// 1,024 take 139 us on average (41 TFLOP/s), those of 1,024 columns by 2,048 and 3,072 109 us. With 64 x 64 tiles and 4 x 4
+// outputs a thread this pass and four steps of two rows took 78.7 ms in products, now 18.5. What bounds it: three wavefronts of the
+// shared-memory pipe a wide load, 12 for a step of k that multiplies for 16 cycles.
 template <bool VEC, int SPLIT>
 __global__ void __launch_bounds__(128) gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x,
                                                        const float* __restrict__ w, int m, int n, int k, long ldx,
@@ -61,37 +62,33 @@ __global__ void __launch_bounds__(128) gemm_f32_kernel(float* __restrict__ out, 
     const int k_first = s_first * length, k_end = min(k, s_last * length);
     const int steps = k_end > k_first ? (k_end - k_first + BK - 1) / BK : 0, per_segment = length / BK;
 
-    const int xr = m0 + (tid >> 1), xk = (tid & 1) * 8, wr = n0 + tid;  // what this thread loads: 8 of a row of x, 16 of one of w
-    float xv[8], wv[16];
+    // What this thread loads: 4 neighbouring k (4 lanes a row, so that a warp's load touches 8 lines and not 32: with a row a lane these
+    // loads took as much of the L1's bandwidth as all reads of shared memory) of 2 rows of x and 4 of w, 32 rows apart.
+    const int lr = tid >> 2, lk = (tid & 3) * 4;
+    float xv[2][4], wv[4][4];
+    auto fetch4 = [&](float (&v)[4], const float* p, bool there, int kk) {
+        if (VEC) {
+            const float4 f = there && kk < k ? *(const float4*)(p + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = there && kk + j < k ? p[kk + j] : 0.f;
+        }
+    };
     auto fetch = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-            const int kk = k0 + xk + i;
-            if (VEC) {
-                const float4 v = xr < m && kk < k ? *(const float4*)(x + (size_t)xr * ldx + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
-                xv[i] = v.x; xv[i + 1] = v.y; xv[i + 2] = v.z; xv[i + 3] = v.w;
-            } else {
+        for (int i = 0; i < 2; ++i) { const int r = m0 + lr + 32 * i; fetch4(xv[i], x + (size_t)(r < m ? r : 0) * ldx, r < m, k0 + lk); }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) xv[i + j] = xr < m && kk + j < k ? x[(size_t)xr * ldx + kk + j] : 0.f;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-            const int kk = k0 + i;
-            if (VEC) {
-                const float4 v = wr < n && kk < k ? *(const float4*)(w + (size_t)wr * k + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
-                wv[i] = v.x; wv[i + 1] = v.y; wv[i + 2] = v.z; wv[i + 3] = v.w;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) wv[i + j] = wr < n && kk + j < k ? w[(size_t)wr * k + kk + j] : 0.f;
-            }
-        }
+        for (int i = 0; i < 4; ++i) { const int r = n0 + lr + 32 * i; fetch4(wv[i], w + (size_t)(r < n ? r : 0) * k, r < n, k0 + lk); }
     };
     auto stage = [&](int buf) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) xs[buf][xk + i][tid >> 1] = xv[i];
+        for (int j = 0; j < 4; ++j) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) ws[buf][i][tid] = wv[i];
+            for (int i = 0; i < 2; ++i) xs[buf][lk + j][lr + 32 * i] = xv[i][j];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ws[buf][lk + j][lr + 32 * i] = wv[i][j];
+        }
     };
     const int row = (warp & 1) * 32 + (lane >> 3) * 8, col = (warp >> 1) * 64 + (lane & 7) * 4;   // 8 rows; 4 columns here, 4 at + 32
     uint64_t acc[8][4];
@@ -167,13 +164,13 @@ __global__ void __launch_bounds__(128) gemm_f32_kernel(float* __restrict__ out, 
 
 // ---------------------------------------------------------------- few rows
 // Bound by reading w once. A block of 256 threads takes 8 columns and all of k: a thread sums one segment of one column
-// for a quarter of the rows, over pieces of 64 of each segment that a ring of three stages brings by cp.async (so 32 KB a
-// block are on their way while 16 are multiplied). Two rows, the same model's step: 10.4 us a product on average, the head
-// of 151,936 columns among them (21 MB of weights each: 2.0 TB/s); as tiles of 64 rows each was a serial walk over k.
+// for a quarter of the rows, over pieces of 64 of each segment that a ring of stages brings by cp.async: three where many
+// blocks share an SM, six where there are few blocks (all of k up to 3,072 is then on its way at once). Two rows, the same
+// model's step: 7.2 us for a product of 1,024 columns (10 with three stages), 13.2 on average for the wider ones, the head of 151,936
+// columns among them (167 us, 3.7 TB/s); as tiles of 64 rows each was a serial walk over k.
 #define FEW_COLS 8
 #define FEW_PIECE 64
 #define FEW_STRIDE (FEW_PIECE + 4)          // neighbouring (segment, column) rows then lie four banks apart
-#define FEW_STAGES 3
 #define FEW_ROWS 16
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool there) {
@@ -181,7 +178,7 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool there)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
 
-template <int RT>                           // rows a thread: 4 RT >= m
+template <int RT, int FEW_STAGES>           // rows a thread: 4 RT >= m
 __global__ void __launch_bounds__(256) gemm_f32_few_kernel(float* __restrict__ out, const float* __restrict__ x,
                                                            const float* __restrict__ w, int m, int n, int k, long ldx,
                                                            long ldo, long x_batch, long o_batch) {
@@ -274,15 +271,24 @@ static int launch_tiles(float* out, const float* x, const float* w, int m, int n
     return 0;
 }
 
+template <int RT, int FEW_STAGES>
+static int launch_few_stages(float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx, long ldo,
+                      long x_batch, long o_batch, cudaStream_t s) {
+    const int smem = FEW_STAGES * SEGMENTS * (FEW_COLS + m) * FEW_STRIDE * (int)sizeof(float);
+    auto kernel = gemm_f32_few_kernel<RT, FEW_STAGES>;
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 FEW_STAGES * SEGMENTS * (FEW_COLS + min(FEW_ROWS, 4 * RT)) * FEW_STRIDE * (int)sizeof(float)));
+    kernel<<<dim3((n + FEW_COLS - 1) / FEW_COLS, 1, batch), 256, smem, s>>>(out, x, w, m, n, k, ldx, ldo, x_batch, o_batch);
+    return 0;
+}
+
 template <int RT>
 static int launch_few(float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx, long ldo,
                       long x_batch, long o_batch, cudaStream_t s) {
-    const int smem = FEW_STAGES * SEGMENTS * (FEW_COLS + m) * FEW_STRIDE * (int)sizeof(float);
-    auto kernel = gemm_f32_few_kernel<RT>;
-    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 FEW_STAGES * SEGMENTS * (FEW_COLS + FEW_ROWS) * FEW_STRIDE * (int)sizeof(float)));
-    kernel<<<dim3((n + FEW_COLS - 1) / FEW_COLS, 1, batch), 256, smem, s>>>(out, x, w, m, n, k, ldx, ldo, x_batch, o_batch);
-    return 0;
+    const bool deep = (long)((n + FEW_COLS - 1) / FEW_COLS) * batch <= 296 && segment_length(k) > 3 * FEW_PIECE;
+    if constexpr (RT == 1)
+        if (deep) return launch_few_stages<RT, 6>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
+    return launch_few_stages<RT, 3>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
 }
 
 static int launch(const char* what, float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx,
@@ -292,7 +298,10 @@ static int launch(const char* what, float* out, const float* x, const float* w, 
         HB_REFUSE("%s: %d rows, %d products are above the kernel's limits", what, m, batch);
     const bool vec = (k % 4 == 0) && (ldx % 4 == 0) && (x_batch % 4 == 0) && (((uintptr_t)x | (uintptr_t)w) % 16 == 0);
     int rc;
-    if (vec && m <= FEW_ROWS) {
+    // The kernel for few rows reads all of x once per 8 columns: from 9 rows on that is more than the tiles spend on their empty rows,
+    // unless there are few columns (k = 1,024 to 3,072, 16 rows: 1,024 columns 17 to 24 us against 24 to 33 as tiles, 6,144 columns 47
+    // against 37; 8 rows, 6,144 columns 23).
+    if (vec && (m <= FEW_ROWS / 2 || (m <= FEW_ROWS && n <= 2048))) {
         if (m <= 4) rc = launch_few<1>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
         else if (m <= 8) rc = launch_few<2>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
         else rc = launch_few<4>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
