@@ -2,18 +2,24 @@
 // reduced precision; what attention_generic.cu computes, with the keys and values of a step read by tiles instead of once
 // per query and head, and a lane's reads 16 bytes wide and side by side.
 //
-// Rows of one token (rows 0 .. n_decode - 1): a block per (row, kv head, up to HEADS of its query heads); eight lanes share
-// a key and 32 such groups of lanes walk the row's keys, each with a softmax of its own, merged at the end.
+// Rows of one token (rows 0 .. n_decode - 1): a cluster of eight blocks per (row, kv head, up to HEADS of its query heads); eight
+// lanes share a key and the 256 such groups of lanes of a cluster walk the row's keys, each with a softmax of its own, merged
+// per block and then through distributed shared memory.
 // Rows of several tokens: a block per (64 queries, head); 64 keys at a time in shared memory, 4 x 4 scores a thread, then
 // 4 rows x D / 16 columns of the output. Bound by the multiply-adds, next to it by shared memory's bandwidth.
-// Measured on 28 layers of 16 heads of 128 over 8 kv heads, two prompts of 333 and 208 tokens and four steps behind them: 97 us
-// a layer for the prompts, 18.8 us for the two one-token rows; a warp per query and head, a lane per key, took 755 us on
+// Measured on 28 layers of 16 heads of 128 over 8 kv heads, two prompts of 333 and 208 tokens and four steps behind them: 98 us
+// a layer for the prompts, 11.4 us for the two one-token rows (18.8 with one block in a cluster's place); a warp per query and head, a lane per key, took 755 us on
 // average over both.
 // Which groups or tiles a key falls into depends on its position alone, so a token's result does not depend on the rows
 // beside it nor on where its prompt was cut.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
+namespace cg = cooperative_groups;
+
 #define F32_ATT_THREADS 256
+#define F32_ATT_PARTS 8
 
 struct F32Rows {
     float* out;
@@ -51,19 +57,21 @@ __device__ __forceinline__ long key_row(const F32Rows& a, const int32_t* table, 
 // Bound by the latency of a key's reads: a group fetches its next key's row and value while it works on the one before.
 template <int D, int HEADS>                 // D: head_dim rounded up to a multiple of 32 (the lanes' share: D / 8 numbers)
 __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(const F32Rows a) {
-    constexpr int N = D / 32, GROUPS = F32_ATT_THREADS / 8;             // 16-byte pieces of a row a lane holds
+    constexpr int N = D / 32, GROUPS = F32_ATT_THREADS / 8, ALL = GROUPS * F32_ATT_PARTS;   // N: 16-byte pieces of a row a lane holds
     __shared__ __align__(16) float qs[HEADS][D];
     __shared__ float merge_m[HEADS][GROUPS], merge_l[HEADS][GROUPS];
     __shared__ __align__(16) float sums[GROUPS / 4][D];
+    __shared__ float part_m[HEADS], part_l[HEADS], part_v[HEADS][D];
     const int per_kv = a.heads / a.kv_heads, chunks = (per_kv + HEADS - 1) / HEADS;
-    const int b = blockIdx.x, hk = blockIdx.y / chunks, h0 = hk * per_kv + blockIdx.y % chunks * HEADS;
+    const int b = blockIdx.y, part = blockIdx.x, hk = blockIdx.z / chunks, h0 = hk * per_kv + blockIdx.z % chunks * HEADS;
     const int count = min(HEADS, (hk + 1) * per_kv - h0);
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 3, sub = tid & 7;
     const int n = a.kv_len[b], t = a.query_start[b];
     const int pos = n - 1;
     float* o = a.out + ((size_t)t * a.heads + h0) * a.head_dim;
-    if (n <= 0) {
-        for (int i = tid; i < count * a.head_dim; i += F32_ATT_THREADS) o[i] = 0.f;
+    if (n <= 0) {                                                        // (all blocks of the cluster alike)
+        if (part == 0)
+            for (int i = tid; i < count * a.head_dim; i += F32_ATT_THREADS) o[i] = 0.f;
         return;
     }
     const float* qr = a.q + ((size_t)t * a.heads + h0) * a.head_dim;
@@ -98,17 +106,17 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
             }
         }
     };
-    // the group of a key: its position mod GROUPS, wherever the window begins
-    int j = first - first % GROUPS + group;
-    if (j < first) j += GROUPS;
-    const int rounds = (pos - first) / GROUPS + 1;                      // (the same for all lanes of a warp)
+    // the group of a key: its position mod ALL, wherever the window begins
+    int j = first - first % ALL + part * GROUPS + group;
+    if (j < first) j += ALL;
+    const int rounds = (pos - first) / ALL + 1;                         // (the same for all lanes of a warp)
     fetch(j);
     for (int round = 0; round < rounds; ++round) {
         ulonglong2 k[N], v[N];
         const bool there = base >= 0;
 #pragma unroll
         for (int i = 0; i < N; ++i) { k[i] = kn[i]; v[i] = vn[i]; }
-        j += GROUPS;
+        j += ALL;
         fetch(j);
 #pragma unroll
         for (int h = 0; h < HEADS; ++h) {
@@ -148,10 +156,9 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
         if (h >= count) break;
         const float top = warp_max(merge_m[h][lane]);                    // GROUPS == 32: a lane per group
         const float mine = merge_m[h][lane] == -INFINITY ? 0.f : expf(merge_m[h][lane] - top);
-        float total = warp_sum(merge_l[h][lane] * mine);
+        const float total = warp_sum(merge_l[h][lane] * mine);
         const float f = m[h] == -INFINITY ? 0.f : expf(m[h] - top);
-        if (a.sinks && total > 0.f) total += expf(a.sinks[h0 + h] - top);
-        const float inv = total > 0.f ? 1.f / total : 0.f;
+        if (tid == 0) { part_m[h] = top; part_l[h] = total; }
         __syncthreads();                                                 // the head before has been read
 #pragma unroll
         for (int i = 0; i < N; ++i) {
@@ -170,9 +177,26 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
             float s = 0.f;
 #pragma unroll
             for (int g = 0; g < GROUPS / 4; ++g) s += sums[g][d];
-            o[(size_t)h * a.head_dim + d] = s * inv;
+            part_v[h][d] = s;
         }
     }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    for (int i = part * F32_ATT_THREADS + tid; i < count * a.head_dim; i += F32_ATT_PARTS * F32_ATT_THREADS) {
+        const int h = i / a.head_dim, d = i - h * a.head_dim;
+        float pm[F32_ATT_PARTS], top = -INFINITY, total = 0.f, s = 0.f;
+#pragma unroll
+        for (int r = 0; r < F32_ATT_PARTS; ++r) { pm[r] = *cluster.map_shared_rank(&part_m[h], r); top = fmaxf(top, pm[r]); }
+#pragma unroll
+        for (int r = 0; r < F32_ATT_PARTS; ++r) {
+            const float f = pm[r] == -INFINITY ? 0.f : expf(pm[r] - top);
+            total += *cluster.map_shared_rank(&part_l[h], r) * f;
+            s += *cluster.map_shared_rank(&part_v[h][d], r) * f;
+        }
+        if (a.sinks && total > 0.f) total += expf(a.sinks[h0 + h] - top);
+        o[(size_t)h * a.head_dim + d] = s * (total > 0.f ? 1.f / total : 0.f);
+    }
+    cluster.sync();                                                      // nobody leaves while its sums are being read
 }
 
 // ---------------------------------------------------------------- rows of several tokens
@@ -347,9 +371,20 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_prompt_kernel(c
 }
 
 template <int D, int HEADS>
-static void launch_decode(const F32Rows& a, int rows, cudaStream_t s) {
+static int launch_decode(const F32Rows& a, int rows, cudaStream_t s) {
     const int per_kv = a.heads / a.kv_heads;
-    attention_f32_decode_kernel<D, HEADS><<<dim3(rows, a.kv_heads * ((per_kv + HEADS - 1) / HEADS)), F32_ATT_THREADS, 0, s>>>(a);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(F32_ATT_PARTS, rows, a.kv_heads * ((per_kv + HEADS - 1) / HEADS));
+    config.blockDim = dim3(F32_ATT_THREADS);
+    config.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = F32_ATT_PARTS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    config.attrs = attr;
+    config.numAttrs = 1;
+    HB_CUDA(cudaLaunchKernelEx(&config, attention_f32_decode_kernel<D, HEADS>, a));
+    return 0;
 }
 
 template <int D>
@@ -374,14 +409,13 @@ extern "C" int hb_attention_f32(float* out, const float* q, const float* kv, con
     F32Rows a = {out, q, kv, block_table, row_slot, query_start, kv_len, sinks,
                  table_stride, heads, kv_heads, head_dim, pages, page_size, window, scale};
     const int per_kv = heads / kv_heads;
+    if (n_decode > 65535) HB_REFUSE("attention_f32: %d rows of one token are above 65535", n_decode);
     if (n_decode > 0) {
-        if (head_dim <= 64) { if (per_kv == 1) launch_decode<64, 1>(a, n_decode, s); else launch_decode<64, 4>(a, n_decode, s); }
-        else if (head_dim <= 128) {
-            if (per_kv == 1) launch_decode<128, 1>(a, n_decode, s);
-            else if (per_kv == 2) launch_decode<128, 2>(a, n_decode, s);
-            else launch_decode<128, 4>(a, n_decode, s);
-        } else if (per_kv == 1) launch_decode<256, 1>(a, n_decode, s);
-        else launch_decode<256, 2>(a, n_decode, s);
+        const int rc = head_dim <= 64 ? (per_kv == 1 ? launch_decode<64, 1>(a, n_decode, s) : launch_decode<64, 4>(a, n_decode, s))
+                     : head_dim <= 128 ? (per_kv == 1 ? launch_decode<128, 1>(a, n_decode, s)
+                                          : per_kv == 2 ? launch_decode<128, 2>(a, n_decode, s) : launch_decode<128, 4>(a, n_decode, s))
+                     : per_kv == 1 ? launch_decode<256, 1>(a, n_decode, s) : launch_decode<256, 2>(a, n_decode, s);
+        if (rc) return rc;
     }
     if (rows > n_decode && tiles > 0) {
         const int rc = head_dim <= 64 ? launch_prompt<64>(a, n_decode, rows, tiles, s)

@@ -485,7 +485,7 @@ class CudaKernels:
         fast = q.dtype == torch.bfloat16 and head_dim % 16 == 0 and head_dim <= 256 and self.attention_bf16 == "fast"
         # (sizes, offsets and row lengths that the float32 kernels' 16-byte reads do not fit stay with the generic one)
         wide = q.dtype == torch.float32 and head_dim % 4 == 0 and head_dim <= 256 \
-            and not (q.data_ptr() | out.data_ptr() | kv.data_ptr()) % 16
+            and rows.n_decode <= 65535 and heads <= 65535 and not (q.data_ptr() | out.data_ptr() | kv.data_ptr()) % 16
         if not fast and not wide:
             return self._attention_generic(out, q, kv, block_table, rows, scale, window, sinks)
         kv_heads = kv.shape[2]
