@@ -726,3 +726,15 @@ def test_sample_follows_the_distribution(K):
         assert 0.5 * (counts - probs).abs().sum() < 0.12
         for i in range(0, n, 97):                                  # and token by token
             assert int(out[i]) == plain.draw(probs, plain.uniform(1234, i))
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 65, 2048), (300, 33, 96), (129, 255, 1000), (40, 1, 64), (40, 257, 64), (40, 64, 64)])
+def test_linear_of_an_odd_number_of_32_bit_columns(K, m, n, k):
+    """bfloat16 rows to 32-bit results whose rows are no multiple of 16 bytes (the first four), and their neighbours: 32-bit sums
+    of exact products."""
+    x, w = rand(m, k, dtype=torch.bfloat16, seed=n), rand(n, k, dtype=torch.bfloat16, seed=k)
+    out = torch.full((m, n), float("nan"), device=DEV)
+    K.linear(out, x.to(DEV), w.to(DEV))
+    want = x.double() @ w.double().T
+    assert K.tcgen05_status() == 0
+    assert (out.cpu() - want).abs().max().item() <= 2 ** -22 * k
