@@ -1,6 +1,6 @@
 // out[m, n] = sum_k x[m, k] * w[n, k] in true 32-bit on CUDA cores: no tensor cores, no reduced-precision mode.
 // One order of summation for every output element, a function of k alone: k is cut into up to eight segments of equal
-// length (a multiple of 16), each summed in ascending order with fused multiply-adds, and the segments' sums are added in
+// length (a multiple of 16, at least 64), each summed in ascending order with fused multiply-adds, and the segments' sums are added in
 // ascending order. So a row's result does not depend on how many other rows the batch holds, nor on which of the kernels
 // and splits below computed it (and eight shorter sums lose less than one long one).
 #include <cooperative_groups.h>
@@ -13,9 +13,11 @@ namespace cg = cooperative_groups;
 #define BN 128
 #define BK 16
 #define SEGMENTS 8
+#define SHORTEST 64                         // terms a segment holds at least: one piece of the kernel for few rows (shorter sums gain nothing)
 
 static __host__ __device__ inline int segment_length(int k) {
-    return ((k + SEGMENTS - 1) / SEGMENTS + BK - 1) / BK * BK;
+    const int share = ((k + SEGMENTS - 1) / SEGMENTS + BK - 1) / BK * BK;
+    return share > SHORTEST ? share : SHORTEST;
 }
 
 // Two 32-bit multiply-adds in one instruction; each rounds as fmaf does.

@@ -20,7 +20,7 @@ def K():
     return load_kernels(torch.device(DEV))
 
 
-# k: one segment, a remainder in the last of eight, segments of 64 + 16, no multiple of 4; n: a cluster of eight, of four
+# k: one segment, two, a remainder in the last of eight, segments of 64 and of 80, no multiple of 4; n: a cluster of eight, of four
 # and no cluster at 65 rows (1, 33 to 120 and more tiles of 64 x 128)
 @pytest.mark.parametrize("k", [4, 16, 60, 128, 132, 636, 1030, 3072])
 @pytest.mark.parametrize("n", [7, 130, 2200, 9000])
