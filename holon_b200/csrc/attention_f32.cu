@@ -12,6 +12,7 @@
 // average over both.
 // Which groups or tiles a key falls into depends on its position alone, so a token's result does not depend on the rows
 // beside it nor on where its prompt was cut.
+// A key that scores minus infinity (its product with the query overflowed) weighs nothing; a query whose keys all do has no answer: NaN.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -62,6 +63,7 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
     __shared__ float merge_m[HEADS][GROUPS], merge_l[HEADS][GROUPS];
     __shared__ __align__(16) float sums[GROUPS / 4][D];
     __shared__ float part_m[HEADS], part_l[HEADS], part_v[HEADS][D];
+    __shared__ int part_seen;                                            // whether this block met a key at all
     const int per_kv = a.heads / a.kv_heads, chunks = (per_kv + HEADS - 1) / HEADS;
     const int b = blockIdx.y, part = blockIdx.x, hk = blockIdx.z / chunks, h0 = hk * per_kv + blockIdx.z % chunks * HEADS;
     const int count = min(HEADS, (hk + 1) * per_kv - h0);
@@ -110,10 +112,12 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
     int j = first - first % ALL + part * GROUPS + group;
     if (j < first) j += ALL;
     const int rounds = (pos - first) / ALL + 1;                         // (the same for all lanes of a warp)
+    bool seen = false;
     fetch(j);
     for (int round = 0; round < rounds; ++round) {
         ulonglong2 k[N], v[N];
         const bool there = base >= 0;
+        seen |= there;
 #pragma unroll
         for (int i = 0; i < N; ++i) { k[i] = kn[i]; v[i] = vn[i]; }
         j += ALL;
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
             s += __shfl_xor_sync(0xffffffffu, s, 4);
             if (!there) continue;
             const float m_new = fmaxf(m[h], s);
-            const float corr = m_new == -INFINITY ? 1.f : expf(m[h] - m_new), p = expf(s - m_new);
+            const float corr = m_new == -INFINITY ? 1.f : expf(m[h] - m_new), p = expf(s - (m_new == -INFINITY ? 0.f : m_new));
             l[h] = l[h] * corr + p;
             m[h] = m_new;
             const uint64_t cc = pair(corr, corr), pp = pair(p, p);
@@ -150,7 +154,8 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
     if (sub == 0)
 #pragma unroll
         for (int h = 0; h < HEADS; ++h) { merge_m[h][group] = m[h]; merge_l[h][group] = l[h]; }
-    __syncthreads();
+    const int any = __syncthreads_or(seen);
+    if (tid == 0) part_seen = any;
 #pragma unroll
     for (int h = 0; h < HEADS; ++h) {
         if (h >= count) break;
@@ -194,7 +199,13 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_decode_kernel(c
             s += *cluster.map_shared_rank(&part_v[h][d], r) * f;
         }
         if (a.sinks && total > 0.f) total += expf(a.sinks[h0 + h] - top);
-        o[(size_t)h * a.head_dim + d] = s * (total > 0.f ? 1.f / total : 0.f);
+        float inv = 1.f / total;
+        if (!(total > 0.f)) {
+            int met = 0;
+            for (int r = 0; r < F32_ATT_PARTS; ++r) met |= *cluster.map_shared_rank(&part_seen, r);
+            inv = met ? NAN : 0.f;
+        }
+        o[(size_t)h * a.head_dim + d] = s * inv;
     }
     cluster.sync();                                                      // nobody leaves while its sums are being read
 }
@@ -237,6 +248,7 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_prompt_kernel(c
 #pragma unroll
         for (int c = 0; c < 2 * COLS; ++c) acc[i][c] = 0;
     }
+    unsigned met = 0;                                                    // bit i: query i met one of this thread's keys
     const int last = n > 0 ? pos0 + queries - 1 : -1;                    // the last key any of these queries sees
     const int first = a.window > 0 ? max(0, pos0 - a.window + 1) : 0;
     for (int j0 = first - first % T; j0 <= last; j0 += T) {
@@ -286,16 +298,17 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_prompt_kernel(c
                 seen[c] = j <= pos && (a.window <= 0 || pos - j < a.window) && bases[tx + 16 * c] >= 0;
                 const float2 d2 = halves(dots[i][c]);
                 s[c] = seen[c] ? d2.x + d2.y : -INFINITY;
+                if (seen[c]) met |= 1u << i;
                 top = fmaxf(top, s[c]);
             }
 #pragma unroll
             for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
             const float m_new = fmaxf(m[i], top);
-            const float corr = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);
+            const float corr = m_new == -INFINITY ? 1.f : expf(m[i] - m_new), ref = m_new == -INFINITY ? 0.f : m_new;
             float sum = 0.f;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const float p = seen[c] ? expf(s[c] - m_new) : 0.f;
+                const float p = expf(s[c] - ref);                        // (0 for what is not seen)
                 ps[(ty * 4 + i) * (T + 4) + tx + 16 * c] = p;
                 sum += p;
             }
@@ -356,9 +369,10 @@ __global__ void __launch_bounds__(F32_ATT_THREADS) attention_f32_prompt_kernel(c
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int r = ty * 4 + i;
+        const unsigned both = __ballot_sync(0xffffffffu, met >> i & 1);  // of the two queries whose lanes share this warp
         if (r >= queries) continue;
         if (a.sinks && l[i] > 0.f) l[i] += expf(a.sinks[h] - m[i]);
-        const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+        const float inv = l[i] > 0.f ? 1.f / l[i] : both >> (tid & 16) & 0xffff ? NAN : 0.f;
         float* o = a.out + ((size_t)(t0 + r) * a.heads + h) * a.head_dim;
 #pragma unroll
         for (int c = 0; c < COLS; ++c) {

@@ -102,3 +102,41 @@ def test_attention_float32_leaves_out_what_is_not_seen(K, bad):
         out.append(o)
     assert torch.equal(out[0][:89], out[1][:89]) and torch.equal(out[0][90:], out[1][90:])
     assert not out[1][89].isfinite().any()
+
+
+def plain_attention(q, kv, table, rows, scale, window):
+    """In 64 bits, except that a score that overflows in 32 bits is minus infinity."""
+    out = torch.zeros_like(q, dtype=torch.float64)
+    group = q.shape[1] // kv.shape[2]
+    for b in range(rows.n_rows):
+        t0, n = int(rows.query_start[b]), int(rows.kv_len[b])
+        j = torch.arange(n)
+        k, v = (kv[table[rows.row_slot[b], j // kv.shape[3]].long(), i, :, j % kv.shape[3]].double() for i in (0, 1))
+        for t in range(t0, int(rows.query_start[b + 1])):
+            pos = n - int(rows.query_start[b + 1]) + t
+            lo = max(0, pos - window + 1) if window else 0
+            for h in range(q.shape[1]):
+                s = k[lo:pos + 1, h // group] @ (q[t, h].double() * scale)
+                out[t, h] = torch.softmax(s.float().double(), 0) @ v[lo:pos + 1, h // group]
+    return out
+
+
+@pytest.mark.parametrize("window", [0, 1, 2, 70])
+def test_attention_float32_scores_of_minus_infinity(K, window):
+    """Keys whose product with the query overflows weigh nothing, wherever they stand among a tile's or a group's keys; a query that
+    sees no other key has no answer. (In 64 bits as in 32: the weights of the rest are not touched.)"""
+    heads, kv_heads, head_dim, page = 4, 2, 64, 16
+    spec = [(332, 1), (40, 1), (0, 200), (63, 5)]
+    q, kv, table, rows = paged_case(heads, kv_heads, head_dim, page, spec, torch.float32, seed=11)
+    q[..., 0] = 8.0
+    for b, (before, new) in enumerate(spec):
+        for j in (0, 5, 63, 64, 127, 199, 331, 332):
+            if j < before + new:
+                kv[table[rows.row_slot[b], j // page], 0, :, j % page, 0] = -3e38
+    want = plain_attention(q, kv, table, rows, 1.0, window)
+    assert window != 1 or want.isnan().any()
+    out = torch.full_like(q, float("nan"), device=DEV)
+    K.paged_attention(out, q.to(DEV), kv.to(DEV), table.to(DEV), on_device(rows), 1.0, window)
+    assert torch.equal(out.isnan().cpu(), want.isnan())
+    # scores of up to 30 in size are off by up to 2^-24 of that times a few roundings, and so are the weights
+    assert (out.cpu() - want).nan_to_num().abs().max().item() <= 1e-4
