@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tcgen05_kernel(
         if (ok) {                                                             // (the tensor-memory loads are warp-collective: no lane skips them)
             if (sinks && l > 0.f) l += at_ex2(fmaf(sinks[(flat0 + r) % heads], 1.4426950408889634f, -m_used));
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            const bool keep = tiles > 0 && l > 0.f, mine = r < rows_here;
+            const bool keep = tiles > 0 && l != 0.f, mine = r < rows_here;   // (a sum that is no number leaves none: O is none then, too)
             bf16* o_row = out + (size_t)(flat_global + (mine ? r : 0)) * rank + v0 * 64;
             for (int c = 0; c < 2 * nv; ++c) {
                 uint32_t o[32];

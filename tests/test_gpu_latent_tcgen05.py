@@ -57,3 +57,36 @@ def test_portions(K, heads, rank, rot, page, window, sink):
 def test_sizes_that_stay_with_the_other_kernel(K):
     for heads, rank, rot, pages, page in [(4, 80, 16, 9, 64), (4, 512, 0, 9, 64), (4, 320, 32, 9, 64), (4, 64, 32, 9, 32), (4, 512, 256, 9, 64)]:
         assert not K._latent_tcgen05_takes(heads, rank, rot, pages, page)
+
+
+def small_case(heads=16, rank=512, rot=64, page=64):
+    new, lens, dk = [70, 5, 40], [170, 133, 40], rank + rot
+    cache = rand(9, page, dk, dtype=torch.bfloat16, seed=1)
+    table = torch.tensor([[3, 1, 6], [0, 4, 7], [5, 8, 8]], dtype=torch.int32)
+    qs = torch.tensor([0] + new, dtype=torch.int32).cumsum(0).to(torch.int32)
+    host = Rows(torch.arange(3, dtype=torch.int32), qs, torch.tensor(lens, dtype=torch.int32), 3, sum(new), 0, max(new), max(lens))
+    return rand(sum(new), heads, dk, dtype=torch.bfloat16, seed=2, scale=3.0), cache, table, host
+
+
+def latent(K, qa, cache, table, host, rank=512, scale=0.04, window=0, sinks=None):
+    out = torch.full((qa.shape[0], qa.shape[1], rank), 7.0, dtype=torch.bfloat16, device=DEV)
+    assert K._latent_tcgen05_takes(qa.shape[1], rank, qa.shape[2] - rank, cache.shape[0], cache.shape[1])
+    K.latent_attention(out, qa.to(DEV), cache.to(DEV), table.to(DEV), on_device(host), scale, rank, window, sinks=sinks)
+    assert K.tcgen05_status() == 0
+    return out.cpu()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("column", [0, 300, 560])
+@pytest.mark.parametrize("sink", [False, True])
+def test_what_is_no_number_stays_none(K, bad, column, sink):
+    """A cached number of the second row's context that is none: every query of that row sees it and has no answer (and not zeros);
+    the other rows keep their bits."""
+    qa, cache, table, host = small_case()
+    qa[..., column] = qa[..., column].abs() + 1.0                     # (an infinity then scores one: a weight without bounds)
+    sinks = rand(16, seed=5).to(DEV) if sink else None
+    clean = latent(K, qa, cache, table, host, sinks=sinks)
+    cache[4, 10, column] = bad
+    out = latent(K, qa, cache, table, host, sinks=sinks)
+    assert out[70:75].isnan().all() and clean.isfinite().all()
+    assert torch.equal(out[:70], clean[:70]) and torch.equal(out[75:], clean[75:])
