@@ -103,9 +103,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tcgen05_kernel(
                 const int s = j % stages;
                 const uint32_t parity = ((j / stages) & 1) ^ 1, dst = kv_s + s * stage_bytes;
                 const int key0 = (tile_lo + j) * LT_BN;
-                int page = table[key0 / page_size];
-                page = page < 0 || page >= pages ? 0 : page;
-                const int row = page * page_size + key0 % page_size;          // of the flattened cache
+                const int page = table[key0 / page_size];
+                // of the flattened cache; a page that is none: past its end, where a load reads zeros
+                const int row = page < 0 || page >= pages ? pages * page_size : page * page_size + key0 % page_size;
                 if (!mbar_wait(a_empty0 + 8 * s, parity, 1)) break;
                 mbar_expect_tx(a_full0 + 8 * s, (blocks - nv) * LT_K_BLOCK);
                 for (int i = 0; i < blocks; ++i)

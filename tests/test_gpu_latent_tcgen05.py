@@ -90,3 +90,14 @@ def test_what_is_no_number_stays_none(K, bad, column, sink):
     out = latent(K, qa, cache, table, host, sinks=sinks)
     assert out[70:75].isnan().all() and clean.isfinite().all()
     assert torch.equal(out[:70], clean[:70]) and torch.equal(out[75:], clean[75:])
+
+
+def test_a_page_that_the_table_does_not_name(K):
+    """Reads as rows of zeros, as in the other kernel."""
+    qa, cache, table, host = small_case()
+    cache[8] = 0
+    table[1, 0] = 8
+    want = latent(K, qa, cache, table, host)
+    for nowhere in (-1, 9, 1 << 30):
+        table[1, 0] = nowhere
+        assert torch.equal(latent(K, qa, cache, table, host), want), nowhere
