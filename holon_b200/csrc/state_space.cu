@@ -40,17 +40,21 @@ __device__ __forceinline__ Chunk find_chunk(const int32_t* __restrict__ query_st
 // permuted by k / 4, so that stores of four k's of one i by eight neighbouring lanes, and of four i's by four, hit different banks.
 __device__ __forceinline__ int group_at(int k, int g) { return k * (SS_T / 4) + (g ^ ((k >> 2) & 7)); }
 
-// total += a^T b over a slice, 16 steps of k to a sum of their own: one sum over all steps loses twice as much (an output's error
-// against 64 bits 2.5e-7 in place of 1.3e-7, the token-by-token scan's 1.0 to 2.1e-7 for decays of 0.875 to 0.984).
+enum Form { STATE_SPACE, FIXED, TOKEN };                   // where decays come from: dt and rate_log; head_decay in rate_log's place; token_decay in dt's
+
+// total += a^T b over a slice. FIXED and TOKEN: 16 steps of k to a sum of their own, since one sum over all steps loses twice as much
+// (an output's error against 64 bits 2.5e-7 in place of 1.3e-7, the token-by-token scan's 1.0 to 2.1e-7 for decays of 0.875 to 0.984).
+// That takes a second set of sums and so three CTAs an SM in place of four; the state space, whose only form for prompts this is, keeps
+// one sum and four (2,048 tokens, 32 heads of 64 over a state of 128: 108 us, 129 us with the sums in parts).
+#define SS_CTAS(FORM) ((FORM) == STATE_SPACE ? 4 : 3)
+template <int FORM>
 __device__ __forceinline__ void tile_step(float (&total)[8][4], const float* a, const float* b, int depth) {
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const float4* a4 = (const float4*)a;
     const float4* b4 = (const float4*)b;
-    for (int k0 = 0; k0 < depth; k0 += 16) {
-        float acc[8][4] = {};
-        const int end = min(depth, k0 + 16);
+    auto steps = [&](float (&acc)[8][4], int from, int to) {
 #pragma unroll 8
-        for (int k = k0; k < end; ++k) {
+        for (int k = from; k < to; ++k) {
             const float4 r0 = a4[group_at(k, ty * 2)], r1 = a4[group_at(k, ty * 2 + 1)], c = b4[group_at(k, tx)];
             const float r[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
 #pragma unroll
@@ -59,11 +63,17 @@ __device__ __forceinline__ void tile_step(float (&total)[8][4], const float* a, 
                 acc[i][2] = fmaf(r[i], c.z, acc[i][2]); acc[i][3] = fmaf(r[i], c.w, acc[i][3]);
             }
         }
+    };
+    if constexpr (FORM == STATE_SPACE) steps(total, 0, depth);
+    else
+        for (int k0 = 0; k0 < depth; k0 += 16) {
+            float acc[8][4] = {};
+            steps(acc, k0, min(depth, k0 + 16));
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) total[i][j] += acc[i][j];
-    }
+                for (int j = 0; j < 4; ++j) total[i][j] += acc[i][j];
+        }
 }
 
 // Slices travel through registers (the next one is on its way while the current one is multiplied), 16 bytes a load: four quads a
@@ -99,8 +109,6 @@ __device__ __forceinline__ void store_across(float* a, const Quads& q) {
     for (int r = 0; r < 4; ++r) ((float4*)a)[group_at(k + 8 * r, threadIdx.x & 15)] = q.v[r];
 }
 __device__ __forceinline__ void scale_quad(float4& v, float f) { v.x *= f; v.y *= f; v.z *= f; v.w *= f; }
-
-enum Form { STATE_SPACE, FIXED, TOKEN };                   // where decays come from: dt and rate_log; head_decay in rate_log's place; token_decay in dt's
 
 // L_i of a chunk's tokens for one head, by warp 0: hi + lo in two floats; tokens past the chunk repeat the last. sign: of the decays'
 // product up to i (not for STATE_SPACE).
@@ -146,7 +154,8 @@ __device__ __forceinline__ void log_decays(float* hi, float* lo, float* steps, f
 }
 
 // ---- products[tile][group][i][j] = C_i . B_j, [64][64] each. grid (tiles, groups)
-__global__ void __launch_bounds__(SS_THREADS, 3) ss_products_kernel(float* __restrict__ products, const float* __restrict__ cb,
+template <int FORM>
+__global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_products_kernel(float* __restrict__ products, const float* __restrict__ cb,
                                                                  const int32_t* __restrict__ query_start, int row0, int rows, int groups, int n) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
     const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
@@ -167,7 +176,7 @@ __global__ void __launch_bounds__(SS_THREADS, 3) ss_products_kernel(float* __res
             fetch_along(qa, src + k0 + SS_K, stride, c.n, n - k0 - SS_K, vec);
             fetch_along(qb, src + (size_t)groups * n + k0 + SS_K, stride, c.n, n - k0 - SS_K, vec);
         }
-        tile_step(acc, a, b, min(SS_K, n - k0));
+        tile_step<FORM>(acc, a, b, min(SS_K, n - k0));
         __syncthreads();
     }
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
@@ -179,7 +188,7 @@ __global__ void __launch_bounds__(SS_THREADS, 3) ss_products_kernel(float* __res
 // ---- own[tile][head][p][n] = sum_j exp(L_last - L_j) dt_j x_j[p] B_j[n]; last[tile][head] = exp(L_last). grid (tiles, heads, tiles of
 // p times tiles of n)
 template <int FORM>
-__global__ void __launch_bounds__(SS_THREADS, 3) ss_own_kernel(float* __restrict__ own, float* __restrict__ last, const float* __restrict__ cb,
+__global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_own_kernel(float* __restrict__ own, float* __restrict__ last, const float* __restrict__ cb,
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const int32_t* __restrict__ query_start,
                                                             int row0, int rows, int heads, int groups, int n, int vdim, int n_tiles) {
@@ -217,7 +226,7 @@ __global__ void __launch_bounds__(SS_THREADS, 3) ss_own_kernel(float* __restrict
             fetch_across(qa, xp + (k0 + SS_K) * xs, xs, vdim - p0, c.n - k0 - SS_K, vx);
             fetch_across(qb, bp + (k0 + SS_K) * bs, bs, n - n0, c.n - k0 - SS_K, vb);
         }
-        tile_step(acc, a, b, min(SS_K, c.n - k0));
+        tile_step<FORM>(acc, a, b, min(SS_K, c.n - k0));
         __syncthreads();
     }
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
@@ -272,7 +281,7 @@ __global__ void ss_walk_kernel(float* __restrict__ own, const float* __restrict_
 
 // ---- y_i[p] of a chunk: the products' part over its own tokens, the state's part over n, the skip. grid (tiles, heads, tiles of p)
 template <int FORM>
-__global__ void __launch_bounds__(SS_THREADS, 3) ss_out_kernel(float* __restrict__ y, const float* __restrict__ products,
+__global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_out_kernel(float* __restrict__ y, const float* __restrict__ products,
                                                             const float* __restrict__ before, const float* __restrict__ cb,
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const float* __restrict__ skip,
@@ -328,12 +337,14 @@ __global__ void __launch_bounds__(SS_THREADS, 3) ss_out_kernel(float* __restrict
                 qa.v[r].x = weight(j, qa.v[r].x); qa.v[r].y = weight(j + 1, qa.v[r].y);
                 qa.v[r].z = weight(j + 2, qa.v[r].z); qa.v[r].w = weight(j + 3, qa.v[r].w);
                 float* x4 = &qb.v[r].x;                             // (a weight of zero would make a NaN of an infinity in an earlier row)
+                if (!(fabsf(x4[0]) + fabsf(x4[1]) + fabsf(x4[2]) + fabsf(x4[3]) < INFINITY)) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (!isfinite(x4[e])) {
-                        atomicMin(&bad[((int)threadIdx.x & 15) * 4 + e], s * SS_K + ((int)threadIdx.x >> 4) + 8 * r);
-                        x4[e] = 0.f;
-                    }
+                    for (int e = 0; e < 4; ++e)
+                        if (!isfinite(x4[e])) {
+                            atomicMin(&bad[((int)threadIdx.x & 15) * 4 + e], s * SS_K + ((int)threadIdx.x >> 4) + 8 * r);
+                            x4[e] = 0.f;
+                        }
+                }
             }
         } else {
 #pragma unroll
@@ -344,7 +355,7 @@ __global__ void __launch_bounds__(SS_THREADS, 3) ss_out_kernel(float* __restrict
         __syncthreads();
         if (s + 1 < slices) fetch(s + 1);
         // (the second half of a chunk's tokens weighs nothing in its first half's rows)
-        if (s >= own_slices || s == 0 || (int)(threadIdx.x >> 5) * 16 + 15 >= s * SS_K) tile_step(acc, a, b, SS_K);
+        if (s >= own_slices || s == 0 || (int)(threadIdx.x >> 5) * 16 + 15 >= s * SS_K) tile_step<FORM>(acc, a, b, SS_K);
         __syncthreads();
     }
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
@@ -381,7 +392,7 @@ static int run_chunks(const char* what, float* y, const float* cb, const float* 
     float* own = products + (size_t)tiles * groups * SS_Q * SS_Q;  // [tiles][heads][vdim][n]
     float* last = own + (size_t)tiles * heads * size;              // [tiles][heads]
     cudaStream_t s = (cudaStream_t)stream;
-    ss_products_kernel<<<dim3(tiles, groups), SS_THREADS, 0, s>>>(products, cb, query_start, row0, rows, groups, n);
+    ss_products_kernel<FORM><<<dim3(tiles, groups), SS_THREADS, 0, s>>>(products, cb, query_start, row0, rows, groups, n);
     HB_LAUNCH_CHECK("state_space_products");
     ss_own_kernel<FORM><<<dim3(tiles, heads, p_tiles * n_tiles), SS_THREADS, 0, s>>>(own, last, cb, x, dt, rate_log, query_start, row0, rows, heads,
                                                                                groups, n, vdim, n_tiles);

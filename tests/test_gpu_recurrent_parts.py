@@ -106,3 +106,24 @@ def test_what_is_no_number_reaches_no_earlier_token(K, form):
     for out, state, where in ((*run(qk, bad_v), (slice(37, None), 1, 5)), (*run(bad_k, v), (slice(38, None), 1))):
         assert torch.equal(out[:37], clean[:37]) and torch.equal(out[:, 0], clean[:, 0])
         assert not out[where].isfinite().any() and not state[0, 1].isfinite().all()
+
+
+def test_a_state_space_value_that_is_no_number_reaches_no_earlier_token(K):
+    t, heads, groups, n, vdim = 220, 4, 2, 64, 64
+    g = torch.Generator(device=DEV).manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)                           # noqa: E731
+    cb, v, dt, rate, skip = r(t, 2, groups, n), r(t, heads, vdim), torch.rand(t, heads, generator=g, device=DEV), r(heads), r(heads)
+    decay, starts = torch.exp(-rate.exp() * dt), torch.tensor([0, t], dtype=torch.int32, device=DEV)
+    rows = Rows(starts[:1], starts, starts[1:], 1, t, 0, t, t, [0, t], [t])
+    outs = []
+    for bad in (None, float("inf"), float("nan")):
+        if bad is not None:
+            v[37, 1, 5] = bad
+        out, state = torch.empty_like(v), torch.zeros(2, heads, vdim, n, device=DEV)
+        K.state_space_scan(out, cb, v, dt, decay, rate, skip, state, rows)
+        outs.append(out)
+    for out in outs[1:]:
+        assert torch.equal(out[:37], outs[0][:37]) and not out[37:, 1, 5].isfinite().any()
+        kept = torch.ones_like(out, dtype=torch.bool)
+        kept[37:, 1, 5] = False
+        assert torch.equal(out[kept], outs[0][kept])
