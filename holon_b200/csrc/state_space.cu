@@ -80,6 +80,10 @@ __device__ __forceinline__ void tile_step(float (&total)[8][4], const float* a, 
 // thread and operand. `along`: the operand's memory runs along k (element (row i, k) at p[i * stride + k]); eight neighbouring lanes
 // load 128 bytes of one row. `across`: it runs along the tile's rows (element (k, i) at p[k * stride + i]).
 struct Quads { float4 v[4]; };
+// Which of x (1) and C, B (2) can be read 16 bytes at a time: rows of whole quads that begin on a 16-byte boundary.
+static int in_quads(const float* x, int vdim, const float* cb, int n) {
+    return (vdim % 4 == 0 && (uintptr_t)x % 16 == 0 ? 1 : 0) | (n % 4 == 0 && (uintptr_t)cb % 16 == 0 ? 2 : 0);
+}
 __device__ __forceinline__ float4 load_quad(const float* p, int left, bool vec) {        // zeros from `left` on
     if (vec && left >= 4) return *(const float4*)p;
     return make_float4(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
@@ -156,7 +160,7 @@ __device__ __forceinline__ void log_decays(float* hi, float* lo, float* steps, f
 // ---- products[tile][group][i][j] = C_i . B_j, [64][64] each. grid (tiles, groups)
 template <int FORM>
 __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_products_kernel(float* __restrict__ products, const float* __restrict__ cb,
-                                                                 const int32_t* __restrict__ query_start, int row0, int rows, int groups, int n) {
+                                                                 const int32_t* __restrict__ query_start, int row0, int rows, int groups, int n, int quads) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
     const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
     if (c.row < 0) return;
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_products_kernel(
     Quads qa, qb;
     const float* src = cb + ((size_t)c.t0 * 2 * groups + g) * n;
     const size_t stride = (size_t)2 * groups * n;
-    const bool vec = (n & 3) == 0;
+    const bool vec = quads & 2;
     fetch_along(qa, src, stride, c.n, n, vec);
     fetch_along(qb, src + (size_t)groups * n, stride, c.n, n, vec);
     for (int k0 = 0; k0 < n; k0 += SS_K) {
@@ -191,7 +195,7 @@ template <int FORM>
 __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_own_kernel(float* __restrict__ own, float* __restrict__ last, const float* __restrict__ cb,
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const int32_t* __restrict__ query_start,
-                                                            int row0, int rows, int heads, int groups, int n, int vdim, int n_tiles) {
+                                                            int row0, int rows, int heads, int groups, int n, int vdim, int n_tiles, int quads) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
     __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q], sign[FORM == STATE_SPACE ? 1 : SS_Q];
     const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_own_kernel(float
     const size_t xs = (size_t)heads * vdim, bs = (size_t)2 * groups * n;
     const float* xp = x + ((size_t)c.t0 * heads + h) * vdim + p0;
     const float* bp = cb + (((size_t)c.t0 * 2 + 1) * groups + g) * n + n0;
-    const bool vx = (vdim & 3) == 0, vb = (n & 3) == 0;
+    const bool vx = quads & 1, vb = quads & 2;
     fetch_across(qa, xp, xs, vdim - p0, c.n, vx);                   // (on its way while the decays are added up)
     fetch_across(qb, bp, bs, n - n0, c.n, vb);
     log_decays<FORM>(hi, lo, steps, sign, dt, c, heads, h, rate_log);
@@ -286,7 +290,7 @@ __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_out_kernel(float
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const float* __restrict__ skip,
                                                             const int32_t* __restrict__ query_start, int row0, int rows, int heads,
-                                                            int groups, int n, int vdim) {
+                                                            int groups, int n, int vdim, int quads) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
     __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q], sign[FORM == STATE_SPACE ? 1 : SS_Q];
     __shared__ int bad[SS_T];                                       // per column: the first token whose value is no finite number
@@ -298,7 +302,7 @@ __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_out_kernel(float
     const float* cp = cb + ((size_t)c.t0 * 2 * groups + g) * n;
     const float* sp = before + (((size_t)blockIdx.x * heads + h) * vdim + p0) * n;
     const size_t xs = (size_t)heads * vdim, cs = (size_t)2 * groups * n;
-    const bool vx = (vdim & 3) == 0, vn = (n & 3) == 0;
+    const bool vx = quads & 1, vn = quads & 2;                      // (the state's rows are read as C's are)
     const int own_slices = (c.n + SS_K - 1) / SS_K, slices = own_slices + (n + SS_K - 1) / SS_K;
     Quads qa, qb;
     auto fetch = [&](int s) {
@@ -387,15 +391,15 @@ static int run_chunks(const char* what, float* y, const float* cb, const float* 
     if (!scratch || ((uintptr_t)scratch & 15) || ((uintptr_t)state & 15)) HB_REFUSE("%s: scratch and state must lie on 16-byte boundaries", what);
     const int p_tiles = (vdim + SS_T - 1) / SS_T, n_tiles = (n + SS_T - 1) / SS_T;
     if (heads > 65535 || (long)p_tiles * n_tiles > 65535) HB_REFUSE("%s: %d heads of %d x %d", what, heads, vdim, n);
-    const int size = vdim * n;
+    const int size = vdim * n, quads = in_quads(x, vdim, cb, n);
     float* products = scratch;                                     // [tiles][groups][64][64]
     float* own = products + (size_t)tiles * groups * SS_Q * SS_Q;  // [tiles][heads][vdim][n]
     float* last = own + (size_t)tiles * heads * size;              // [tiles][heads]
     cudaStream_t s = (cudaStream_t)stream;
-    ss_products_kernel<FORM><<<dim3(tiles, groups), SS_THREADS, 0, s>>>(products, cb, query_start, row0, rows, groups, n);
+    ss_products_kernel<FORM><<<dim3(tiles, groups), SS_THREADS, 0, s>>>(products, cb, query_start, row0, rows, groups, n, quads);
     HB_LAUNCH_CHECK("state_space_products");
     ss_own_kernel<FORM><<<dim3(tiles, heads, p_tiles * n_tiles), SS_THREADS, 0, s>>>(own, last, cb, x, dt, rate_log, query_start, row0, rows, heads,
-                                                                               groups, n, vdim, n_tiles);
+                                                                               groups, n, vdim, n_tiles, quads);
     HB_LAUNCH_CHECK("state_space_own");
     const bool vec = size % 4 == 0;
     const int elements = vec ? size / 4 : size, slices = (elements + 127) / 128;
@@ -404,7 +408,7 @@ static int run_chunks(const char* what, float* y, const float* cb, const float* 
     else ss_walk_kernel<false><<<dim3(rows - row0, heads, slices), 128, 0, s>>>(own, last, state, query_start, row_slot, row0, heads, size);
     HB_LAUNCH_CHECK("state_space_walk");
     ss_out_kernel<FORM><<<dim3(tiles, heads, p_tiles), SS_THREADS, 0, s>>>(y, products, own, cb, x, dt, rate_log, skip, query_start, row0, rows, heads,
-                                                                     groups, n, vdim);
+                                                                     groups, n, vdim, quads);
     HB_LAUNCH_CHECK("state_space_out");
     return 0;
 }

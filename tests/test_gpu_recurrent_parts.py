@@ -127,3 +127,35 @@ def test_a_state_space_value_that_is_no_number_reaches_no_earlier_token(K):
         kept = torch.ones_like(out, dtype=torch.bool)
         kept[37:, 1, 5] = False
         assert torch.equal(out[kept], outs[0][kept])
+
+
+def off_by(x, floats):
+    """x at an address that many floats behind a 16-byte boundary."""
+    y = torch.empty(x.numel() + floats, device=x.device)[floats:].view(x.shape)
+    assert y.data_ptr() % 16 == 4 * floats and y.is_contiguous()
+    return y.copy_(x)
+
+
+@pytest.mark.parametrize("form", ["fixed", "token", "delta", "general", "state space"])
+@pytest.mark.parametrize("vdim", [64, 7])
+def test_values_anywhere_in_memory(K, form, vdim):
+    """v (and a state space's C and B) need no 16-byte boundary: the same bits as on one."""
+    t, heads, dim = 220, 4, 64
+    g = torch.Generator(device=DEV).manual_seed(2)
+    qk = torch.nn.functional.normalize(torch.randn(t, 2, heads, dim, generator=g, device=DEV), dim=-1)
+    v, decay = torch.randn(t, heads, vdim, generator=g, device=DEV), 1 - torch.rand(t, heads, dim, generator=g, device=DEV) * 0.1
+    beta, rate = torch.rand(t, heads, generator=g, device=DEV), torch.rand(t, heads, dim, generator=g, device=DEV)
+    starts = torch.tensor([0, t], dtype=torch.int32, device=DEV)
+    rows = Rows(starts[:1], starts, starts[1:], 1, t, 0, t, t, [0, t], [t])
+    outs = []
+    for floats in (0, 1, 2):
+        out, state, values = torch.empty_like(v), torch.zeros(2, heads, vdim, dim, device=DEV), off_by(v, floats)
+        if form == "state space":
+            K.state_space_scan(out, off_by(qk, floats), values, beta, torch.exp(-beta), torch.zeros(heads, device=DEV), beta[0].clone(), state, rows)
+        else:
+            K.recurrent_scan(out, qk, values, decay if form in ("delta", "general") else None, decay[0, :, 0].contiguous() if form == "fixed" else None,
+                             beta if form == "delta" else None, state, rows, token_decay=decay[:, :, 0].contiguous() if form == "token" else None,
+                             rate=rate if form == "general" else None)
+        outs.append((out, state))
+    for out, state in outs[1:]:
+        assert torch.equal(out, outs[0][0]) and torch.equal(state, outs[0][1])
