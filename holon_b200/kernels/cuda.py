@@ -1229,19 +1229,20 @@ class CudaKernels:
                 or (take is not None and take.shape != (t, heads)) or (skip is not None and skip.shape != (heads,)):
             raise KernelError("recurrent_scan: qk [tokens, 2, kv_heads, dim], v and out [tokens, heads, vdim], state "
                               "[slots, heads, vdim, dim], decay [tokens, heads, dim] or head_decay [heads], beta [tokens, heads]")
-        # Rows of many tokens: in chunks of 64 where the decay is one number per head, with a delta rule eight tokens at a time.
-        # What the launches depend on are counts of rows and tokens, so that they can be captured.
+        # Rows of many tokens: in chunks of 64 where the decay is one number per head, with a delta rule eight tokens at a time (what else
+        # was given goes to the scan, which takes or refuses it). What the launches depend on are counts of rows and tokens, so that they
+        # can be captured.
         scanned, ones, portions = rows.n_rows, rows.n_decode, rows.n_rows - rows.n_decode
         more = t - ones
         ends = (self._i32(rows.query_start, "query_start"), self._i32(rows.row_slot, "row_slot"), ones, rows.n_rows)
-        if self.scan_parts and portions and take is None and decay is None and beta is None and more >= self.CHUNK_TOKENS * portions \
-                and not (qk.data_ptr() | state.data_ptr()) % 16:
+        parts = self.scan_parts and portions and take is None and skip is None and not state.data_ptr() % 16
+        if parts and decay is None and beta is None and more >= self.CHUNK_TOKENS * portions and not qk.data_ptr() % 16 \
+                and dim <= 1024 and vdim <= 4096:
             scanned, tiles = ones, more // 64 + portions                               # (the most that any cut into those rows has)
             scratch = torch.empty(tiles * (heads * vdim * dim + kv_heads * 64 * 64 + heads), dtype=torch.float32, device=self.device)
             self._call("hb_recurrent_chunks", self._p(out), self._p(qk), self._p(v), self._p(head_decay), self._p(token_decay),
                        self._p(state), self._p(scratch), *ends, tiles, heads, kv_heads, dim, vdim)
-        elif self.scan_parts and portions and (beta is not None) != (rate is not None) and token_decay is None \
-                and more >= self.BLOCK_TOKENS * portions and not state.data_ptr() % 16:
+        elif parts and (beta is not None) != (rate is not None) and token_decay is None and more >= self.BLOCK_TOKENS * portions:
             floats = self.lib.hb_recurrent_blocks_floats(int(rate is not None), dim)   # (0: a key size that is not taken)
             if floats:
                 scanned, blocks = ones, more // 8 + portions

@@ -1,0 +1,61 @@
+"""Which function of the compiled library a call of the kernel table goes to, without a GPU: the table's methods on CPU tensors
+with a library that only writes down what it is asked for."""
+import types
+
+import pytest
+import torch
+
+from holon_b200.engine.batch import Rows
+from holon_b200.kernels.cuda import CudaKernels
+
+F32 = torch.float32
+
+
+class Noted(CudaKernels):
+    def __init__(self):
+        self.device, self.called, self.scan_parts, self._pending, self._splits = torch.device("cpu"), [], True, [], {}
+        self.gemm, self.gemm_pair, self.attention_bf16, self.prefill_attention, self.skinny32 = "auto", True, "fast", "tcgen05", True
+        self.lib = types.SimpleNamespace(hb_recurrent_blocks_floats=lambda general, dim: 1 if dim in (64, 128, 256) else 0,
+                                         hb_latent_tcgen05_takes=lambda *sizes: 1)
+
+    def _check(self, *tensors):
+        assert all(t is None or t.is_contiguous() for t in tensors)
+
+    def _call(self, name, *args):
+        self.called.append(name)
+
+    def linear_tcgen05(self, out, x, weight, swiglu=False, pair=None):
+        self.called.append("linear_tcgen05")
+
+
+def rows_of(counts, host=False):
+    counts = sorted(counts, key=lambda n: n != 1)
+    starts = [sum(counts[:i]) for i in range(len(counts) + 1)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32)                                # noqa: E731
+    return Rows(i32(list(range(len(counts)))), i32(starts), i32(counts), len(counts), starts[-1], counts.count(1), max(counts), max(counts),
+                starts if host else None, counts if host else None)
+
+
+def scan(counts, *, heads=2, kv_heads=2, dim=64, vdim=8, host=False, **given):
+    """The calls of a scan over `counts`; given: decay, head, token, beta, rate, take, skip."""
+    k, rows = Noted(), rows_of(counts, host)
+    t = rows.n_tokens
+    shapes = dict(decay=(t, heads, dim), head=(heads,), token=(t, heads), beta=(t, heads), rate=(t, heads, dim), take=(t, heads), skip=(heads,))
+    x = {name: torch.zeros(shape) if given.get(name) else None for name, shape in shapes.items()}
+    k.recurrent_scan(torch.zeros(t, heads, vdim), torch.zeros(t, 2, kv_heads, dim), torch.zeros(t, heads, vdim), x["decay"], x["head"], x["beta"],
+                     torch.zeros(len(counts), heads, vdim, dim), rows, token_decay=x["token"], rate=x["rate"], take=x["take"], skip=x["skip"])
+    return k.called
+
+
+@pytest.mark.parametrize("given", [dict(head=True), dict(token=True), dict(decay=True, beta=True), dict(head=True, beta=True), dict(decay=True, rate=True)])
+@pytest.mark.parametrize("more", [dict(take=True), dict(skip=True), dict(take=True, skip=True)])
+def test_factors_and_skips_go_to_the_scan(given, more):
+    """What the token-by-token scan refuses (all of these but a decay per token with both) is not run without them."""
+    assert scan([300], **given, **more) == ["hb_recurrent_scan"]
+
+
+def test_sizes_that_the_scan_refuses_are_refused():
+    for given in (dict(head=True), dict(token=True)):
+        assert scan([300], **given) == ["hb_recurrent_chunks"]
+        assert scan([300], dim=1028, **given) == ["hb_recurrent_scan"]               # (a key size above 1024)
+        assert scan([300], heads=1, kv_heads=1, dim=1024, vdim=4200, **given) == ["hb_recurrent_scan"]   # (states that the chunks refuse)
