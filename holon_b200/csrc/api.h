@@ -413,12 +413,17 @@ int hb_softcap(float* x, long count, float cap, hb_stream stream);
 int hb_recurrent_scan(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
                       const float* token_decay, const float* beta, const float* rate, const float* take, const float* skip,
                       float* state, const int32_t* query_start, const int32_t* row_slot, int rows, int heads, int kv_heads, int dim, int vdim, int most, hb_stream stream);
-// The same with beta or rate for rows row0 .. rows - 1, eight tokens at a time (csrc/recurrent_blocks.cu), key sizes 64, 128 and 256.
-// blocks: at least the sum over the rows of ceil(tokens / 8); scratch: blocks * heads * hb_recurrent_blocks_floats(rate given, dim)
-// floats (0: a key size that is not taken) on a 16-byte boundary.
+// The same without the rows of `below` or more tokens (0: with them).
+int hb_recurrent_scan_below(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
+                            const float* token_decay, const float* beta, const float* rate, const float* take, const float* skip,
+                            float* state, const int32_t* query_start, const int32_t* row_slot, int rows, int heads, int kv_heads, int dim, int vdim, int most,
+                            int below, hb_stream stream);
+// The same with beta or rate for those of rows row0 .. rows - 1 that bring `least` tokens or more, eight tokens at a time
+// (csrc/recurrent_blocks.cu), key sizes 64, 128 and 256. `taken`: how many these rows are; blocks: at least the sum over them of ceil(tokens / 8); scratch:
+// blocks * heads * hb_recurrent_blocks_floats(rate given, dim) floats (0: a key size that is not taken) on a 16-byte boundary.
 int hb_recurrent_blocks(float* out, const float* qk, const float* v, const float* decay, const float* head_decay, const float* beta,
                         const float* rate, float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
-                        int rows, int blocks, int heads, int kv_heads, int dim, int vdim, hb_stream stream);
+                        int rows, int blocks, int least, int taken, int heads, int kv_heads, int dim, int vdim, hb_stream stream);
 int hb_recurrent_blocks_floats(int general, int dim);
 // The generalized delta rule's inputs from its first product, rows [r | k | v | g | a] of `dtype` (each heads dim wide,
 // `ld` apart) and the low-rank decay projection's output `pre` [tokens, heads dim] in 32-bit: qk = (r, k), v,
@@ -467,10 +472,11 @@ size_t hb_state_space_prompt_scratch_floats(int tiles, int heads, int groups, in
 int hb_state_space_prompt(float* y, const float* cb, const float* x, const float* dt, const float* rate_log, const float* skip,
                           float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0, int rows,
                           int tiles, int heads, int groups, int n, int vdim, hb_stream stream);
-// hb_recurrent_scan for rows row0 .. rows - 1 in the same chunks, with one decay per head (head_decay [heads]) or per head and token
-// (token_decay [tokens, heads]), without beta, rate, take and skip; tiles and scratch as above (groups = kv_heads, n = dim).
+// hb_recurrent_scan for those of rows row0 .. rows - 1 that bring `least` tokens or more, in the same chunks, with one decay per head
+// (head_decay [heads]) or per head and token (token_decay [tokens, heads]), without beta, rate, take and skip; tiles (of these rows)
+// and scratch as above (groups = kv_heads, n = dim).
 int hb_recurrent_chunks(float* out, const float* qk, const float* v, const float* head_decay, const float* token_decay, float* state,
-                        float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0, int rows, int tiles, int heads,
+                        float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0, int rows, int tiles, int least, int heads,
                         int kv_heads, int dim, int vdim, hb_stream stream);
 
 // ---- the matrix memory with exponential gates (csrc/mlstm.cu): the kernels around hb_recurrent_scan with token_decay.

@@ -55,7 +55,7 @@ __global__ void recurrent_scan_kernel(float* __restrict__ out, const float* __re
                                       const float* __restrict__ beta, const float* __restrict__ rate, const float* __restrict__ take,
                                       const float* __restrict__ skip, float* __restrict__ state,
                                       const int32_t* __restrict__ query_start, const int32_t* __restrict__ row_slot,
-                                      int heads, int kv_heads, int dim, int vdim, int VT, int tb) {
+                                      int heads, int kv_heads, int dim, int vdim, int VT, int tb, int below) {
     extern __shared__ __align__(16) float sm[];
     constexpr int DP = P * DPT;
     const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * VT;
@@ -63,6 +63,7 @@ __global__ void recurrent_scan_kernel(float* __restrict__ out, const float* __re
     const int p = threadIdx.x % P, cl = threadIdx.x / P, c = c0 + cl;
     const bool col = cl < VT && c < vdim;
     const int t0 = query_start[b], n = query_start[b + 1] - t0;
+    if (below > 0 && n >= below) return;                              // (a row that goes in parts: state_space.cu, recurrent_blocks.cu)
     float* S_g = state + (((size_t)row_slot[b] * heads + h) * vdim + (col ? c : 0)) * dim;   // this thread's column
     // a stage: q [tb][DP], k [tb][DP], decays [tb][DP] (per-channel decays only), v [tb][VT], beta [tb]; two of them
     float S[DPT];
@@ -327,7 +328,7 @@ __global__ void recurrent_scan_kernel(float* __restrict__ out, const float* __re
 template <int DPT, int P>
 static int launch_scan(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
                        const float* token_decay, const float* beta, const float* rate, const float* take, const float* skip, float* state, const int32_t* query_start, const int32_t* row_slot, int rows,
-                       int heads, int kv_heads, int dim, int vdim, int most, cudaStream_t s) {
+                       int heads, int kv_heads, int dim, int vdim, int most, int below, cudaStream_t s) {
     const int unit = 32 / P > 1 ? 32 / P : 1;                         // columns a warp holds
     int VT = vdim < 256 / P ? vdim : 256 / P;
     if (VT < 1) VT = 1;
@@ -349,14 +350,16 @@ static int launch_scan(float* out, const float* qk, const float* v, const float*
     if (rate) kernel = recurrent_scan_kernel<DPT, P, true, false, false, true>;
     if (smem > 46 * 1024) HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<dim3(rows, heads, tiles), threads, smem, s>>>(out, qk, v, decay, head_decay, beta, rate, take, skip, state, query_start, row_slot,
-                                                          heads, kv_heads, dim, vdim, VT, tb);
+                                                          heads, kv_heads, dim, vdim, VT, tb, below);
     HB_LAUNCH_CHECK("recurrent_scan");
     return 0;
 }
 
-extern "C" int hb_recurrent_scan(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
-                                 const float* token_decay, const float* beta, const float* rate, const float* take, const float* skip,
-                                 float* state, const int32_t* query_start, const int32_t* row_slot, int rows, int heads, int kv_heads, int dim, int vdim, int most, hb_stream stream) {
+// Rows of `below` or more tokens (0: none) are passed over.
+extern "C" int hb_recurrent_scan_below(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
+                                       const float* token_decay, const float* beta, const float* rate, const float* take, const float* skip,
+                                       float* state, const int32_t* query_start, const int32_t* row_slot, int rows, int heads, int kv_heads, int dim, int vdim, int most,
+                                       int below, hb_stream stream) {
     if (rows == 0) return 0;
     if (kv_heads < 1 || heads % kv_heads) HB_REFUSE("recurrent_scan: %d heads are no multiple of %d key heads", heads, kv_heads);
     if (dim < 1 || dim > 1024 || vdim < 1) HB_REFUSE("recurrent_scan: key size %d (1 to 1024), value size %d", dim, vdim);
@@ -368,7 +371,7 @@ extern "C" int hb_recurrent_scan(float* out, const float* qk, const float* v, co
     if ((((uintptr_t)qk | (uintptr_t)decay | (uintptr_t)rate) & 15) != 0) HB_REFUSE("recurrent_scan: qk, decay and rate must lie on 16-byte boundaries");
     cudaStream_t s = (cudaStream_t)stream;
 #define HB_SCAN(D, PP) return launch_scan<D, PP>(out, qk, v, decay, head_decay, token_decay, beta, rate, take, skip, state, query_start, row_slot, rows, heads, \
-                                                 kv_heads, dim, vdim, most, s)
+                                                 kv_heads, dim, vdim, most, below, s)
     // Four channels a thread up to a key size of 64, then more channels a thread. (Key size 128, 2,048 tokens of 16 heads,
     // microseconds a token with the delta rule: 16 lanes of 8 channels 0.37, 32 lanes of 4 0.40, 8 lanes of 16 0.40, 4 lanes of
     // 32 0.51: a token is one chain of dependent steps whatever the lanes, and the warps of an SM fill one another's gaps.)
@@ -382,6 +385,13 @@ extern "C" int hb_recurrent_scan(float* out, const float* qk, const float* v, co
     if (dim <= 512) HB_SCAN(16, 32);
     HB_SCAN(32, 32);
 #undef HB_SCAN
+}
+
+extern "C" int hb_recurrent_scan(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
+                                 const float* token_decay, const float* beta, const float* rate, const float* take, const float* skip,
+                                 float* state, const int32_t* query_start, const int32_t* row_slot, int rows, int heads, int kv_heads, int dim, int vdim, int most, hb_stream stream) {
+    return hb_recurrent_scan_below(out, qk, v, decay, head_decay, token_decay, beta, rate, take, skip, state, query_start, row_slot, rows, heads,
+                                   kv_heads, dim, vdim, most, 0, stream);
 }
 
 // ---------------------------------------------------------------- what the delta-rule mixer's first product becomes

@@ -2,7 +2,7 @@
 // cores, for key sizes of 64, 128 and 256.
 //
 // Token by token a scan is a chain: decay, a sum over the key channels' lanes, the write, the next token (2,048 tokens of 16
-// heads of 128 by 128 with the delta rule: 569 us, 278 ns a token). Over a block of T = 8 tokens with the state S before it, the
+// heads of 128 by 128 with the delta rule: 568 us, 278 ns a token). Over a block of T = 8 tokens with the state S before it, the
 // inputs' decayed products and the sums that involve S alone need no such chain. With G_j = g_1 o .. o g_j (per key channel)
 // and j, i counting the block's tokens,
 //     o_j = S^T (G_j o q_j) + sum_(i <= j) N_ji u_i,           N_ji = q_j . (g_(i+1) o .. o g_j o k_i)
@@ -20,7 +20,7 @@
 //                             thread holds 8 (4) channels of two or four columns, so that a vector's 16 bytes from shared memory meet as
 //                             many numbers of S; sums over the 16 (32) lanes of a column by halving the values a lane still
 //                             holds, 15 shuffles for 16 sums; packed multiply-adds; blocks arrive by cp.async, two ahead.
-// Bound by the issue of its instructions, about 1,200 a block for a warp of eight columns, at one warp a scheduler. 367 us at the size above.
+// Bound by the issue of its instructions, about 1,200 a block for a warp of eight columns, at one warp a scheduler. 305 us at the size above.
 #include "common.cuh"
 
 #define RB_T 8
@@ -108,21 +108,27 @@ __device__ __forceinline__ float rb_dot(const Channels<C>& a, const Channels<C>&
     return s;
 }
 
+// Blocks of row b: ceil(tokens / 8), and none of a row of fewer than `least` tokens (the token-by-token scan's).
+__device__ __forceinline__ int blocks_of(const int32_t* __restrict__ query_start, int b, int least) {
+    const int n = query_start[b + 1] - query_start[b];
+    return n >= least ? (n + RB_T - 1) / RB_T : 0;
+}
+
 // grid (blocks, heads / 4), 128 threads
 template <int C, int MODE>
 __global__ void __launch_bounds__(128) recurrent_block_kernel(float* __restrict__ scratch, const float* __restrict__ qk,
                                                               const float* __restrict__ decay, const float* __restrict__ head_decay,
                                                               const float* __restrict__ beta, const float* __restrict__ rate,
-                                                              const int32_t* __restrict__ query_start, int row0, int rows, int heads,
-                                                              int kv_heads) {
+                                                              const int32_t* __restrict__ query_start, int row0, int rows, int least,
+                                                              int heads, int kv_heads) {
     constexpr int DIM = 32 * C;
     __shared__ float products[4][2][RB_T][2 * RB_T], system[4][2][RB_T][RB_T];   // per warp: [N | M] of k, of r o k; A, B
     const int h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (h >= heads) return;
     int left = blockIdx.x, t0 = 0, m = 0;
     for (int b = row0; b < rows; ++b) {
-        const int n = query_start[b + 1] - query_start[b], blocks = (n + RB_T - 1) / RB_T;
-        if (left < blocks) { t0 = query_start[b] + left * RB_T; m = min(RB_T, n - left * RB_T); break; }
+        const int blocks = blocks_of(query_start, b, least);
+        if (left < blocks) { t0 = query_start[b] + left * RB_T; m = min(RB_T, query_start[b + 1] - t0); break; }
         left -= blocks;
     }
     if (m == 0) return;                                                  // (more blocks were launched than the step has)
@@ -243,21 +249,24 @@ __global__ void __launch_bounds__(128) recurrent_block_kernel(float* __restrict_
     }
 }
 
-// grid (rows, heads, column tiles), P * 16 / NC threads: thread (g, p) holds channels (i P + p) 4 .. + 3, i < DPT / 4, of columns
+// grid: rows x column tiles x heads, the heads of a row's tile next to one another (a long row's CTAs are then spread over the chip
+// before those of rows that end sooner or are passed over), P * 16 / NC threads: thread (g, p) holds channels (i P + p) 4 .. + 3, i < DPT / 4, of columns
 // NC g .. NC g + NC - 1 of the CTA's 16
 template <int DPT, int P, int NC, int MODE>
 __global__ void __launch_bounds__(P * RB_VT / NC) recurrent_blocks_kernel(
         float* __restrict__ out, const float* __restrict__ scratch, const float* __restrict__ v, float* __restrict__ state,
-        const int32_t* __restrict__ query_start, const int32_t* __restrict__ row_slot, int row0, int heads, int vdim) {
+        const int32_t* __restrict__ query_start, const int32_t* __restrict__ row_slot, int row0, int least, int heads, int vdim) {
     constexpr int DIM = DPT * P, VT = RB_VT, THREADS = P * VT / NC, T = RB_T;
     constexpr int FLOATS = rb_floats(MODE, DIM), STAGE = FLOATS + T * VT, V = 2 * T, QUADS = DPT / 4;
     extern __shared__ float4 smem4[];
     float* sm = (float*)smem4;                                           // [RB_STAGES][STAGE], then the outputs [2][T][VT]
     float* so = sm + RB_STAGES * STAGE;
-    const int b = row0 + blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * VT, tid = threadIdx.x, p = tid % P, g4 = tid / P * NC;
-    const int t0 = query_start[b], n = query_start[b + 1] - t0, blocks = (n + T - 1) / T;
+    const int h = blockIdx.x % heads, part = blockIdx.x / heads, tiles = (vdim + VT - 1) / VT;
+    const int b = row0 + part / tiles, c0 = part % tiles * VT, tid = threadIdx.x, p = tid % P, g4 = tid / P * NC;
+    const int t0 = query_start[b], n = query_start[b + 1] - t0, blocks = blocks_of(query_start, b, least);
+    if (blocks == 0) return;
     int first = 0;                                                       // the row's first block
-    for (int a = row0; a < b; ++a) first += (query_start[a + 1] - query_start[a] + T - 1) / T;
+    for (int a = row0; a < b; ++a) first += blocks_of(query_start, a, least);
     const float* src = scratch + ((size_t)first * heads + h) * FLOATS;
     float* S_g = state + ((size_t)row_slot[b] * heads + h) * vdim * DIM;
     uint64_t S[NC][2 * QUADS];
@@ -383,7 +392,7 @@ __global__ void __launch_bounds__(P * RB_VT / NC) recurrent_blocks_kernel(
         }
     }
     __syncthreads();
-    if (blocks > 0) write(blocks - 1);
+    write(blocks - 1);
 #pragma unroll
     for (int c = 0; c < NC; ++c)
         if (c0 + g4 + c < vdim)
@@ -404,39 +413,40 @@ extern "C" int hb_recurrent_blocks_floats(int general, int dim) {
 template <int DPT, int P, int NC, int MODE>
 static int launch_blocks(float* out, const float* qk, const float* v, const float* decay, const float* head_decay, const float* beta,
                          const float* rate, float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
-                         int rows, int blocks, int heads, int kv_heads, int vdim, cudaStream_t s) {
+                         int rows, int blocks, int least, int heads, int kv_heads, int vdim, cudaStream_t s) {
     constexpr int DIM = DPT * P, VT = RB_VT;
     recurrent_block_kernel<DIM / 32, MODE><<<dim3(blocks, (heads + 3) / 4), 128, 0, s>>>(
-        scratch, qk, decay, head_decay, beta, rate, query_start, row0, rows, heads, kv_heads);
+        scratch, qk, decay, head_decay, beta, rate, query_start, row0, rows, least, heads, kv_heads);
     HB_LAUNCH_CHECK("recurrent_block");
     const int smem = (RB_STAGES * (rb_floats(MODE, DIM) + RB_T * VT) + 2 * RB_T * VT) * (int)sizeof(float);
     auto kernel = recurrent_blocks_kernel<DPT, P, NC, MODE>;
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kernel<<<dim3(rows - row0, heads, (vdim + VT - 1) / VT), P * VT / NC, smem, s>>>(out, scratch, v, state, query_start, row_slot, row0, heads, vdim);
+    kernel<<<dim3((unsigned)((rows - row0) * ((vdim + VT - 1) / VT) * heads)), P * VT / NC, smem, s>>>(out, scratch, v, state, query_start, row_slot, row0, least, heads, vdim);
     HB_LAUNCH_CHECK("recurrent_blocks");
     return 0;
 }
 
-// Rows row0 .. rows - 1 of the batch, otherwise as hb_recurrent_scan with beta or with rate. blocks: at least the sum over the rows of
-// ceil(tokens / 8); scratch: blocks * heads * hb_recurrent_blocks_floats(...) floats on a 16-byte boundary.
+// Those of rows row0 .. rows - 1 of the batch that bring `least` tokens or more, otherwise as hb_recurrent_scan with beta or with rate.
+// `taken`: how many these are (or may be), for the choice below; blocks: at least the sum over them of ceil(tokens / 8); scratch: blocks * heads * hb_recurrent_blocks_floats(...) floats on a 16-byte boundary.
 extern "C" int hb_recurrent_blocks(float* out, const float* qk, const float* v, const float* decay, const float* head_decay,
                                    const float* beta, const float* rate, float* state, float* scratch, const int32_t* query_start,
-                                   const int32_t* row_slot, int row0, int rows, int blocks, int heads, int kv_heads, int dim, int vdim,
-                                   hb_stream stream) {
+                                   const int32_t* row_slot, int row0, int rows, int blocks, int least, int taken,
+                                   int heads, int kv_heads, int dim, int vdim, hb_stream stream) {
     if (rows <= row0 || blocks <= 0) return 0;
     if (kv_heads < 1 || heads % kv_heads) HB_REFUSE("recurrent_blocks: %d heads are no multiple of %d key heads", heads, kv_heads);
     if (vdim < 1 || !hb_recurrent_blocks_floats(0, dim)) HB_REFUSE("recurrent_blocks: key size %d (64, 128 or 256), value size %d", dim, vdim);
     if ((decay != nullptr) == (head_decay != nullptr)) HB_REFUSE("recurrent_blocks: give decays per channel and token, or one per head");
     if ((rate != nullptr) == (beta != nullptr) || (rate && !decay)) HB_REFUSE("recurrent_blocks: either a delta rule's beta or, with decays per channel, removal rates");
-    if (heads > 65535 || (vdim + RB_VT - 1) / RB_VT > 65535) HB_REFUSE("recurrent_blocks: %d heads, value size %d", heads, vdim);
+    if (heads > 65535 || (long)(rows - row0) * heads * ((vdim + RB_VT - 1) / RB_VT) > 0x7fffffffL)
+        HB_REFUSE("recurrent_blocks: %d rows, %d heads, value size %d", rows - row0, heads, vdim);
     if ((((uintptr_t)qk | (uintptr_t)decay | (uintptr_t)rate | (uintptr_t)state | (uintptr_t)scratch) & 15) != 0)
         HB_REFUSE("recurrent_blocks: qk, decay, rate, state and scratch must lie on 16-byte boundaries");
     cudaStream_t s = (cudaStream_t)stream;
     // Four columns a thread halve the reads of shared memory a column; two keep an SM's four schedulers busy where there is no more
-    // than a CTA or two for each (2,048 tokens, 16 heads of 128 by 128: 350 us with two, 403 with four; 32 heads and two rows of
-    // 1,500 and 938 tokens: 602 and 484).
-    const bool many = (long)(rows - row0) * heads * ((vdim + RB_VT - 1) / RB_VT) > 296;
-#define RB_ARGS out, qk, v, decay, head_decay, beta, rate, state, scratch, query_start, row_slot, row0, rows, blocks, heads, kv_heads, vdim, s
+    // than a CTA or two for each (heads of 128 by 128, the delta rule: 16 heads and 2,048 tokens 304 us with two, 403 with four; 16 heads and
+    // rows of 1,500 and 938 tokens 295 and 311; 32 heads and 2,048 tokens 454 and 431; 32 heads and the two rows 529 and 475).
+    const bool many = (long)taken * heads * ((vdim + RB_VT - 1) / RB_VT) > 296;
+#define RB_ARGS out, qk, v, decay, head_decay, beta, rate, state, scratch, query_start, row_slot, row0, rows, blocks, least, heads, kv_heads, vdim, s
 #define RB_GO(D, P) do { \
         if (many) return rate ? launch_blocks<D, P, 4, RB_GENERAL>(RB_ARGS) : launch_blocks<D, P, 4, RB_DELTA>(RB_ARGS); \
         return rate ? launch_blocks<D, P, 2, RB_GENERAL>(RB_ARGS) : launch_blocks<D, P, 2, RB_DELTA>(RB_ARGS); \

@@ -9,7 +9,7 @@
 // With a decay given as itself (FIXED: one per head, TOKEN: per head and token) dt = 1, there is no skip, and L sums the logarithms of
 // its magnitude in double precision, a zero counting as -10^4 (below which an exponential is zero); signs are kept beside it. A value that is no finite
 // number reaches the outputs from its token on and no earlier one.
-// 2,048 tokens of 16 heads of 128 by 128 with a decay per head: 154 us in chunks, 422 us token by token (recurrent.cu).
+// 2,048 tokens of 16 heads of 128 by 128 with a decay per head: 144 us in chunks, 417 us token by token (recurrent.cu).
 // Four kernels: the chunks' products C_i . B_j, per group; the chunks' own contributions to the state, per head; the walk over a
 // row's chunks, an element of the state a thread, which leaves every chunk's S_in behind and writes the row's state back; the
 // chunks' outputs, per head. Only the third is sequential, one multiply-add a chunk. Blocks find their (row, chunk) in the step's
@@ -25,11 +25,17 @@
 
 struct Chunk { int row, t0, n, first_tile; };              // the batch row, first token, tokens, the row's first tile
 
-// Tile number -> chunk (row -1: there is none). Rows row0 .. rows - 1 in order, each ceil(tokens / 64) tiles.
-__device__ __forceinline__ Chunk find_chunk(const int32_t* __restrict__ query_start, int row0, int rows, int tile) {
+// Tiles of row b: ceil(tokens / 64), and none of a row of fewer than `least` tokens.
+__device__ __forceinline__ int tiles_of(const int32_t* __restrict__ query_start, int b, int least) {
+    const int n = query_start[b + 1] - query_start[b];
+    return n >= least ? (n + SS_Q - 1) / SS_Q : 0;
+}
+
+// Tile number -> chunk (row -1: there is none). Rows row0 .. rows - 1 in order.
+__device__ __forceinline__ Chunk find_chunk(const int32_t* __restrict__ query_start, int row0, int rows, int tile, int least) {
     int left = tile;
     for (int b = row0; b < rows; ++b) {
-        const int n = query_start[b + 1] - query_start[b], tiles = (n + SS_Q - 1) / SS_Q;
+        const int n = query_start[b + 1] - query_start[b], tiles = tiles_of(query_start, b, least);
         if (left < tiles) return {b, query_start[b] + left * SS_Q, min(SS_Q, n - left * SS_Q), tile - left};
         left -= tiles;
     }
@@ -160,9 +166,9 @@ __device__ __forceinline__ void log_decays(float* hi, float* lo, float* steps, f
 // ---- products[tile][group][i][j] = C_i . B_j, [64][64] each. grid (tiles, groups)
 template <int FORM>
 __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_products_kernel(float* __restrict__ products, const float* __restrict__ cb,
-                                                                 const int32_t* __restrict__ query_start, int row0, int rows, int groups, int n, int quads) {
+                                                                 const int32_t* __restrict__ query_start, int row0, int rows, int groups, int n, int quads, int least) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
-    const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
+    const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x, least);
     if (c.row < 0) return;
     const int g = blockIdx.y;
     float acc[8][4] = {};
@@ -195,10 +201,10 @@ template <int FORM>
 __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_own_kernel(float* __restrict__ own, float* __restrict__ last, const float* __restrict__ cb,
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const int32_t* __restrict__ query_start,
-                                                            int row0, int rows, int heads, int groups, int n, int vdim, int n_tiles, int quads) {
+                                                            int row0, int rows, int heads, int groups, int n, int vdim, int n_tiles, int quads, int least) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
     __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q], sign[FORM == STATE_SPACE ? 1 : SS_Q];
-    const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
+    const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x, least);
     if (c.row < 0) return;
     const int h = blockIdx.y, g = h / (heads / groups);
     const int p0 = ((int)blockIdx.z / n_tiles) * SS_T, n0 = ((int)blockIdx.z % n_tiles) * SS_T;
@@ -250,12 +256,13 @@ __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_own_kernel(float
 // slices of the state), an element (V: four) a thread.
 template <bool V>
 __global__ void ss_walk_kernel(float* __restrict__ own, const float* __restrict__ last, float* __restrict__ state,
-                               const int32_t* __restrict__ query_start, const int32_t* __restrict__ row_slot, int row0, int heads, int size) {
+                               const int32_t* __restrict__ query_start, const int32_t* __restrict__ row_slot, int row0, int heads, int size,
+                               int least) {
     typedef typename std::conditional<V, float4, float>::type E;
     const int b = row0 + (int)blockIdx.x, h = blockIdx.y, e = blockIdx.z * blockDim.x + threadIdx.x;
     int first = 0;
-    for (int r = row0; r < b; ++r) first += (query_start[r + 1] - query_start[r] + SS_Q - 1) / SS_Q;
-    const int tiles = (query_start[b + 1] - query_start[b] + SS_Q - 1) / SS_Q;
+    for (int r = row0; r < b; ++r) first += tiles_of(query_start, r, least);
+    const int tiles = tiles_of(query_start, b, least);
     if (e >= (V ? size >> 2 : size) || tiles == 0) return;
     E* st = (E*)(state + ((size_t)row_slot[b] * heads + h) * size) + e;
     const size_t stride = (size_t)heads * size / (V ? 4 : 1);
@@ -290,11 +297,11 @@ __global__ void __launch_bounds__(SS_THREADS, SS_CTAS(FORM)) ss_out_kernel(float
                                                             const float* __restrict__ x, const float* __restrict__ dt,
                                                             const float* __restrict__ rate_log, const float* __restrict__ skip,
                                                             const int32_t* __restrict__ query_start, int row0, int rows, int heads,
-                                                            int groups, int n, int vdim, int quads) {
+                                                            int groups, int n, int vdim, int quads, int least) {
     __shared__ __align__(16) float a[SS_K * SS_T], b[SS_K * SS_T];
     __shared__ float hi[SS_Q], lo[SS_Q], steps[SS_Q], w[SS_Q], sign[FORM == STATE_SPACE ? 1 : SS_Q];
     __shared__ int bad[SS_T];                                       // per column: the first token whose value is no finite number
-    const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x);
+    const Chunk c = find_chunk(query_start, row0, rows, blockIdx.x, least);
     if (c.row < 0) return;
     const int h = blockIdx.y, g = h / (heads / groups), p0 = (int)blockIdx.z * SS_T;
     const float* cbp = products + ((size_t)blockIdx.x * groups + g) * SS_Q * SS_Q;
@@ -385,7 +392,7 @@ extern "C" size_t hb_state_space_prompt_scratch_floats(int tiles, int heads, int
 template <int FORM>
 static int run_chunks(const char* what, float* y, const float* cb, const float* x, const float* dt, const float* rate_log, const float* skip,
                                      float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
-                                     int rows, int tiles, int heads, int groups, int n, int vdim, hb_stream stream) {
+                                     int rows, int tiles, int heads, int groups, int n, int vdim, int least, hb_stream stream) {
     if (rows <= row0 || tiles == 0) return 0;
     if (groups < 1 || heads % groups || n < 1 || vdim < 1) HB_REFUSE("%s: %d heads of %d, %d groups of %d", what, heads, vdim, groups, n);
     if (!scratch || ((uintptr_t)scratch & 15) || ((uintptr_t)state & 15)) HB_REFUSE("%s: scratch and state must lie on 16-byte boundaries", what);
@@ -396,19 +403,19 @@ static int run_chunks(const char* what, float* y, const float* cb, const float* 
     float* own = products + (size_t)tiles * groups * SS_Q * SS_Q;  // [tiles][heads][vdim][n]
     float* last = own + (size_t)tiles * heads * size;              // [tiles][heads]
     cudaStream_t s = (cudaStream_t)stream;
-    ss_products_kernel<FORM><<<dim3(tiles, groups), SS_THREADS, 0, s>>>(products, cb, query_start, row0, rows, groups, n, quads);
+    ss_products_kernel<FORM><<<dim3(tiles, groups), SS_THREADS, 0, s>>>(products, cb, query_start, row0, rows, groups, n, quads, least);
     HB_LAUNCH_CHECK("state_space_products");
     ss_own_kernel<FORM><<<dim3(tiles, heads, p_tiles * n_tiles), SS_THREADS, 0, s>>>(own, last, cb, x, dt, rate_log, query_start, row0, rows, heads,
-                                                                               groups, n, vdim, n_tiles, quads);
+                                                                               groups, n, vdim, n_tiles, quads, least);
     HB_LAUNCH_CHECK("state_space_own");
     const bool vec = size % 4 == 0;
     const int elements = vec ? size / 4 : size, slices = (elements + 127) / 128;
     if (slices > 65535) HB_REFUSE("%s: states of %d numbers", what, size);
-    if (vec) ss_walk_kernel<true><<<dim3(rows - row0, heads, slices), 128, 0, s>>>(own, last, state, query_start, row_slot, row0, heads, size);
-    else ss_walk_kernel<false><<<dim3(rows - row0, heads, slices), 128, 0, s>>>(own, last, state, query_start, row_slot, row0, heads, size);
+    if (vec) ss_walk_kernel<true><<<dim3(rows - row0, heads, slices), 128, 0, s>>>(own, last, state, query_start, row_slot, row0, heads, size, least);
+    else ss_walk_kernel<false><<<dim3(rows - row0, heads, slices), 128, 0, s>>>(own, last, state, query_start, row_slot, row0, heads, size, least);
     HB_LAUNCH_CHECK("state_space_walk");
     ss_out_kernel<FORM><<<dim3(tiles, heads, p_tiles), SS_THREADS, 0, s>>>(y, products, own, cb, x, dt, rate_log, skip, query_start, row0, rows, heads,
-                                                                     groups, n, vdim, quads);
+                                                                     groups, n, vdim, quads, least);
     HB_LAUNCH_CHECK("state_space_out");
     return 0;
 }
@@ -417,19 +424,19 @@ extern "C" int hb_state_space_prompt(float* y, const float* cb, const float* x, 
                                      float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
                                      int rows, int tiles, int heads, int groups, int n, int vdim, hb_stream stream) {
     return run_chunks<STATE_SPACE>("state_space_prompt", y, cb, x, dt, rate_log, skip, state, scratch, query_start, row_slot, row0, rows, tiles,
-                                   heads, groups, n, vdim, stream);
+                                   heads, groups, n, vdim, 1, stream);
 }
 
-// hb_recurrent_scan for rows row0 .. rows - 1 with one decay per head (head_decay) or per head and token (token_decay) and no delta rule:
+// hb_recurrent_scan for those of rows row0 .. rows - 1 that bring `least` tokens or more, with one decay per head (head_decay) or per head and token (token_decay) and no delta rule:
 // qk [tokens, 2, kv_heads, dim]. tiles and scratch as above, with kv_heads and dim in the places of groups and n.
 extern "C" int hb_recurrent_chunks(float* out, const float* qk, const float* v, const float* head_decay, const float* token_decay,
                                    float* state, float* scratch, const int32_t* query_start, const int32_t* row_slot, int row0,
-                                   int rows, int tiles, int heads, int kv_heads, int dim, int vdim, hb_stream stream) {
+                                   int rows, int tiles, int least, int heads, int kv_heads, int dim, int vdim, hb_stream stream) {
     if ((head_decay != nullptr) == (token_decay != nullptr)) HB_REFUSE("recurrent_chunks: one decay per head, or one per head and token");
     if ((uintptr_t)qk & 15) HB_REFUSE("recurrent_chunks: qk must lie on a 16-byte boundary");
     if (token_decay)
         return run_chunks<TOKEN>("recurrent_chunks", out, qk, v, token_decay, nullptr, nullptr, state, scratch, query_start, row_slot, row0,
-                                 rows, tiles, heads, kv_heads, dim, vdim, stream);
+                                 rows, tiles, heads, kv_heads, dim, vdim, least, stream);
     return run_chunks<FIXED>("recurrent_chunks", out, qk, v, nullptr, head_decay, nullptr, state, scratch, query_start, row_slot, row0, rows,
-                             tiles, heads, kv_heads, dim, vdim, stream);
+                             tiles, heads, kv_heads, dim, vdim, least, stream);
 }

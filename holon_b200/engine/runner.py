@@ -118,6 +118,8 @@ class Runner:
             self.ctx.kernels.scatter_rows(g.table_device, dev[f"table_slots.{g.index}"], dev[f"table_rows.{g.index}"])
         rows_ = Rows(dev["row_slot"], dev["query_start"], dev["kv_len"], b, t, n_decode + pad_rows,
                      max(counts), int(kv_len.max()), query_start, kv_len)
+        if bucket:
+            rows_.plan["any cut"] = True              # (a graph's launches serve every cut of its tokens into its rows)
         groups = [GroupStep(g.table_device, dev[f"write_index.{g.index}"], g.page_size) for g in c.groups]
         step = StepContext(dev["token_ids"], dev["positions"], dev["logits_index"], rows_, groups, c)
         step.extra = {name: dev[name] for name in (extra or {})}

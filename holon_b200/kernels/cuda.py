@@ -1203,12 +1203,32 @@ class CudaKernels:
             if t is not None and t.dtype != torch.float32:
                 raise KernelError(f"{what}: 32-bit tensors expected, got {t.dtype}")
 
-    # Tokens a row on average from which the scan goes in chunks of 64 (four launches: 16 heads of 128 by 128, one row of 128 tokens
-    # 33 us token by token and 43 in chunks, 256 tokens 60 and 49, 2,048 tokens 422 and 154; eight rows of 100 96 and 106).
-    CHUNK_TOKENS = 192
-    # And eight tokens at a time (two launches: the delta rule with 32 tokens 17 us token by token and 24 in blocks, 48 tokens 21 and
-    # 21, 64 tokens 25 and 23, 2,048 tokens 574 and 367; eight rows of 40 70 and 35; the generalized rule alike).
-    BLOCK_TOKENS = 48
+    # Whether a row goes in parts is decided by its own tokens, whatever lies beside it, so that its bits do not depend on the batch; rows
+    # of both kinds then follow one another. Graphs of calls, 16 heads of 128 by 128, microseconds.
+    # In chunks of 64 (four launches) from 128 tokens on: one row of 100 tokens 34 in chunks and 26 token by token, 128 34 and 31, 160 38
+    # and 37, 256 37 and 44, 2,048 144 and 417. The line lies a little below the crossing for the sake of two kinds in one step: rows of
+    # 200 and 191 tokens 50 from 128 on, 96 from 192 on.
+    CHUNK_TOKENS = 128
+    # Eight tokens at a time (two launches; with a delta rule) from 16 tokens on: one row of 8 tokens 9.0 in blocks and 7.4 token by token,
+    # 16 10.3 and 11.0, 64 17 and 19, 2,048 305 and 568; eleven rows of 16 23 and 52; the generalized rule alike.
+    BLOCK_TOKENS = 16
+
+    @staticmethod
+    def _long_rows(rows, least: int, size: int) -> tuple[int, int, bool]:
+        """Of the rows of several tokens: how many bring `least` tokens or more, the parts of `size` tokens these are cut into, and
+        whether there are others. Exact where this step alone is launched; for a launch that is captured, and serves every cut of as
+        many tokens into as many rows, what any cut needs."""
+        portions, tokens = rows.n_rows - rows.n_decode, rows.n_tokens - rows.n_decode
+        starts = None if "any cut" in rows.plan else rows.host_query_start
+        if starts is None and portions > 1:
+            count = min(portions, tokens // least)
+            return count, tokens // size + count, True
+        key = "long", least, size
+        if key not in rows.plan:
+            counts = [tokens] if starts is None else [int(starts[b + 1]) - int(starts[b]) for b in range(rows.n_decode, rows.n_rows)]
+            counts = [n for n in counts[:portions] if n >= least]
+            rows.plan[key] = len(counts), sum(-(-n // size) for n in counts), len(counts) < portions
+        return rows.plan[key]
 
     def recurrent_scan(self, out, qk, v, decay, head_decay, beta, state, rows, token_decay=None, rate=None, take=None,
                        skip=None) -> None:
@@ -1230,31 +1250,34 @@ class CudaKernels:
             raise KernelError("recurrent_scan: qk [tokens, 2, kv_heads, dim], v and out [tokens, heads, vdim], state "
                               "[slots, heads, vdim, dim], decay [tokens, heads, dim] or head_decay [heads], beta [tokens, heads]")
         # Rows of many tokens: in chunks of 64 where the decay is one number per head, with a delta rule eight tokens at a time (what else
-        # was given goes to the scan, which takes or refuses it). What the launches depend on are counts of rows and tokens, so that they
-        # can be captured.
-        scanned, ones, portions = rows.n_rows, rows.n_decode, rows.n_rows - rows.n_decode
-        more = t - ones
-        ends = (self._i32(rows.query_start, "query_start"), self._i32(rows.row_slot, "row_slot"), ones, rows.n_rows)
-        parts = self.scan_parts and portions and take is None and skip is None and not state.data_ptr() % 16
-        if parts and decay is None and beta is None and more >= self.CHUNK_TOKENS * portions and not qk.data_ptr() % 16 \
-                and dim <= 1024 and vdim <= 4096:
-            scanned, tiles = ones, more // 64 + portions                               # (the most that any cut into those rows has)
-            scratch = torch.empty(tiles * (heads * vdim * dim + kv_heads * 64 * 64 + heads), dtype=torch.float32, device=self.device)
-            self._call("hb_recurrent_chunks", self._p(out), self._p(qk), self._p(v), self._p(head_decay), self._p(token_decay),
-                       self._p(state), self._p(scratch), *ends, tiles, heads, kv_heads, dim, vdim)
-        elif parts and (beta is not None) != (rate is not None) and token_decay is None and more >= self.BLOCK_TOKENS * portions:
-            floats = self.lib.hb_recurrent_blocks_floats(int(rate is not None), dim)   # (0: a key size that is not taken)
+        # was given goes to the scan, which takes or refuses it).
+        ones, least, scanned = rows.n_decode, 0, rows.n_rows
+        ends = (self._i32(rows.query_start, "query_start"), self._i32(rows.row_slot, "row_slot"))
+        parts = self.scan_parts and take is None and skip is None and not state.data_ptr() % 16
+        if parts and decay is None and beta is None and not qk.data_ptr() % 16 and dim <= 1024 and vdim <= 4096:
+            count, tiles, others = self._long_rows(rows, self.CHUNK_TOKENS, 64)
+            if count:
+                least, scanned = self.CHUNK_TOKENS, rows.n_rows if others else ones
+                scratch = torch.empty(tiles * (heads * vdim * dim + kv_heads * 64 * 64 + heads), dtype=torch.float32, device=self.device)
+                self._call("hb_recurrent_chunks", self._p(out), self._p(qk), self._p(v), self._p(head_decay), self._p(token_decay),
+                           self._p(state), self._p(scratch), *ends, ones, rows.n_rows, tiles, least, heads, kv_heads, dim, vdim)
+        elif parts and (beta is not None) != (rate is not None) and token_decay is None:
+            count, blocks, others = self._long_rows(rows, self.BLOCK_TOKENS, 8)
+            floats = self.lib.hb_recurrent_blocks_floats(int(rate is not None), dim) if count else 0   # (0: a key size that is not taken)
             if floats:
-                scanned, blocks = ones, more // 8 + portions
+                least, scanned = self.BLOCK_TOKENS, rows.n_rows if others else ones
                 scratch = torch.empty(blocks * heads * floats, dtype=torch.float32, device=self.device)
                 self._call("hb_recurrent_blocks", self._p(out), self._p(qk), self._p(v), self._p(decay), self._p(head_decay),
-                           self._p(beta), self._p(rate), self._p(state), self._p(scratch), *ends, blocks, heads, kv_heads, dim, vdim)
+                           self._p(beta), self._p(rate), self._p(state), self._p(scratch), *ends, ones, rows.n_rows, blocks, least, count,
+                           heads, kv_heads, dim, vdim)
         if scanned:
-            self._call("hb_recurrent_scan", self._p(out), self._p(qk), self._p(v), self._p(decay), self._p(head_decay),
-                       self._p(token_decay), self._p(beta), self._p(rate), self._p(take), self._p(skip), self._p(state),
-                       self._i32(rows.query_start, "query_start"),
-                       self._i32(rows.row_slot, "row_slot"), scanned, heads, kv_heads, dim, vdim,
-                       int(getattr(rows, "max_q", 0) or 0))
+            given = (self._p(out), self._p(qk), self._p(v), self._p(decay), self._p(head_decay), self._p(token_decay), self._p(beta),
+                     self._p(rate), self._p(take), self._p(skip), self._p(state), *ends, scanned, heads, kv_heads, dim, vdim,
+                     int(getattr(rows, "max_q", 0) or 0))
+            if least and scanned > ones:
+                self._call("hb_recurrent_scan_below", *given, least)
+            else:
+                self._call("hb_recurrent_scan", *given)
 
     def delta_prepare(self, qk, v, beta, decay, gate, first, conv, conv_state, low2, dt_bias, rate_log, rows, q_scale,
                       unit_eps, carry=False) -> None:

@@ -159,3 +159,35 @@ def test_values_anywhere_in_memory(K, form, vdim):
         outs.append((out, state))
     for out, state in outs[1:]:
         assert torch.equal(out, outs[0][0]) and torch.equal(state, outs[0][1])
+
+
+@pytest.mark.parametrize("form", ["fixed", "token", "delta", "general"])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 128, 64), (8, 8, 256, 128)])
+def test_a_row_does_not_depend_on_the_rows_beside_it(K, form, heads, kv_heads, dim, vdim):
+    """Rows below, at and above the lengths from which a row goes in parts: the same bits alone and together."""
+    counts = [1, 1, 15, 47, 16, 127, 128, 300, 2, 449]
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    t, slots = sum(counts), [9, 0, 3, 1, 2, 8, 5, 7, 4, 6]
+    qk = torch.nn.functional.normalize(torch.randn(t, 2, kv_heads, dim, generator=g, device=DEV), dim=-1)
+    v = torch.randn(t, heads, vdim, generator=g, device=DEV)
+    decay = 1 - torch.rand(t, heads, dim, generator=g, device=DEV) * 0.1
+    beta, rate = torch.rand(t, heads, generator=g, device=DEV), torch.rand(t, heads, dim, generator=g, device=DEV)
+    begin = torch.randn(10, heads, vdim, dim, generator=g, device=DEV) * 0.1
+
+    def run(first, counts, slots, host):
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)                # noqa: E731
+        starts, at = [sum(counts[:i]) for i in range(len(counts) + 1)], slice(first, first + sum(counts))
+        rows = Rows(i32(slots), i32(starts), i32(counts), len(counts), starts[-1], counts.count(1), max(counts), 0, starts if host else None)
+        state, out = begin.clone(), torch.empty_like(v[at])
+        K.recurrent_scan(out, qk[at].contiguous(), v[at].contiguous(), decay[at].contiguous() if form in ("delta", "general") else None,
+                         decay[0, :, 0].contiguous() if form == "fixed" else None, beta[at].contiguous() if form == "delta" else None, state, rows,
+                         token_decay=decay[at, :, 0].contiguous() if form == "token" else None,
+                         rate=rate[at].contiguous() if form == "general" else None)
+        return out, state
+
+    for host in (False, True):
+        together, states = run(0, counts, slots, host)
+        for i, n in enumerate(counts):
+            first = sum(counts[:i])
+            alone, state = run(first, [n], [slots[i]], host)
+            assert torch.equal(alone, together[first:first + n]) and torch.equal(state[slots[i]], states[slots[i]]), (n, host)

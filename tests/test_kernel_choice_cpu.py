@@ -59,3 +59,37 @@ def test_sizes_that_the_scan_refuses_are_refused():
         assert scan([300], **given) == ["hb_recurrent_chunks"]
         assert scan([300], dim=1028, **given) == ["hb_recurrent_scan"]               # (a key size above 1024)
         assert scan([300], heads=1, kv_heads=1, dim=1024, vdim=4200, **given) == ["hb_recurrent_scan"]   # (states that the chunks refuse)
+
+
+BLOCKS = dict(decay=True, beta=True)
+
+
+def test_a_row_goes_in_parts_by_its_own_tokens(monkeypatch):
+    """Long rows in parts and short ones by the scan, whatever the average; no launch for rows that the host knows not to be there."""
+    monkeypatch.setattr(CudaKernels, "CHUNK_TOKENS", 192)
+    monkeypatch.setattr(CudaKernels, "BLOCK_TOKENS", 48)
+    parts, short, scanned = "hb_recurrent_chunks", "hb_recurrent_scan_below", "hb_recurrent_scan"
+    for host, counts, want in ((True, [191], [scanned]), (True, [192], [parts]), (True, [1, 192], [parts, scanned]),
+                               (True, [191, 191, 1], [scanned]), (True, [2048, *[16] * 11], [parts, short]), (True, [300, 192], [parts]),
+                               (False, [191], [scanned]), (False, [192], [parts]), (False, [96, 96], [parts, short]), (False, [96, 95], [scanned]),
+                               (True, [1] * 300, [scanned])):
+        assert scan(counts, host=host, head=True) == want, counts
+        assert scan(counts, host=host, token=True) == want, counts
+    for host, counts, want in ((True, [47], [scanned]), (True, [48, 100], ["hb_recurrent_blocks"]), (True, [47, 48], ["hb_recurrent_blocks", short])):
+        assert scan(counts, host=host, **BLOCKS) == want, counts
+    assert scan([100], dim=96, host=True, **BLOCKS) == [scanned]
+
+
+def test_parts_of_any_cut():
+    """For a captured launch the parts of every cut of so many tokens into so many rows fit what is launched."""
+    import random
+    rng = random.Random(1)
+    for _ in range(300):
+        portions, least, size = rng.randint(1, 6), rng.choice([48, 192]), rng.choice([8, 64])
+        counts = [rng.randint(2, 400) for _ in range(portions)]
+        exact = CudaKernels._long_rows(rows_of(counts, host=True), least, size)
+        captured = rows_of(counts, host=True)
+        captured.plan["any cut"] = True
+        most = CudaKernels._long_rows(captured, least, size)
+        assert exact[0] <= most[0] and exact[1] <= most[1] and exact[2] <= most[2]
+        assert exact[:2] == (sum(n >= least for n in counts), sum(-(-n // size) for n in counts if n >= least))
