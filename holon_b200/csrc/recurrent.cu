@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(128) delta_prepare_wide_kernel(
             for (int i = 0; i < 4; ++i) w[j][i] = to_f32(conv[(size_t)(c + i) * TAPS + j]);
         int b = row_of_token(query_start, rows, begin);
         for (int t = begin; t < end; ++t) {
-            while (t >= query_start[b + 1]) ++b;
+            while (b + 1 < rows && t >= query_start[b + 1]) ++b;          // (tokens behind the last row count as its own)
             const int t0 = query_start[b];
             T* st = TAPS > 1 ? conv_state + (size_t)row_slot[b] * (TAPS - 1) * C + c : nullptr;
             auto input = [&](int from, float (&x)[4]) {                  // the inputs of token `from` of this row

@@ -500,3 +500,17 @@ def test_retention_prepare_four_numbers_a_thread(K, dtype, dim, vdim, rot_dims):
         REF.retention_prepare(*want, first, positions, table, rot_dims, 0.3, silu=silu)
         for g, w in zip(got, want):
             close(g, w, torch.float32)
+
+
+def test_delta_prepare_with_tokens_behind_the_last_row(K):
+    """They count as the last row's, and the search for a token's row ends there."""
+    heads, kv_heads, dim, vdim, taps, t = 4, 2, 64, 32, 4, 90
+    c, nv = 2 * kv_heads * dim + heads * vdim, heads * vdim
+    given = [x.to(DEV) for x in (rand(t, c + heads, seed=1), rand(c, taps, seed=3), rand(2, taps - 1, c, seed=6), rand(t, heads * dim + nv, seed=2),
+                                 rand(heads * dim, seed=4), rand(heads, seed=5))]
+    outs = []
+    for counts in ([20, 70], [20, 50]):
+        out = [torch.full(s, float("nan"), device=DEV) for s in ((t, 2, kv_heads, dim), (t, heads, vdim), (t, heads), (t, heads, dim), (t, nv))]
+        K.delta_prepare(*out, *given, rows_of(counts, [1, 0]), dim ** -0.5, 1e-6)
+        outs.append(out)
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
