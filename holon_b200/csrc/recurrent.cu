@@ -461,7 +461,7 @@ __global__ void delta_prepare_kernel(float* __restrict__ qk, float* __restrict__
     if (e < nv) gate[(size_t)t * nv + e] = sigmoid_f(z[heads * dim + e]);
 }
 
-// The same for steps of many tokens, four neighbouring numbers a thread over `run` tokens in turn: the convolution's weights and inputs wait in
+// The same with four neighbouring numbers a thread over `run` tokens in turn: the convolution's weights and inputs wait in
 // registers from token to token, each head of q and k is dim / 4 neighbouring lanes (a power of two up to 32), whose inputs are read once. grid
 // (runs of tokens, blocks of the quads of q, k and v | of beta's heads | of the decays' quads | of the gate's). Bound by memory: 2,048 tokens,
 // 16 heads of 128 by 128 over 4 key heads move 105 MB in 35 us (3.0 TB/s); an element a thread and token took 113 us.
@@ -559,16 +559,17 @@ extern "C" int hb_delta_prepare(float* qk, float* v, float* beta, float* decay, 
     if (segments > 65535) HB_REFUSE("delta_prepare: %ld segments a token are above 65535", segments);
     dim3 grid(tokens, (unsigned)segments);
     cudaStream_t s = (cudaStream_t)stream;
-    // From 64 tokens on, with two to four taps and rows that 16-byte (bfloat16: 8-byte) reads fit (16 heads of 128 by 128 over 4 key heads,
-    // bfloat16, 2,048 tokens: 35 us, an element a thread 113).
+    // With two to four taps and rows that 16-byte (bfloat16: 8-byte) reads fit, whatever the number of tokens: a head's sum of squares has another
+    // order there than in the kernel above, and a row's bits are not to depend on the rows beside it (16 heads of 128 by 128 over 4 key heads,
+    // bfloat16: 2,048 tokens 37 us, an element a thread 113; eight rows of one token 3.2 and 5.9, one 2.5 and 5.2).
     const size_t four = dtype == HB_F32 ? 16 : 8;
     const int lanes = dim / 4;
-    if (tokens >= 64 && taps >= 2 && taps <= 4 && dim % 4 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && vdim % 4 == 0 && ld % 4 == 0
+    if (taps >= 2 && taps <= 4 && dim % 4 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && vdim % 4 == 0 && ld % 4 == 0
         && (((uintptr_t)qk | (uintptr_t)v | (uintptr_t)decay | (uintptr_t)gate | (uintptr_t)low2 | (uintptr_t)dt_bias) & 15) == 0
         && (((uintptr_t)first | (uintptr_t)conv_state) % four) == 0 && (dtype == HB_F32 || dtype == HB_BF16)) {
         const int nd = heads * dim, nv = heads * vdim, C = 2 * kv_heads * dim + nv;
         const int conv_blocks = (C / 4 + 127) / 128, beta_blocks = (heads + 127) / 128, decay_blocks = (nd / 4 + 127) / 128;
-        const int run = tokens >= 1024 ? 8 : tokens >= 256 ? 4 : 2;
+        const int run = tokens >= 1024 ? 8 : tokens >= 256 ? 4 : tokens >= 128 ? 2 : 1;
         const long segs = (long)conv_blocks + beta_blocks + decay_blocks + (nv / 4 + 127) / 128;
         if (segs <= 65535) {
             const dim3 wide((tokens + run - 1) / run, (unsigned)segs);

@@ -514,3 +514,27 @@ def test_delta_prepare_with_tokens_behind_the_last_row(K):
         K.delta_prepare(*out, *given, rows_of(counts, [1, 0]), dim ** -0.5, 1e-6)
         outs.append(out)
     assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim", [64, 96, 128])
+def test_delta_prepare_does_not_depend_on_the_rows_beside_it(K, dtype, dim):
+    heads, kv_heads, vdim, taps, counts = 4, 2, 32, 4, [1, 1, 5, 63, 64, 30]
+    t, nv = sum(counts), heads * vdim
+    c = 2 * kv_heads * dim + nv
+    first, low2 = rand(t, c + heads, dtype=dtype, seed=1).to(DEV), rand(t, heads * dim + nv, seed=2).to(DEV)
+    conv, dt_bias, rate_log = rand(c, taps, dtype=dtype, seed=3).to(DEV), rand(heads * dim, seed=4).to(DEV), rand(heads, seed=5).to(DEV)
+    carried = rand(len(counts), taps - 1, c, dtype=dtype, seed=6).to(DEV)
+
+    def run(at, counts, slots):
+        n = sum(counts)
+        out = [torch.empty(s, device=DEV) for s in ((n, 2, kv_heads, dim), (n, heads, vdim), (n, heads), (n, heads, dim), (n, nv))]
+        K.delta_prepare(*out, first[at:at + n].contiguous(), conv, carried.clone(), low2[at:at + n].contiguous(), dt_bias, rate_log,
+                        rows_of(counts, slots), dim ** -0.5, 1e-6, carry=True)
+        return out
+
+    together, at = run(0, counts, list(range(len(counts)))), 0
+    for i, n in enumerate(counts):
+        for a, b in zip(run(at, [n], [i]), together):
+            assert torch.equal(a, b[at:at + n]), n
+        at += n
