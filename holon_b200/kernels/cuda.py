@@ -760,15 +760,23 @@ class CudaKernels:
                        self._p(weight), m, n, k, 0, 0)
         elif self.gemm == "tcgen05" and k % 8 == 0:      # the hand-written tensor-memory kernel in place of the library
             self.linear_tcgen05(out, x, weight)
-        elif out.dtype == torch.float32 and n % 4 and n <= 256 and k % 8 == 0 \
+        elif out.dtype == torch.float32 and n % 4 and self.gemm == "auto" and self._odd_takes(m, n) and k % 8 == 0 \
                 and not (x.data_ptr() | weight.data_ptr() | out.data_ptr()) % 16:
-            # rows of an odd number of 32-bit numbers (a router with one gate more): the library has an unaligned kernel for
-            # them only (2,048 rows, 65 x 2,048: 34 us, 20 here)
             self.linear_tcgen05(out, x, weight, pair=False)
         elif out.dtype == torch.float32:                 # the head: bfloat16 operands, 32-bit logits
             torch.mm(x, weight.t(), out_dtype=torch.float32, out=out)
         else:
             torch.mm(x, weight.t(), out=out)
+
+    @staticmethod
+    def _odd_takes(m: int, n: int) -> bool:
+        """Whether a product whose rows are an odd number of 32-bit numbers (a router with one gate more) runs on the tcgen05 kernel:
+        from as many rows on as make the library, which has unaligned kernels only for such rows, take its slow one. Its time jumps at
+        about 48 K results (columns in steps of 32), of more than 160 columns later; one CTA here walks all of k, whatever the rows.
+        Library and tcgen05, us, 2,048 columns of k (4,096 alike): 33 columns, 640 rows 12.9 and 16.6, 768 rows 26.3 and 16.4; 65
+        columns, 256 rows 14.7 and 18.8, 512 rows 28.7 and 20.7, 2,048 rows 37.9 and 19.8; 129 columns, 320 rows 28.3 and 24.3; 255
+        columns, 512 rows 30.3 and 34.4, 640 rows 36.9 and 34.6; 1 column, 1,536 rows 6.0 and 14.0."""
+        return 16 < n <= 256 and m * (-(-n // 32) * 32) >= 48 << 10 and (n <= 160 or m >= 640)
 
     # Elements of a weight up to which a prompt's product takes the activation into its epilogue (2,048 rows: 9,216 x 2,048 71.7 us
     # against the library's 59.7 and 14.7 for the activation; 18,432 x 4,096 218 against 183 and 25).

@@ -728,9 +728,10 @@ def test_sample_follows_the_distribution(K):
             assert int(out[i]) == plain.draw(probs, plain.uniform(1234, i))
 
 
-@pytest.mark.parametrize("m,n,k", [(17, 65, 2048), (300, 33, 96), (129, 255, 1000), (40, 1, 64), (40, 257, 64), (40, 64, 64)])
+@pytest.mark.parametrize("m,n,k", [(17, 65, 2048), (300, 33, 96), (129, 255, 1000), (40, 1, 64), (40, 257, 64), (40, 64, 64),
+                                   (1536, 17, 72), (771, 63, 2048), (513, 65, 1000), (641, 255, 96), (1000, 129, 64)])
 def test_linear_of_an_odd_number_of_32_bit_columns(K, m, n, k):
-    """bfloat16 rows to 32-bit results whose rows are no multiple of 16 bytes (the first four), and their neighbours: 32-bit sums
+    """bfloat16 rows to 32-bit results whose rows are no multiple of 16 bytes, from few and from many rows, and their neighbours: 32-bit sums
     of exact products."""
     x, w = rand(m, k, dtype=torch.bfloat16, seed=n), rand(n, k, dtype=torch.bfloat16, seed=k)
     out = torch.full((m, n), float("nan"), device=DEV)

@@ -93,3 +93,26 @@ def test_parts_of_any_cut():
         most = CudaKernels._long_rows(captured, least, size)
         assert exact[0] <= most[0] and exact[1] <= most[1] and exact[2] <= most[2]
         assert exact[:2] == (sum(n >= least for n in counts), sum(-(-n // size) for n in counts if n >= least))
+
+
+def product(m, n, k=256, out=F32, gemm="auto"):
+    table = Noted()
+    table.gemm = gemm
+    mm = []
+    real, torch.mm = torch.mm, lambda *a, **kw: mm.append("library")
+    try:
+        table.linear(torch.zeros(m, n, dtype=out), torch.zeros(m, k, dtype=torch.bfloat16), torch.zeros(n, k, dtype=torch.bfloat16))
+    finally:
+        torch.mm = real
+    return table.called + mm
+
+
+@pytest.mark.parametrize("n,rows", [(1, None), (15, None), (17, 1536), (33, 768), (63, 768), (65, 512), (97, 384), (129, 308), (162, 640), (255, 640)])
+def test_products_of_an_odd_number_of_32_bit_columns(n, rows):
+    """The library's up to `rows` rows (None: always), and at any number of them where it is asked for."""
+    for m in (17, 64, 256, 307, 383, 511, 639, 767, 1535, 1536, 4096):
+        tcgen05 = rows is not None and m >= rows
+        assert product(m, n) == ["linear_tcgen05" if tcgen05 else "library"], m
+        assert product(m, n, gemm="cublas") == product(m, n, out=torch.bfloat16) == product(m, n, k=252) == ["library"]
+    assert product(2048, 64) == product(2048, 257) == ["library"]
+    assert product(16, n) == ["hb_gemm_bf16_skinny"]
