@@ -994,7 +994,8 @@ class CudaKernels:
         if rows.n_rows > ones:
             # prompt portions: on tcgen05 wherever it takes the sizes (2,048 tokens of 16 heads, rank 512 + 64: 730 us on
             # mma.sync, 219 us on tcgen05; a tile step of either costs the same for few queries as for many)
-            if self.prefill_attention == "tcgen05" and scale > 0 and (t - ones) * heads // 128 + rows.n_rows <= 65535 \
+            tiles = -(-(t - ones) * heads // 128) + rows.n_rows - ones       # (the most that the kernel launches)
+            if self.prefill_attention == "tcgen05" and scale > 0 and tiles <= 65535 and t * heads < 1 << 31 \
                     and self._latent_tcgen05_takes(heads, rank, rot, cache.shape[0], cache.shape[1]):
                 return self._call("hb_latent_attention_tcgen05", self._p(out), self._p(qa), self._p(cache), *common, ones,
                                   rows.n_rows, t, t - ones, *sizes, self._p(sinks))

@@ -116,3 +116,21 @@ def test_products_of_an_odd_number_of_32_bit_columns(n, rows):
         assert product(m, n, gemm="cublas") == product(m, n, out=torch.bfloat16) == product(m, n, k=252) == ["library"]
     assert product(2048, 64) == product(2048, 257) == ["library"]
     assert product(16, n) == ["hb_gemm_bf16_skinny"]
+
+
+@pytest.mark.parametrize("heads,tokens,ones,rows,kernel", [
+    (16, 2048, 0, 1, "hb_latent_attention_tcgen05"), (1, 65534 * 128, 0, 1, "hb_latent_attention_tcgen05"),
+    (1, 65534 * 128 + 1, 0, 1, "hb_latent_attention_bf16"), (1, 65535 * 128, 0, 1, "hb_latent_attention_bf16"),
+    (1, 65532 * 128 + 3, 1, 3, "hb_latent_attention_tcgen05"), (1, 65533 * 128 + 130, 1, 3, "hb_latent_attention_bf16"),
+    (128, 1 << 24, (1 << 24) - 2, (1 << 24) - 1, "hb_latent_attention_bf16")])
+def test_latent_prompts_of_more_tiles_than_a_launch_has(heads, tokens, ones, rows, kernel):
+    """What the tcgen05 kernel refuses (more than 65,535 tiles, or 2^31 queries and heads in a step) stays with the other one."""
+    k, rank = Noted(), 64
+    k._check = lambda *tensors: None
+    k.latent_split = 1
+    k.sms = 148
+    wide = lambda *shape: torch.zeros(1, dtype=torch.bfloat16).expand(*shape)         # noqa: E731
+    i32 = torch.zeros(1, dtype=torch.int32)
+    k.latent_attention(wide(tokens, heads, rank), wide(tokens, heads, rank + 16), wide(2, 64, rank + 16), i32.view(1, 1),
+                       Rows(i32, i32, i32, rows, tokens, ones, 1, 1), 0.1, rank, 0)
+    assert k.called[-1] == kernel
