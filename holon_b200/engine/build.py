@@ -61,10 +61,26 @@ def _peak_of(device, run) -> int:
     return max(0, torch.cuda.max_memory_reserved(device) - reserved, torch.cuda.max_memory_allocated(device) - allocated)
 
 
+def _cuts(tokens: int, rows: int, longest: int, lengths=()) -> list[list[int]]:
+    """Ways to cut a step's `tokens` into at most `rows` rows of at most `longest` tokens: even ones, as few as can be, and for each of
+    `lengths` as many rows of that length as fit, the rest behind them."""
+    even = [tokens // rows + (i < tokens % rows) for i in range(rows)]
+    cuts = [[n for n in even if n]]
+    for n in (longest, *lengths):
+        counts, left = [], tokens
+        while left:
+            fit = max(n, left - (rows - len(counts) - 1) * longest)        # (what the rows behind this one cannot hold)
+            counts.append(left if len(counts) == rows - 1 or left < 2 * n and left <= longest else min(fit, left, longest))
+            left -= counts[-1]
+        cuts.append(counts)
+    return [c for i, c in enumerate(cuts) if c not in cuts[:i]]
+
+
 def _measure(model, ctx, entries, *, page_size: int, max_seqs: int, max_model_len: int, max_step_tokens: int,
              chunk_with_decode: int, dtype, device) -> tuple[int, int]:
     """The activation peaks of (1) the largest step the scheduler can make: `max_step_tokens` prompt tokens in as
-    many rows as may end a prompt in one step, every row sampled; (2) the largest step replayed from a CUDA graph:
+    many rows as may end a prompt in one step, every row sampled, and the same tokens in other cuts, since scratch may grow
+    with a row's length (`costly_rows` of a kernel table: the lengths at which it is largest for the tokens); (2) the largest step replayed from a CUDA graph:
     one token for every sequence beside `chunk_with_decode` prompt tokens. Both run through the engine's own step
     function on pools just large enough to hold them, which are freed again (executor.py:208-234 does the same on
     minimum-size pools)."""
@@ -93,8 +109,8 @@ def _measure(model, ctx, entries, *, page_size: int, max_seqs: int, max_model_le
         for e in batch:
             cache.release(e.slot)
 
-    share = [tokens // rows + (i < tokens % rows) for i in range(rows)]
-    largest = _peak_of(device, lambda: step([n for n in share if n]))
+    cuts = _cuts(tokens, rows, max_model_len - 1, getattr(ctx.kernels, "costly_rows", ()))
+    largest = max(_peak_of(device, lambda counts=counts: step(counts)) for counts in cuts)
     graphed = _peak_of(device, lambda: step(ones + [n for n in portion if n > 0]))
     del runner, cache
     torch.cuda.empty_cache()

@@ -1222,6 +1222,12 @@ class CudaKernels:
     # 16 10.3 and 11.0, 64 17 and 19, 2,048 305 and 568; eleven rows of 16 23 and 52; the generalized rule alike.
     BLOCK_TOKENS = 16
 
+    @property
+    def costly_rows(self) -> tuple[int, ...]:
+        """The lengths of rows whose scratch is largest for the tokens they bring: the shortest that go in parts and leave the last
+        part all but empty."""
+        return self.CHUNK_TOKENS + 1, self.BLOCK_TOKENS + 1
+
     @staticmethod
     def _long_rows(rows, least: int, size: int) -> tuple[int, int, bool]:
         """Of the rows of several tokens: how many bring `least` tokens or more, the parts of `size` tokens these are cut into, and

@@ -398,3 +398,31 @@ def test_the_sampling_kernel_draws_what_the_reference_sampler_drew():
                        full(1.0, torch.float32), full(0.0, torch.float32), as_i32(case["seed"] & 0xFFFFFFFF),
                        as_i32(case["seed"] >> 32), full(case["position"], torch.int32), False)
         assert tokens.tolist() == case["tokens"], case
+
+
+def test_the_measured_peak_covers_one_long_prompt():
+    """A recurrence's scratch grows with a row's length: a prompt of the largest step's tokens needs no more than was measured, although
+    the measured step has as many rows as the engine has seats."""
+    import torch
+    from holon_b200.engine import StepEntry, build
+    from holon_b200.engine.build import _peak_of
+    from holon_b200.weights import RandomSource
+    mixer = {"heads": 16, "dim": 128, "vdim": 128, "decay": [0.99] * 16, "rot": {"base": 10000.0, "dims": 128}}
+    config = {"architecture": "Kasovik", "width": 256, "vocab": 1024, "norm": {"eps": 1e-6},
+              "embedding": {"scale": 1.0, "bigram": {"buckets": 97, "mul_prev": 31, "mul_cur": 7}},
+              "layers": [{"type": "retention", "mixer": mixer, "mlp": {"kind": "dense", "ff": 256, "limit": 7.0}}]}
+    with torch.inference_mode():
+        built = build(RandomSource(config, seed=1, device="cuda:0", dtype=torch.bfloat16), dtype="bfloat16", device="cuda:0", page_size=64,
+                      max_seqs=64, max_model_len=4097, max_step_tokens=4096, memory_fraction=0.05)
+        cache = built.cache
+
+        def step(counts):
+            slots = [cache.admit() for _ in counts]
+            entries = [StepEntry(slot, [5] * n, 0, [n - 1]) for slot, n in zip(slots, counts)]
+            assert all(cache.reserve(slot, n) for slot, n in zip(slots, counts))
+            built.runner.step(entries)
+            for slot in slots:
+                cache.release(slot)
+
+        for counts in ([4096], [2000, 2096], [129] * 31, [200] * 20):
+            assert _peak_of(built.ctx.device, lambda: step(counts)) <= built.memory.activations + (2 << 20), counts

@@ -134,3 +134,23 @@ def test_latent_prompts_of_more_tiles_than_a_launch_has(heads, tokens, ones, row
     k.latent_attention(wide(tokens, heads, rank), wide(tokens, heads, rank + 16), wide(2, 64, rank + 16), i32.view(1, 1),
                        Rows(i32, i32, i32, rows, tokens, ones, 1, 1), 0.1, rank, 0)
     assert k.called[-1] == kernel
+
+
+def test_cuts_of_a_step():
+    """Every cut holds the step's tokens in rows that can be; no other cut needs noticeably more parts than the measured ones."""
+    import random
+    from holon_b200.engine.build import _cuts
+    rng = random.Random(2)
+    for _ in range(300):
+        rows, longest = rng.randint(1, 70), rng.choice([40, 200, 5000])
+        tokens = rng.randint(1, min(4096, rows * longest))
+        lengths = [n for n in (CudaKernels.CHUNK_TOKENS + 1, CudaKernels.BLOCK_TOKENS + 1)]
+        cuts = _cuts(tokens, rows, longest, lengths)
+        assert all(sum(c) == tokens and len(c) <= rows and 1 <= min(c) and max(c) <= longest for c in cuts)
+        for least, size in ((CudaKernels.CHUNK_TOKENS, 64), (CudaKernels.BLOCK_TOKENS, 8)):
+            parts = lambda c: sum(-(-n // size) for n in c if n >= least)             # noqa: E731
+            for _ in range(5):
+                ends = sorted(rng.randint(0, tokens) for _ in range(rng.randint(1, rows) - 1))
+                counts = [b - a for a, b in zip([0, *ends], [*ends, tokens])]
+                if max(counts) <= longest:
+                    assert parts(counts) <= 1.03 * max(map(parts, cuts)) + 2, (tokens, rows, longest, counts, cuts)
