@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) prefill_tcgen05_kernel(
         if (ok && qn > 0) {                                           // (the tensor-memory loads are warp-collective: no lane skips them)
             if (sinks && l > 0.f) l += at_ex2(fmaf(sinks[h], 1.4426950408889634f, -m_used));   // the sink: a weight without a value
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            const bool keep = r < qn && my_tiles > 0 && l > 0.f;
+            const bool keep = r < qn && my_tiles > 0 && l != 0.f;    // (a sum that is no number leaves none: O is none then, too)
             bf16* o_row = out + ((size_t)(t0 + g * AT_BM + (r < qn ? r : 0)) * gridDim.x + blockIdx.x) * AT_D;
 #pragma unroll
             for (int c = 0; c < AT_D / 32; ++c) {

@@ -739,3 +739,21 @@ def test_linear_of_an_odd_number_of_32_bit_columns(K, m, n, k):
     want = x.double() @ w.double().T
     assert K.tcgen05_status() == 0
     assert (out.cpu() - want).abs().max().item() <= 2 ** -22 * k
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("what", [0, 1])
+def test_prefill_attention_of_what_is_no_number(K, bad, what):
+    """A cached key (0) or value (1) that is none: the queries that see it have no answer (and not zeros), the other rows keep their bits."""
+    q, kv, table, rows = paged_case(8, 2, 128, 64, [(100, 70), (30, 200), (0, 40)], torch.bfloat16, seed=4)
+    q[..., 3] = q[..., 3].abs() + 1.0
+    outs = []
+    for plant in (False, True):
+        if plant:
+            kv[table[rows.row_slot[1], 0], what, 0, 10, 3] = bad
+        out = torch.full_like(q, 7.0, device=DEV)
+        K.paged_attention(out, q.to(DEV), kv.to(DEV), table.to(DEV), on_device(rows), 0.1, 0)
+        outs.append(out.cpu())
+    assert outs[0].isfinite().all() and K.tcgen05_status() == 0
+    assert not outs[1][70:270, :4, 3].isfinite().any() and (what or outs[1][70:270, :4].isnan().all())
+    assert torch.equal(outs[1][:70], outs[0][:70]) and torch.equal(outs[1][270:], outs[0][270:]) and torch.equal(outs[1][70:270, 4:], outs[0][70:270, 4:])
