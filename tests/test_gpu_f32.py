@@ -40,6 +40,12 @@ def test_products_do_not_depend_on_the_kernel(K, n, k):
         assert torch.equal(out, whole[:m]), m
 
 
+@pytest.mark.parametrize("k", [4100, 6144])
+def test_products_whose_stages_are_filled_again(K, k):
+    """Few rows and columns with more pieces of k than the ring of the kernel for few rows has stages."""
+    test_products_do_not_depend_on_the_kernel(K, 130, k)
+
+
 @pytest.mark.parametrize("m", [3, 16, 17, 200])
 @pytest.mark.parametrize("heads,n,k", [(5, 64, 36), (40, 130, 128), (3, 96, 30)])
 def test_products_per_head_on_views(K, m, heads, n, k):
@@ -86,6 +92,20 @@ def test_attention_float32_does_not_depend_on_the_cut(K, window):
         K.paged_attention(out, q[skip:].contiguous().to(DEV), kv.to(DEV), table.to(DEV), on_device(part), 0.09, window)
         outs.append(out)
     assert torch.equal(outs[0][33:], outs[1])
+
+
+@pytest.mark.parametrize("window", [0, 50])
+def test_attention_float32_of_a_portion_of_one_token(K, window):
+    """It runs as a one-token row does, with the keys in another order: the same up to rounding."""
+    from holon_b200.engine.batch import Rows
+    q, kv, table, rows = paged_case(4, 2, 128, 16, [(160, 70)], torch.float32, seed=3)
+    outs = []
+    for n in (70, 1):
+        part = Rows(rows.row_slot, torch.tensor([0, n], dtype=torch.int32), rows.kv_len, 1, n, int(n == 1), n, 230)
+        out = torch.empty(n, 4, 128, device=DEV)
+        K.paged_attention(out, q[70 - n:].contiguous().to(DEV), kv.to(DEV), table.to(DEV), on_device(part), 0.09, window)
+        outs.append(out)
+    assert (outs[0][69] - outs[1][0]).abs().max().item() <= 2e-6
 
 
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])

@@ -38,7 +38,7 @@ def plain(qk, v, state, counts, slots, decay, beta, rate):
 
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 64, 64), (3, 3, 128, 129), (5, 5, 256, 20), (6, 2, 128, 128), (2, 1, 64, 7),
-                                                     (40, 8, 64, 70), (3, 1, 36, 10)])
+                                                     (40, 8, 64, 70), (3, 1, 36, 10), (10, 5, 256, 70)])
 def test_against_the_formula(K, form, heads, kv_heads, dim, vdim, monkeypatch):
     for name in ("CHUNK_TOKENS", "BLOCK_TOKENS"):                                      # (short rows too)
         monkeypatch.setattr(type(K), name, 2, raising=False)
