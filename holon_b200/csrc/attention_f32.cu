@@ -6,12 +6,14 @@
 // lanes share a key and the 256 such groups of lanes of a cluster walk the row's keys, each with a softmax of its own, merged
 // per block and then through distributed shared memory.
 // Rows of several tokens: a block per (64 queries, head); 64 keys at a time in shared memory, 4 x 4 scores a thread, then
-// 4 rows x D / 16 columns of the output. Bound by the multiply-adds, next to it by shared memory's bandwidth.
-// Measured on 28 layers of 16 heads of 128 over 8 kv heads, two prompts of 333 and 208 tokens and four steps behind them: 98 us
-// a layer for the prompts, 11.4 us for the two one-token rows (18.8 with one block in a cluster's place); a warp per query and head, a lane per key, took 755 us on
+// 4 rows x D / 16 columns of the output. 15 % of the multiply-adds' rate: a tile's keys, then its values, are loaded between barriers with
+// nothing in flight beside the arithmetic.
+// Measured on 28 layers of 16 heads of 128 over 8 kv heads, two prompts of 333 and 208 tokens and four steps behind them: 95 us
+// a layer for the prompts, 9.7 us for the two one-token rows (18.8 with one block in a cluster's place); a warp per query and head, a lane per key, took 755 us on
 // average over both.
 // Which groups or tiles a key falls into depends on its position alone, so a token's result does not depend on the rows
-// beside it nor on where its prompt was cut.
+// beside it nor on where its prompt was cut into portions of two tokens and more (a portion of one goes to the other kernel, whose
+// order of the keys is another).
 // A key that scores minus infinity (its product with the query overflowed) weighs nothing; a query whose keys all do has no answer: NaN.
 #include <cooperative_groups.h>
 

@@ -1,5 +1,5 @@
-// Paged attention for any sizes on CUDA cores, 32-bit arithmetic throughout: the float32 engine's attention, and
-// the bfloat16 engine's for shapes its tensor-core kernels refuse. One warp per (query token, query head).
+// Paged attention for any sizes on CUDA cores, 32-bit arithmetic throughout: for shapes and addresses that the float32 engine's
+// kernels (attention_f32.cu) and the bfloat16 engine's tensor-core kernels do not take. One warp per (query token, query head).
 // Each lane scores one key of a block of 32; the block's softmax weights then sweep the values, each lane owning
 // every 32nd dimension of the output.
 #include "common.cuh"

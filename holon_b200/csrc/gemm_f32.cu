@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(128) gemm_f32_kernel(float* __restrict__ out, 
 // ---------------------------------------------------------------- few rows
 // Bound by reading w once. A block of 256 threads takes 8 columns and all of k: a thread sums one segment of one column
 // for a quarter of the rows, over pieces of 64 of each segment that a ring of stages brings by cp.async: three where many
-// blocks share an SM, six where there are few blocks (all of k up to 3,072 is then on its way at once). Two rows, the same
+// blocks share an SM, six where there are few blocks (the first five, all of k up to 2,560, are then on their way at once). Two rows, the same
 // model's step: 7.2 us for a product of 1,024 columns (10 with three stages), 13.2 on average for the wider ones, the head of 151,936
 // columns among them (167 us, 3.7 TB/s); as tiles of 64 rows each was a serial walk over k.
 #define FEW_COLS 8

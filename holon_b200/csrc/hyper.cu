@@ -30,8 +30,8 @@ __global__ void __launch_bounds__((S > 0 && S <= 4) ? 1024 : 256) hyper_mix_norm
     if constexpr (S > 0 && S <= 4) {
         if (dim <= (int)blockDim.x * 4) {
             // A row that the block's threads hold whole (four columns a thread): coefficients straight from global
-            // memory, every load of the row in flight at once, the norm's weight read before the block-wide sum; the
-            // values and their order are those of the general path below.
+            // memory, every load of the row in flight at once, the norm's weight read before the block-wide sum. A column's
+            // values are those of the general path below; the squares are added in another order where a thread has neighbouring columns.
             float cm[S * S], co[S], ci[S];
 #pragma unroll
             for (int i = 0; i < S * S; ++i) cm[i] = mix ? __ldg(mix + i) : 0.f;
@@ -181,7 +181,7 @@ static int hyper_launch(void* out, float* xs, const float* src, const void* y, c
                         const float* inc, const void* weight, float eps, float offset, const int32_t* index, int rows,
                         int dim, int streams, cudaStream_t s) {
     // up to four streams: four columns a thread hold a whole row of up to 4,096; more streams: the kernel with many registers
-    const int wide = dim > 2048 && rows <= 512 ? 1024 : dim > 1024 ? 512 : dim > 512 ? 256 : 128;   // (many rows: blocks of 512 fill the SMs better)
+    const int wide = dim > 2048 && rows <= 512 ? 1024 : dim > 1024 ? 512 : dim > 512 ? 256 : 128;   // (many rows: blocks of 512 filled the SMs better with a column a load; such rows of more than 2,048 columns take the general path)
     const int threads = streams <= 4 ? wide : (wide < 256 ? wide : 256);
     const size_t smem = (size_t)dim * sizeof(float);
     // 2,048 rows of four streams of 2,048 columns, 151 MB: 23 us (6.5 TB/s), a column a load 37 us.

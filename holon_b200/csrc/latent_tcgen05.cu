@@ -25,7 +25,6 @@
 
 #define LT_BM 128                                 // (token, head) pairs a CTA
 #define LT_BN 64                                  // cache rows a tile
-#define LT_MAX_BLOCKS 12                          // 64-column blocks of a row: what shared memory holds of queries and one tile
 #define LT_STAGES 3
 #define LT_Q_BLOCK (LT_BM * 128)                  // bytes of a [128 x 64] block of queries
 #define LT_K_BLOCK (LT_BN * 128)
@@ -313,8 +312,8 @@ extern "C" int hb_latent_tcgen05_status(unsigned int* status) {
 // Whether the kernel takes these sizes (host only).
 extern "C" int hb_latent_tcgen05_takes(int heads, int rank, int rot, int pages, int page_size) {
     if (rank < 64 || rank > 512 || rank % (rank <= 256 ? 64 : 128) || rot < 16 || rot % 16 || page_size % LT_BN || heads < 1) return 0;
-    const int blocks = (rank + rot + 63) / 64;
-    return blocks <= LT_MAX_BLOCKS && blocks * (LT_Q_BLOCK + LT_K_BLOCK) + 1024 <= LT_SMEM_MAX - 1024
+    const long blocks = ((long)rank + rot + 63) / 64;
+    return blocks * (LT_Q_BLOCK + LT_K_BLOCK) + 1024 <= LT_SMEM_MAX - 1024       // the queries and one tile: up to nine blocks
         && (long)pages * page_size <= 0x7fffffffL;
 }
 

@@ -514,6 +514,42 @@ def state_space(k, args) -> None:
             print(f"state space {len(counts)} row(s) of {counts[0]:5d} tokens, {heads} heads of {n} x {vdim}, {name:14s}: {us:8.1f} us  ({moved / us / 1e3:7.0f} GB/s)")
 
 
+def f32(k, args) -> None:
+    """The float32 engine's products (`--hidden` columns of k, as many and four times as many results) and attention (`--heads` heads of
+    `--dim` over `--kv-heads`; one prompt of `--rows` tokens, or so many one-token rows of `--context` tokens up to 16)."""
+    dev, n = k.device, args.hidden
+    for t in args.rows:
+        for wide in (n, 4 * n):
+            sets = [(torch.randn(t, n, device=dev), torch.randn(wide, n, device=dev), torch.empty(t, wide, device=dev)) for _ in range(4)]
+            us = in_graph([lambda s=s: k.linear(s[2], s[0], s[1]) for s in sets], 3)
+            print(f"float32 product {t:5d} rows, {wide} x {n}: {us:8.1f} us  ({2 * t * n * wide / us / 1e6:5.1f} TFLOP/s, {4 * n * wide / us / 1e3:5.0f} GB/s of weights)")
+        counts, lens = ([1] * t, [args.context] * t) if t <= 16 else ([t], [t])
+        batch, per = _rows_on(dev, counts, lens), -(-max(lens) // 64)
+        table = torch.arange(len(counts) * per, device=dev, dtype=torch.int32).view(len(counts), per).contiguous()
+        pools = [torch.randn(len(counts) * per + 1, 2, args.kv_heads, 64, args.dim, device=dev) for _ in range(3)]
+        q = torch.randn(t, args.heads, args.dim, device=dev)
+        out = torch.empty_like(q)
+        us = in_graph([lambda kv=kv: k.paged_attention(out, q, kv, table, batch, args.dim ** -0.5, 0) for kv in pools], 3)
+        print(f"float32 attention {len(counts)} row(s) of {counts[0]} over {lens[0]} tokens, {args.heads} heads of {args.dim} over {args.kv_heads}: {us:8.1f} us")
+
+
+def latent(k, args) -> None:
+    """Latent attention (`latent_attention`) of one prompt of `--rows` tokens, `--heads` heads over rank 512 + 64: the tcgen05 kernel and
+    the mma.sync one."""
+    dev, heads = k.device, args.heads
+    for t in args.rows:
+        per = -(-t // 64)
+        table, batch = torch.arange(per, device=dev, dtype=torch.int32).view(1, per).contiguous(), _rows_on(dev, [t], [t])
+        sets = [(torch.empty(t, heads, 512, device=dev, dtype=torch.bfloat16), torch.randn(t, heads, 576, device=dev).bfloat16(),
+                 torch.randn(per + 1, 64, 576, device=dev).bfloat16()) for _ in range(3)]
+        for kernel in ("tcgen05", "mma"):
+            k.prefill_attention, before = kernel, k.prefill_attention
+            us = in_graph([lambda s=s: k.latent_attention(*s, table, batch, 576 ** -0.5, 512, 0) for s in sets], 2)
+            k.prefill_attention = before
+            print(f"latent attention, {t} tokens of {heads} heads, rank 512 + 64, {kernel}: {us:8.1f} us  ({t * (t + 1) * heads * 1088 / us / 1e6:5.0f} TFLOP/s)")
+    print("status", k.tcgen05_status())
+
+
 def out_norm(k, args) -> None:
     """The norm on an output that is added to the stream (`out_norm_add`), and on a pair of outputs (`out_norm_pair_add`), beside
     `add_rmsnorm`, over rows of `--hidden`. Two sets of buffers alternate; many rows are larger than the L2."""
@@ -565,7 +601,7 @@ def expert_glu(k, args) -> None:
 
 def main() -> None:
     ap = argparse.ArgumentParser(description=__doc__.split("\n\n")[0])
-    ap.add_argument("what", choices=("decode_attention", "gemm", "prefill_attention", "chain", "layer", "scan", "layernorm", "expert_glu", "maps", "state_space", "out_norm"))
+    ap.add_argument("what", choices=("decode_attention", "gemm", "prefill_attention", "chain", "layer", "scan", "layernorm", "expert_glu", "maps", "state_space", "out_norm", "f32", "latent"))
     ap.add_argument("--heads", type=int, default=16, help="scan: value heads")
     ap.add_argument("--kv-heads", type=int, default=4, help="scan: query/key heads of the delta rule")
     ap.add_argument("--dim", type=int, default=128, help="scan: key size")
@@ -608,6 +644,9 @@ def main() -> None:
         elif args.what == "out_norm":
             args.rows = args.rows or [8, 2048, 8192]
             out_norm(k, args)
+        elif args.what in ("f32", "latent"):
+            args.rows = args.rows or [2048]
+            (f32 if args.what == "f32" else latent)(k, args)
         elif args.what == "scan":
             args.rows = args.rows or [2048, 256, 1]
             scan(k, args)
