@@ -171,6 +171,20 @@ int hb_latent_attention_tcgen05(void* out, const void* qa, const void* cache, co
                                 float scale, int window, const float* sinks, hb_stream stream);
 int hb_latent_tcgen05_takes(int heads, int rank, int rot, int pages, int page_size);
 int hb_latent_tcgen05_status(unsigned int* status);
+// The same with every head's keys and values made first (csrc/latent_prompt.cu), for sizes that hb_latent_prompt_takes answers
+// with 1. hb_latent_gather: the cache rows that rows row0 .. rows - 1 of the batch see, each request's from its window's first tile
+// of 64 on, padded to whole tiles by zeros, one request after the other: out [total, dk]. hb_latent_prompt: out [tokens, heads, vdim];
+// q [tokens, q_ld] holds per head [dim own | rot] query entries (the first dim are read), qa [tokens, heads, rank + rot] the rotated ones behind
+// column rank, keys_values [total, heads (dim + vdim)] all heads' keys, then all heads' values, lat the gathered rows.
+int hb_latent_prompt_takes(int dim, int rot, int vdim, int rank);
+int hb_latent_gather(void* out, const void* cache, const int32_t* block_table, int table_stride, const int32_t* row_slot,
+                     const int32_t* query_start, const int32_t* kv_len, int row0, int rows, int dk, int pages, int page_size,
+                     int window, int total, hb_stream stream);
+int hb_latent_prompt(void* out, const void* q, int q_ld, const void* qa, const void* keys_values, const void* lat,
+                     const int32_t* query_start, const int32_t* kv_len, int row0, int rows, int q_tiles, int tokens, int heads,
+                     int dim, int rot, int vdim, int rank, int total, float scale, int window, int tile_q, const float* sinks,
+                     hb_stream stream);
+int hb_latent_prompt_status(unsigned int* status);
 
 // The same on tensor cores in bfloat16 (csrc/latent_bf16.cu) for rows row0 .. row1 - 1 of the batch, which bring `tokens`
 // tokens in all, the first of them token `first_token` of the step; rank and rot multiples of 16, rank up to 512.

@@ -857,7 +857,7 @@ class CudaKernels:
         out = 0
         for name in ("hb_gemm_tcgen05_status", "hb_gemm_tcgen05_pair_status", "hb_attention_tcgen05_status",
                      "hb_gemm_chain_status", "hb_gemm_tickets_status", "hb_gemm_mid_status", "hb_experts_tcgen05_status", "hb_attention_maps_status",
-                     "hb_latent_tcgen05_status"):
+                     "hb_latent_tcgen05_status", "hb_latent_prompt_status"):
             status = ctypes.c_uint(0)
             if getattr(self.lib, name)(ctypes.byref(status)):
                 raise KernelError(self.lib.hb_last_error().decode())
@@ -964,8 +964,9 @@ class CudaKernels:
                 self.flush()
             torch.bmm(x.transpose(0, 1), w.transpose(1, 2), out=out.transpose(0, 1))
 
-    def latent_attention(self, out, qa, cache, block_table, rows, scale, rank, window, sinks=None) -> None:
-        """`sinks` (float32 [heads], or None): exp(sinks[h]) stands in each head's softmax denominator besides."""
+    def latent_attention(self, out, qa, cache, block_table, rows, scale, rank, window, sinks=None, portions=True) -> None:
+        """`sinks` (float32 [heads], or None): exp(sinks[h]) stands in each head's softmax denominator besides. `portions` False:
+        only the rows of one token, the first `rows.n_decode`."""
         self._check(out, qa, cache, block_table, rows.row_slot, rows.query_start, rows.kv_len, sinks)
         self._f32("latent_attention", sinks)
         if sinks is not None and sinks.shape != (qa.shape[1],):
@@ -991,7 +992,7 @@ class CudaKernels:
                 if splits > 1 else None
             self._call("hb_latent_attention_bf16", self._p(out), self._p(scratch), self._p(qa), self._p(cache), *common,
                        0, ones, 0, ones, *sizes, splits, self._p(sinks))
-        if rows.n_rows > ones:
+        if rows.n_rows > ones and portions:
             # prompt portions: on tcgen05 wherever it takes the sizes (2,048 tokens of 16 heads, rank 512 + 64: 730 us on
             # mma.sync, 219 us on tcgen05; a tile step of either costs the same for few queries as for many)
             tiles = -(-(t - ones) * heads // 128) + rows.n_rows - ones       # (the most that the kernel launches)
@@ -1001,6 +1002,69 @@ class CudaKernels:
                                   rows.n_rows, t, t - ones, *sizes, self._p(sinks))
             self._call("hb_latent_attention_bf16", self._p(out), None, self._p(qa), self._p(cache), *common, ones,
                        rows.n_rows, ones, t - ones, *sizes, 1, self._p(sinks))
+
+    # Cache rows a new token up to which keys and values are made of them: as far as measured, this form is the faster one (rank 512, 16 and 32
+    # heads of 128 + 64, in us with all products, folded and made: 512 tokens behind 3,584 227 and 97, 423 and 122; 128 behind 384 40 and 21,
+    # 42 and 23; 64 tokens alone 16 and 13). With more rows a token, making them is most of the work.
+    LATENT_KEYS = 8
+    LATENT_SCRATCH = 512 << 20                # bytes of keys, values and gathered rows a call may take
+
+    def latent_expands(self, rows, heads, dim, rot, vdim, rank, window, scale, *tensors) -> bool:
+        """Whether a step's prompt portions go through `latent_prompt` (every head's keys and values made of the cache rows they see)
+        rather than through folded queries: bfloat16 heads of the sizes its kernel has, rows whose lengths the host knows (not
+        under a graph that serves every cut of its tokens), and few enough rows seen for the tokens that see them. `tensors`: what the
+        kernel reads in 16-byte pieces."""
+        if rows.n_rows == rows.n_decode or rows.host_kv_len is None or rows.host_query_start is None or "any cut" in rows.plan \
+                or self.prefill_attention != "tcgen05" or self.attention_bf16 != "fast" or not scale > 0 \
+                or any(t.dtype != torch.bfloat16 or t.data_ptr() % 16 or t.stride(0) % 8 for t in tensors):
+            return False
+        key = ("latent prompt", dim, rot, vdim, rank)
+        if key not in self._splits:
+            self._splits[key] = int(self.lib.hb_latent_prompt_takes(dim, rot, vdim, rank))
+        total = self._latent_rows(rows, window)
+        return bool(self._splits[key]) and total <= self.LATENT_KEYS * (rows.n_tokens - rows.n_decode) + 64 * (rows.n_rows - rows.n_decode) \
+            and 2 * total * (heads * (dim + vdim) + rank + rot) <= self.LATENT_SCRATCH and self._query_tiles(rows, 128) <= 65535
+
+    @staticmethod
+    def _latent_rows(rows, window: int) -> int:
+        """The cache rows that the portions see, each request's in whole tiles of 64 from its window's first tile on."""
+        key = ("latent rows", window)
+        if key not in rows.plan:
+            qs, lens, total = rows.host_query_start, rows.host_kv_len, 0
+            for b in range(rows.n_decode, rows.n_rows):
+                n, new = int(lens[b]), int(qs[b + 1]) - int(qs[b])
+                first = max(0, n - new - window + 1) // 64 * 64 if window > 0 else 0
+                total += -(-(n - first) // 64) * 64
+            rows.plan[key] = total
+        return rows.plan[key]
+
+    def latent_prompt(self, out, q, qa, cache, block_table, rows, scale, weight, dim, vdim, rank, window, sinks=None) -> None:
+        """Latent attention of the step's portions (csrc/latent_prompt.cu), where `latent_expands` says so: out [tokens, heads, vdim];
+        q [tokens, >= heads (dim + rot)] (a view of rows that may be wider), qa [tokens, heads, rank + rot] with the rotated query parts,
+        weight [heads (dim + vdim), rank]: every head's W_uk, then every head's W_uv."""
+        self._check(out, qa, cache, block_table, rows.row_slot, rows.query_start, rows.kv_len, sinks, weight)
+        self._f32("latent_prompt", sinks)
+        t, heads, dk = qa.shape
+        rot = dk - rank
+        if out.shape != (t, heads, vdim) or q.shape[0] != t or q.shape[1] < heads * (dim + rot) or q.stride(1) != 1 or q.get_device() != self._index \
+                or cache.dim() != 3 or cache.shape[2] != dk or weight.shape != (heads * (dim + vdim), rank) \
+                or not (out.dtype == q.dtype == qa.dtype == cache.dtype == weight.dtype == torch.bfloat16) \
+                or (sinks is not None and sinks.shape != (heads,)):
+            raise KernelError("latent_prompt: out [tokens, heads, vdim], q [tokens, >= heads (dim + rot)], qa [tokens, heads, rank + rot], "
+                              "cache [pages, page_size, rank + rot], weight [heads (dim + vdim), rank], bfloat16; sinks float32 [heads]")
+        total, ones = self._latent_rows(rows, window), rows.n_decode
+        lat = torch.empty(total, dk, dtype=q.dtype, device=self.device)
+        self._call("hb_latent_gather", self._p(lat), self._p(cache), self._i32(block_table, "block_table"), block_table.shape[1],
+                   self._i32(rows.row_slot, "row_slot"), self._i32(rows.query_start, "query_start"), self._i32(rows.kv_len, "kv_len"),
+                   ones, rows.n_rows, dk, cache.shape[0], cache.shape[1], int(window), total)
+        made = torch.empty(total, heads * (dim + vdim), dtype=q.dtype, device=self.device)
+        torch.mm(lat[:, :rank], weight.t(), out=made)
+        tile_q, tiles = 256, self._query_tiles(rows, 256)
+        if self.prefill_tile == 128 or (self.prefill_tile is None and 4 * heads * tiles < 3 * self.sms):
+            tile_q, tiles = 128, self._query_tiles(rows, 128)
+        self._call("hb_latent_prompt", self._p(out), self._p(q), q.stride(0), self._p(qa), self._p(made), self._p(lat),
+                   self._i32(rows.query_start, "query_start"), self._i32(rows.kv_len, "kv_len"), ones, rows.n_rows, tiles, t, heads, dim, rot,
+                   vdim, rank, total, ctypes.c_float(scale), int(window), tile_q, self._p(sinks))
 
     def _latent_tcgen05_takes(self, *sizes: int) -> bool:
         key = ("latent", *sizes)

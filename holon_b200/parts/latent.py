@@ -9,8 +9,10 @@ unrotated) | q_h^r (rot_dim, rotated)], keys k_{h,j} = [W_uk,h c_j | k_r,j] and 
 
 Because W_uk,h and W_uv,h act on the cached row only, they are applied on the query's side: a_h(i) = W_uk,hᵀ q_h^u(i)
 (`rank` numbers) makes q_h^u · W_uk,h c_j = a_h · c_j, so every head attends over the same rows [c_j | k_r,j] with
-the query [a_h | q_h^r], the attention's value is c_j itself, and W_uv,h is applied once to the weighted sum. Keys and
-values per head are never made; that holds for prompts and for decoding alike.
+the query [a_h | q_h^r], the attention's value is c_j itself, and W_uv,h is applied once to the weighted sum. So one-token rows
+never make keys and values per head. A prompt's tokens share the work of making them, and attention over keys of dim + rot_dim
+and values of vdim is a third of that over the folded ones: where the kernel table offers it (`latent_expands`), the
+portions of a step go that way; the cache holds the same rows.
 
 A layer without a down-projection of its own (`own_latent=False`) reads the cache entry another layer fills (the
 run order says which) with its own W_uk, W_uv, queries, gate and output product.
@@ -51,8 +53,8 @@ class LatentAttention(Part):
             self.q_norm = self.add_child("q_norm", ctx.part(norm, dim=q_rank))
             self.uq = self.add_child("up_q", Linear(ctx, "weight", q_rank, {"uq": heads * (dim + rot_dim)}))
         self.sink = self.add_param("sink", (heads,), "coef") if sink else None
-        self.uk = self.add_param("uk", (heads * dim, rank), "matrix")
-        self.uv = self.add_param("uv", (heads * vdim, rank), "matrix")
+        self.ukv = self.add_param("ukv", (heads * (dim + vdim), rank), "matrix",
+                                  {"uk": (0, heads * dim), "uv": (heads * dim, heads * (dim + vdim))})
         self.out = self.add_child("out", Linear(ctx, "weight", heads * vdim, {"o": hidden}))
         self.latent_norm = self.add_child("latent_norm", ctx.part(norm, dim=rank)) if own_latent else None
         self.position = self.add_child("position", ctx.part(position, head_dim=rot_dim)) if position and rot_dim else None
@@ -69,8 +71,8 @@ class LatentAttention(Part):
 
     def finalize(self) -> None:
         super().finalize()
-        if self.uk.tensor is not None:
-            self.uk_t = self.uk.tensor.view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
+        if self.ukv.tensor is not None:
+            self.uk_t = self.ukv.tensor[:self.heads * self.dim].view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
 
     def cache(self) -> PagedLatent:
         return PagedLatent(self.rank, self.rot_dim, self.window)
@@ -108,13 +110,19 @@ class LatentAttention(Part):
                              cq_weight=self.q_norm.weight.tensor, **neighbours)
             q = self.uq.forward(cq)
             k.latent_prepare(qa, q, heads, dim, rot, rank, -1, *turn, None, 0.0, None, None, **neighbours)
-        q_u = q[:, :heads * (dim + rot)].view(t, heads, dim + rot)[:, :, :dim]
-        k.linear_heads(qa[:, :, :rank], q_u, self.uk_t)                   # a_h = W_uk,hᵀ q_h^u
-        mix = ctx.empty(t, heads, rank)
         sinks = {"sinks": self.sink.tensor} if self.sink is not None else {}
-        k.latent_attention(mix, qa, cache.kv, cache.group.block_table, step.rows, self.scale, rank, self.window, **sinks)
-        o = ctx.empty(t, heads, vdim)
-        k.linear_heads(o, mix, self.uv.tensor.view(heads, vdim, rank))    # W_uv,h on the weighted sum of latents
+        pages, rows, uv = (cache.kv, cache.group.block_table, step.rows), step.rows, self.ukv.tensor[heads * dim:].view(heads, vdim, rank)
+        o, folded = ctx.empty(t, heads, vdim), t                          # `folded`: tokens whose queries are folded, the first ones
+        expands = getattr(k, "latent_expands", None)
+        if expands is not None and expands(rows, heads, dim, rot, vdim, rank, self.window, self.scale, q, qa, o, cache.kv, self.ukv.tensor):
+            k.latent_prompt(o, q, qa, *pages, self.scale, self.ukv.tensor, dim, vdim, rank, self.window, **sinks)
+            folded, sinks["portions"] = rows.n_decode, False
+        if folded:
+            q_u = q[:folded, :heads * (dim + rot)].view(folded, heads, dim + rot)[:, :, :dim]
+            k.linear_heads(qa[:folded, :, :rank], q_u, self.uk_t)         # a_h = W_uk,hᵀ q_h^u
+            mix = ctx.empty(t, heads, rank)
+            k.latent_attention(mix, qa, *pages, self.scale, rank, self.window, **sinks)
+            k.linear_heads(o[:folded], mix[:folded], uv)                  # W_uv,h on the weighted sum of latents
         o = o.view(t, heads * vdim)
         if self.gate:
             k.sigmoid_gate(o, first[:, n_q:n_q + n_g])
