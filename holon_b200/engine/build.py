@@ -155,4 +155,4 @@ def build(source, *, dtype: str, device, kernels=None, page_size: int, max_seqs:
                          state_memory=state_memory, pages=pages, prefix_cache=prefix_cache)
     free_after = torch.cuda.mem_get_info(device)[0] if device.type == "cuda" else None
     memory = Memory(weight_bytes, cache.bytes, activations, graphs, free_before, free_after)
-    return Built(config, model, cache, Runner(model, cache, ctx, max_step_tokens), ctx, weight_bytes, memory)
+    return Built(config, model, cache, Runner(model, cache, ctx, max_step_tokens, cuda_graphs), ctx, weight_bytes, memory)
