@@ -103,6 +103,98 @@ __global__ void talking_prepare_kernel(T* __restrict__ q_out, T* __restrict__ kv
     }
 }
 
+// The same for sizes up to 128, four neighbouring channels a lane (key and value sizes, rotated channels and, half-split, half of them
+// multiples of 4; pointers on 16-byte boundaries): a half-split pair's other member comes from its lane, neighbours are at hand.
+template <typename T>
+__global__ void __launch_bounds__(256) talking_prepare4_kernel(T* __restrict__ q_out, T* __restrict__ kv, float* __restrict__ keep,
+                                        const T* __restrict__ qkv, const void* __restrict__ bias, int bias_f32,
+                                        const void* __restrict__ q_weight, const void* __restrict__ k_weight, int weight_f32,
+                                        float eps, const int32_t* __restrict__ positions, const float* __restrict__ table,
+                                        int rot_dims, int table_rows, int interleaved, const float* __restrict__ first,
+                                        const float* __restrict__ blend, const int32_t* __restrict__ write_index,
+                                        int pages, int page_size, int tokens, int heads, int kv_heads, int kd, int vd) {
+    const int lane = threadIdx.x & 31, slots = heads + 2 * kv_heads, d = lane * 4;
+    const long item = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (item >= (long)tokens * slots) return;
+    const int t = (int)(item / slots), slot = (int)(item % slots);
+    const T* row = qkv + (size_t)t * (heads * kd + kv_heads * (kd + vd));
+    const long w = write_index ? write_index[t] : -1;
+    const bool stored = w >= 0 && w < (long)pages * page_size, is_v = slot >= heads + kv_heads, is_q = slot < heads;
+    const int head = is_q ? slot : is_v ? slot - heads - kv_heads : slot - heads;
+    const int at = (is_q ? 0 : heads * kd) + (is_v ? kv_heads * kd + head * vd : head * kd) + d;
+    const bool mine = d < (is_v ? vd : kd);
+    float x[4] = {0.f, 0.f, 0.f, 0.f}, b[4];
+    auto load4 = [](const void* p, int f32, int i, float (&v)[4]) {
+        if (f32) Vec4<float>::load((const float*)p + i, v);
+        else Vec4<bf16>::load((const bf16*)p + i, v);
+    };
+    if (mine) {
+        Vec4<T>::load(row + at, x);
+        if (bias) {
+            load4(bias, bias_f32, at, b);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] += b[e];
+        }
+    }
+    T* cell = stored ? kv + (((size_t)(w / page_size) * kv_heads + (is_q ? 0 : head)) * page_size + w % page_size) * (kd + vd) : nullptr;
+    if (is_v) {
+        if (!mine) return;
+        const size_t kept = ((size_t)t * kv_heads + head) * vd + d;
+        if (keep) Vec4<float>::store(keep + kept, x);
+        if (blend) {
+            const float lam = blend[0];
+            Vec4<float>::load(first + kept, b);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] = (1.f - lam) * x[e] + lam * b[e];
+        }
+        if (cell) Vec4<T>::store(cell + kd + d, x);
+        return;
+    }
+    const void* weight = is_q ? q_weight : k_weight;
+    if (weight) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss = fmaf(x[e], x[e], ss);
+        const float r = rsqrtf(warp_sum(ss) / (float)kd + eps);
+        if (mine) {
+            load4(weight, weight_f32, d, b);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] = x[e] * r * b[e];
+        }
+    }
+    if (table) {
+        int pos = positions[t];
+        pos = pos < 0 ? 0 : (pos >= table_rows && table_rows > 0 ? table_rows - 1 : pos);
+        const float* cs = table + (size_t)pos * rot_dims;
+        const int half = rot_dims >> 1;
+        if (interleaved) {
+            if (d < rot_dims) {
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                    const float co = cs[(d + e) >> 1], si = cs[half + ((d + e) >> 1)], u = x[e], v = x[e + 1];
+                    x[e] = u * co - v * si;
+                    x[e + 1] = v * co + u * si;
+                }
+            }
+        } else {
+            const bool lead = d < half;
+            const int from = lead ? lane + (half >> 2) : lane - (half >> 2);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) b[e] = __shfl_sync(0xffffffffu, x[e], from & 31);
+            if (d < rot_dims) {
+                float co[4], si[4];
+                Vec4<float>::load(cs + (lead ? d : d - half), co);
+                Vec4<float>::load(cs + half + (lead ? d : d - half), si);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = lead ? x[e] * co[e] - b[e] * si[e] : x[e] * co[e] + b[e] * si[e];
+            }
+        }
+    }
+    if (!mine) return;
+    if (is_q) Vec4<T>::store(q_out + ((size_t)t * heads + head) * kd + d, x);
+    else if (cell) Vec4<T>::store(cell + d, x);
+}
+
 extern "C" int hb_qkv_talking_prepare(void* q_out, void* kv, float* keep, const void* qkv, int dtype, const void* bias,
                                       int bias_dtype, const void* q_weight, const void* k_weight, int weight_dtype, float eps,
                                       const int32_t* positions, const float* table, int rot_dims, int table_rows,
@@ -120,6 +212,18 @@ extern "C" int hb_qkv_talking_prepare(void* q_out, void* kv, float* keep, const 
     const size_t smem = (size_t)TP_WARPS * key_dim * sizeof(float);
     cudaStream_t s = (cudaStream_t)stream;
     if (!rot_dims) table = nullptr;
+    const uintptr_t addresses = (uintptr_t)q_out | (uintptr_t)kv | (uintptr_t)keep | (uintptr_t)qkv | (uintptr_t)bias | (uintptr_t)q_weight |
+                                (uintptr_t)k_weight | (uintptr_t)table | (uintptr_t)first;
+    if (key_dim % 4 == 0 && value_dim % 4 == 0 && key_dim <= 128 && value_dim <= 128 && rot_dims % (interleaved ? 4 : 8) == 0 && addresses % 16 == 0 &&
+        (dtype == HB_F32 || dtype == HB_BF16)) {
+#define HB_QUADS(T) talking_prepare4_kernel<T><<<(unsigned)((items + 7) / 8), 256, 0, s>>>((T*)q_out, (T*)kv, keep, (const T*)qkv, bias, bias_dtype == HB_F32, \
+            q_weight, k_weight, weight_dtype == HB_F32, eps, positions, table, rot_dims, table_rows, interleaved, first, blend, write_index, pages, \
+            page_size, tokens, heads, kv_heads, key_dim, value_dim)
+        if (dtype == HB_F32) HB_QUADS(float); else HB_QUADS(bf16);
+#undef HB_QUADS
+        HB_LAUNCH_CHECK("qkv_talking_prepare");
+        return 0;
+    }
     if (dtype == HB_F32)
         talking_prepare_kernel<float><<<blocks, TP_WARPS * 32, smem, s>>>(
             (float*)q_out, (float*)kv, keep, (const float*)qkv, bias, bias_dtype == HB_F32, q_weight, k_weight,
@@ -590,6 +694,42 @@ extern "C" int hb_attention_talking(void* out, const void* q, const void* kv, in
     HB_REFUSE("attention_talking: dtype %d", dtype);
 }
 
+// The same in bfloat16 with groups of G query heads a kv head and 2 neighbouring values a thread, which makes a group's G outputs of
+// them at once: every value is read from shared memory once per kv head, as it is stored, in place of once per query head as two 32-bit numbers.
+template <int G>
+__global__ void __launch_bounds__(256) talking_mix2_kernel(bf16* __restrict__ out, const bf16* __restrict__ wide_in, int token0, int heads, int kv_heads,
+                                                           int vd, const float* __restrict__ talk) {
+    extern __shared__ float4 tk_quads[];
+    uint32_t* rows = (uint32_t*)tk_quads;                    // [heads][kv_heads * vd / 2] pairs
+    const size_t t = (size_t)token0 + blockIdx.x;
+    const int all = kv_heads * vd, pairs = all >> 1, n = heads * all;
+    float* mix = (float*)(rows + heads * pairs);             // [kv_heads][heads g][G]: talk[kv G + i][g]
+    const uint4* src = (const uint4*)(wide_in + t * n);
+    for (int e = threadIdx.x; e < (n >> 3); e += blockDim.x) ((uint4*)rows)[e] = __ldg(src + e);
+    for (int e = threadIdx.x; e < heads * heads; e += blockDim.x) {
+        const int h = e / heads, g = e - h * heads;
+        mix[((h / G) * heads + g) * G + h % G] = talk[e];
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+        const int c = 2 * p / vd;                            // the kv head whose values these are
+        const float* m = mix + c * heads * G;
+        float2 o[G];
+#pragma unroll
+        for (int i = 0; i < G; ++i) o[i] = make_float2(0.f, 0.f);
+#pragma unroll 4
+        for (int g = 0; g < heads; ++g) {
+            const uint32_t v = rows[g * pairs + p];
+            const float a = __uint_as_float(v << 16), b = __uint_as_float(v & 0xffff0000u);
+#pragma unroll
+            for (int i = 0; i < G; ++i) { o[i].x = fmaf(m[g * G + i], a, o[i].x); o[i].y = fmaf(m[g * G + i], b, o[i].y); }
+        }
+#pragma unroll
+        for (int i = 0; i < G; ++i)
+            *(__nv_bfloat162*)(out + (t * heads + c * G + i) * vd + 2 * p - c * vd) = __floats2bfloat162_rn(o[i].x, o[i].y);
+    }
+}
+
 // out [tokens, heads, value_dim] for tokens token0 .. token0 + count - 1 from wide [tokens, heads, value_heads, value_dim]
 // (value_heads: kv_heads, or 1 with one kv head).
 extern "C" int hb_talking_mix(void* out, const void* wide, int dtype, int token0, int count, int heads, int kv_heads,
@@ -599,6 +739,17 @@ extern "C" int hb_talking_mix(void* out, const void* wide, int dtype, int token0
     const size_t smem = ((size_t)heads * kv_heads * value_dim + (size_t)heads * heads) * sizeof(float);
     if (smem > 200 * 1024) HB_REFUSE("talking_mix: %zu bytes of shared memory a token", smem);
     cudaStream_t s = (cudaStream_t)stream;
+    const int group = heads / kv_heads;
+    if (dtype == HB_BF16 && talk && value_dim % 2 == 0 && heads * kv_heads * value_dim % 8 == 0 && ((uintptr_t)out | (uintptr_t)wide) % 16 == 0 &&
+        (group == 1 || group == 2 || group == 4 || group == 8)) {
+        const size_t bytes = (size_t)heads * kv_heads * value_dim * 2 + (size_t)heads * heads * sizeof(float);
+#define2(G) do { if (bytes > 46 * 1024) HB_CUDA(cudaFuncSetAttribute(talking_mix2_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); \
+        talking_mix2_kernel<G><<<count, 256, bytes, s>>>((bf16*)out, (const bf16*)wide, token0, heads, kv_heads, value_dim, talk); } while (0)
+        if (group == 1)2(1); else if (group == 2)2(2); else if (group == 4)2(4); else2(8);
+#undef2
+        HB_LAUNCH_CHECK("talking_mix");
+        return 0;
+    }
     if (dtype == HB_BF16) {
         if (smem > 46 * 1024) HB_CUDA(cudaFuncSetAttribute(talking_mix_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         talking_mix_kernel<bf16><<<count, 256, smem, s>>>((bf16*)out, (const bf16*)wide, token0, heads, kv_heads, value_dim, talk);

@@ -71,7 +71,7 @@ extern "C" int hb_mlstm_gates(float* out, const float* pre, int ld, const void* 
     if (rows == 0 || tokens == 0) return 0;
     if (heads < 1 || heads > 65535 || ld < 2 * heads) HB_REFUSE("mlstm_gates: %d heads in rows of %d", heads, ld);
     if (!(cap > 0.f)) HB_REFUSE("mlstm_gates: the gates' cap must be positive");
-    mlstm_gates_kernel<<<dim3(rows, heads), 128, 0, (cudaStream_t)stream>>>(out, pre, ld, bias, bias_dtype == HB_F32, cap, m_state,
+    mlstm_gates_kernel<<<dim3(rows, heads), tokens > 128 * rows ? 512 : 128, 0, (cudaStream_t)stream>>>(out, pre, ld, bias, bias_dtype == HB_F32, cap, m_state,
                                                                            query_start, row_slot, (long)tokens, heads);
     HB_LAUNCH_CHECK("mlstm_gates");
     return 0;
@@ -96,6 +96,33 @@ __global__ void mlstm_prepare_kernel(float* __restrict__ qk, float* __restrict__
     }
 }
 
+// The same, four neighbouring numbers a thread (dim and heads (vdim + 1) multiples of 4, rows and pointers on whole quads).
+template <typename T>
+__global__ void mlstm_prepare4_kernel(float* __restrict__ qk, float* __restrict__ v1, const float* __restrict__ take,
+                                      const T* __restrict__ first, int ld, int heads, int dim, int vdim, float q_scale) {
+    const size_t t = blockIdx.x;
+    const int e = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    const int nq = heads * dim, nv = heads * (vdim + 1);
+    const T* row = first + t * ld;
+    float x[4];
+    if (e < 2 * nq) {
+        const float f = e < nq ? q_scale : take[t * heads + (e - nq) / dim];
+        Vec4<T>::load(row + e, x);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] *= f;
+        Vec4<float>::store(qk + t * 2 * nq + e, x);
+    } else if (e < 2 * nq + nv) {
+        const int at = e - 2 * nq;
+        int h = at / (vdim + 1), d = at - h * (vdim + 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            x[i] = d < vdim ? to_f32(row[2 * nq + h * vdim + d]) : 1.f;
+            if (++d > vdim) { d = 0; ++h; }
+        }
+        Vec4<float>::store(v1 + t * nv + at, x);
+    }
+}
+
 extern "C" int hb_mlstm_prepare(float* qk, float* v1, const float* take, const void* first, int dtype, int ld, int tokens,
                                 int heads, int dim, int vdim, float q_scale, hb_stream stream) {
     if (tokens == 0) return 0;
@@ -104,6 +131,13 @@ extern "C" int hb_mlstm_prepare(float* qk, float* v1, const float* take, const v
     if (segments > 65535 || ld < 2 * heads * dim + heads * vdim) HB_REFUSE("mlstm_prepare: %ld numbers a token, rows of %d", per, ld);
     const dim3 grid(tokens, (unsigned)segments);
     cudaStream_t s = (cudaStream_t)stream;
+    if (dim % 4 == 0 && heads * (vdim + 1) % 4 == 0 && ld % 4 == 0 && ((uintptr_t)qk | (uintptr_t)v1 | (uintptr_t)first) % 16 == 0 && (dtype == HB_F32 || dtype == HB_BF16)) {
+        const dim3 grid4(tokens, (unsigned)((per / 4 + 255) / 256));
+        if (dtype == HB_F32) mlstm_prepare4_kernel<float><<<grid4, 256, 0, s>>>(qk, v1, take, (const float*)first, ld, heads, dim, vdim, q_scale);
+        else mlstm_prepare4_kernel<bf16><<<grid4, 256, 0, s>>>(qk, v1, take, (const bf16*)first, ld, heads, dim, vdim, q_scale);
+        HB_LAUNCH_CHECK("mlstm_prepare");
+        return 0;
+    }
     if (dtype == HB_F32) mlstm_prepare_kernel<float><<<grid, 256, 0, s>>>(qk, v1, take, (const float*)first, ld, heads, dim, vdim, q_scale);
     else if (dtype == HB_BF16) mlstm_prepare_kernel<bf16><<<grid, 256, 0, s>>>(qk, v1, take, (const bf16*)first, ld, heads, dim, vdim, q_scale);
     else HB_REFUSE("mlstm_prepare: dtype %d", dtype);
