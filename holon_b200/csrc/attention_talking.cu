@@ -743,10 +743,10 @@ extern "C" int hb_talking_mix(void* out, const void* wide, int dtype, int token0
     if (dtype == HB_BF16 && talk && value_dim % 2 == 0 && heads * kv_heads * value_dim % 8 == 0 && ((uintptr_t)out | (uintptr_t)wide) % 16 == 0 &&
         (group == 1 || group == 2 || group == 4 || group == 8)) {
         const size_t bytes = (size_t)heads * kv_heads * value_dim * 2 + (size_t)heads * heads * sizeof(float);
-#define2(G) do { if (bytes > 46 * 1024) HB_CUDA(cudaFuncSetAttribute(talking_mix2_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); \
+#define HB_MIX2(G) do { if (bytes > 46 * 1024) HB_CUDA(cudaFuncSetAttribute(talking_mix2_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)); \
         talking_mix2_kernel<G><<<count, 256, bytes, s>>>((bf16*)out, (const bf16*)wide, token0, heads, kv_heads, value_dim, talk); } while (0)
-        if (group == 1)2(1); else if (group == 2)2(2); else if (group == 4)2(4); else2(8);
-#undef2
+        if (group == 1) HB_MIX2(1); else if (group == 2) HB_MIX2(2); else if (group == 4) HB_MIX2(4); else HB_MIX2(8);
+#undef HB_MIX2
         HB_LAUNCH_CHECK("talking_mix");
         return 0;
     }
