@@ -230,14 +230,11 @@ int hb_expert_combine(void* out, const void* y, int dtype, const int32_t* place,
 // from the rows an expert gets on average).
 int hb_expert_linear_bf16(void* out, const void* x, const int32_t* token_of, const void* w, const int32_t* starts, int rows,
                           int experts, int n, int k, int act, int tile_rows, hb_stream stream);
-// The same for prompts on tcgen05 tensor cores (csrc/experts_tcgen05.cu: tiles of 128 rows x 256 columns, TMA, tensor
-// memory). token_of given: x is first gathered into `gathered` [rows, k]. table: 3 * hb_expert_linear_tcgen05_tiles(rows,
-// experts) int32 of scratch. hb_experts_tcgen05_status synchronises the device and returns (and clears) the kernel's
-// bounded-wait status word.
-int hb_expert_linear_tcgen05_tiles(int rows, int experts);
+// The same for prompts on tcgen05 tensor cores (csrc/experts_tcgen05.cu: pairs of CTAs, TMA, tensor memory; up to 1,024
+// experts). token_of given: x is first gathered into `gathered` [rows, k]. hb_experts_tcgen05_status synchronises the device and
+// returns (and clears) the kernel's bounded-wait status word.
 int hb_expert_linear_tcgen05(void* out, const void* x, const int32_t* token_of, void* gathered, const void* w,
-                             const int32_t* starts, int32_t* table, int rows, int experts, int n, int k, int act,
-                             hb_stream stream);
+                             const int32_t* starts, int rows, int experts, int n, int k, int act, hb_stream stream);
 // The clamped gated unit in the products' epilogues: out [rows, inter] = g sigmoid(alpha g) (u + 1) with g = min(f gate, limit),
 // u = clamp(f up, -limit, limit), f = row_scale[row] (null: 1), gate and up the row's products with an expert's first and last
 // inter rows of w [experts, 2 inter, k]; bfloat16. _few: on CUDA cores for a row or two an expert (k a multiple of 8);
@@ -245,8 +242,11 @@ int hb_expert_linear_tcgen05(void* out, const void* x, const int32_t* token_of, 
 int hb_expert_glu_few(void* out, const void* x, const int32_t* token_of, const void* w, const int32_t* starts,
                       const float* row_scale, float limit, float alpha, int rows, int experts, int inter, int k, hb_stream stream);
 int hb_expert_glu_tcgen05(void* out, const void* x, const int32_t* token_of, void* gathered, const void* w,
-                          const int32_t* starts, int32_t* table, const float* row_scale, float limit, float alpha, int rows,
-                          int experts, int inter, int k, hb_stream stream);
+                          const int32_t* starts, const float* row_scale, float limit, float alpha, int rows, int experts,
+                          int inter, int k, hb_stream stream);
+// out [rows, inter] = silu(gate) up in the product's epilogue; otherwise as hb_expert_glu_tcgen05.
+int hb_expert_swiglu_tcgen05(void* out, const void* x, const int32_t* token_of, void* gathered, const void* w, const int32_t* starts,
+                             int rows, int experts, int inter, int k, hb_stream stream);
 int hb_experts_tcgen05_status(unsigned int* status);
 // x = act(x) in place (act as above, 3 the tanh form of gelu, 4 xielu with the two numbers `numbers`, 5 tanh);
 // o [tokens, n] *= sigmoid(g[t * ld + i]).

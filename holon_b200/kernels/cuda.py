@@ -1156,6 +1156,7 @@ class CudaKernels:
                    self._i32(chosen, "chosen"), t, top, int(experts), self._p(None), self._p(None))
 
     EXPERT_TCGEN05_ROWS = 96                  # rows an expert on average from which its products run on tcgen05
+    EXPERT_TCGEN05_MOST = 1024                # experts that kernel takes
 
     def expert_linear(self, out, x, token_of, w, starts, act: int) -> None:
         self._check(out, x, token_of, w, starts)
@@ -1165,15 +1166,12 @@ class CudaKernels:
                 or (token_of is None and x.shape[0] != rows) or (token_of is not None and token_of.shape[0] != rows):
             raise KernelError("expert_linear: x [*, k], w [experts, n, k], out [rows, n], starts int32 [experts + 1]")
         aligned = k % 8 == 0 and n % 8 == 0 and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0
-        if x.dtype == torch.bfloat16 and aligned and (self.expert_products == "tcgen05" or (
+        if x.dtype == torch.bfloat16 and aligned and e <= self.EXPERT_TCGEN05_MOST and (self.expert_products == "tcgen05" or (
                 self.expert_products == "fast" and self.expert_tile_rows == 0 and rows >= self.EXPERT_TCGEN05_ROWS * e)):
             # prompts (a hundred rows an expert and more): the tcgen05 kernel, x gathered expert by expert first
-            tiles = -(-rows // 128) + min(e, rows)
-            table = torch.empty(3 * tiles, dtype=torch.int32, device=self.device)
             gathered = torch.empty((rows, k), dtype=x.dtype, device=self.device) if token_of is not None else None
             return self._call("hb_expert_linear_tcgen05", self._p(out), self._p(x), self._i32(token_of, "token_of"),
-                              self._p(gathered), self._p(w), self._i32(starts, "starts"), self._i32(table, "table"), rows, e, n, k,
-                              int(act))
+                              self._p(gathered), self._p(w), self._i32(starts, "starts"), rows, e, n, k, int(act))
         if x.dtype == torch.bfloat16 and aligned and self.expert_products in ("fast", "mma"):
             return self._call("hb_expert_linear_bf16", self._p(out), self._p(x), self._i32(token_of, "token_of"), self._p(w),
                               self._i32(starts, "starts"), rows, e, n, k, int(act), int(self.expert_tile_rows))
@@ -1252,19 +1250,36 @@ class CudaKernels:
         common = (self._p(out), self._p(x), self._i32(token_of, "token_of"))
         unit = (self._p(row_scale), ctypes.c_float(limit), ctypes.c_float(alpha), rows, e, inter, k)
         aligned = k % 8 == 0 and inter % 8 == 0 and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0
-        if x.dtype == torch.bfloat16 and aligned and (self.expert_products == "tcgen05" or (
+        if x.dtype == torch.bfloat16 and aligned and e <= self.EXPERT_TCGEN05_MOST and (self.expert_products == "tcgen05" or (
                 self.expert_products == "fast" and self.expert_tile_rows == 0 and rows >= self.EXPERT_TCGEN05_ROWS * e)):
-            tiles = -(-rows // 128) + min(e, rows)
-            table = torch.empty(3 * tiles, dtype=torch.int32, device=self.device)
             gathered = torch.empty((rows, k), dtype=x.dtype, device=self.device) if token_of is not None else None
             return self._call("hb_expert_glu_tcgen05", *common, self._p(gathered), self._p(w), self._i32(starts, "starts"),
-                              self._i32(table, "table"), *unit)
+                              *unit)
         if x.dtype == torch.bfloat16 and aligned and self.expert_products in ("fast", "mma") and self.expert_tile_rows in (0, 8) \
                 and (rows <= 8 * e or self.expert_tile_rows == 8) and k <= 12800:
             return self._call("hb_expert_glu_few", *common, self._p(w), self._i32(starts, "starts"), *unit)
         both = torch.empty(out.shape[0], w.shape[1], dtype=out.dtype, device=self.device)
         self.expert_linear(both, x, token_of, w, starts, 0)
         self.glu_clamped(out, both, None, limit, alpha, row_scale=row_scale)
+
+    def expert_swiglu(self, out, x, token_of, w, starts) -> None:
+        """out [rows, inter] = silu(gate) · up for rows laid out expert by expert, through w [experts, 2 inter, k] (an expert's gate rows,
+        then its up rows): in the product's epilogue where the product runs on tcgen05, else a kernel behind it."""
+        self._check(out, x, token_of, w, starts)
+        e, n2, k = w.shape
+        rows, inter = out.shape
+        if n2 != 2 * inter or x.shape[1] != k or not (out.dtype == x.dtype == w.dtype) or starts.shape[0] != e + 1 \
+                or (token_of is not None and token_of.shape[0] != rows) or (token_of is None and x.shape[0] != rows):
+            raise KernelError("expert_swiglu: x [*, k], w [experts, 2 inter, k], out [rows, inter], starts int32 [experts + 1]")
+        aligned = k % 8 == 0 and inter % 8 == 0 and (x.data_ptr() | w.data_ptr() | out.data_ptr()) % 16 == 0
+        if x.dtype == torch.bfloat16 and aligned and e <= self.EXPERT_TCGEN05_MOST and (self.expert_products == "tcgen05" or (
+                self.expert_products == "fast" and self.expert_tile_rows == 0 and rows >= self.EXPERT_TCGEN05_ROWS * e)):
+            gathered = torch.empty((rows, k), dtype=x.dtype, device=self.device) if token_of is not None else None
+            return self._call("hb_expert_swiglu_tcgen05", self._p(out), self._p(x), self._i32(token_of, "token_of"), self._p(gathered),
+                              self._p(w), self._i32(starts, "starts"), rows, e, inter, k)
+        both = torch.empty(rows, n2, dtype=out.dtype, device=self.device)
+        self.expert_linear(both, x, token_of, w, starts, 0)
+        self.silu_mul(out, both)
 
     def glu_clamped(self, out, gate_up, bias, limit, alpha, row_scale=None) -> None:
         """`row_scale` (float32 [tokens] or None): a factor on each row of gate_up, before the bias."""

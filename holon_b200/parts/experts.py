@@ -136,6 +136,8 @@ class Experts(Part):
         if self.clamped:
             k.expert_glu(act, x, token_of, self.up.tensor.view(e, 2 * self.inter, self.hidden), starts, self.limit, self.alpha,
                          row_weight)
+        elif self.gated and hasattr(k, "expert_swiglu"):
+            k.expert_swiglu(act, x, token_of, self.up.tensor.view(e, 2 * self.inter, self.hidden), starts)
         elif self.gated:
             both = ctx.empty(t * top, 2 * self.inter)
             k.expert_linear(both, x, token_of, self.up.tensor.view(e, 2 * self.inter, self.hidden), starts, 0)

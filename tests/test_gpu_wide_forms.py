@@ -78,3 +78,20 @@ def test_out_norm_add(K, dim, kept, y_dtype, cast_dtype):
     close(out[0][0], out[1][0], torch.float32, scale=4.0)
     close(out[0][1], out[1][1], torch.float32, scale=8.0)
     close(out[0][2], out[1][2], cast_dtype, scale=8.0)
+
+
+@pytest.mark.parametrize("rows,experts,inter,k", [(900, 5, 264, 136), (400, 3, 8, 64), (2000, 6, 512, 72)])
+@pytest.mark.parametrize("products", ["tcgen05", "mma"])
+def test_swiglu_of_experts(K, rows, experts, inter, k, products, monkeypatch):
+    monkeypatch.setattr(K, "expert_products", products)
+    g = torch.Generator().manual_seed(rows)
+    starts = torch.tensor([0, *torch.sort(torch.randint(0, rows + 1, (experts - 1,), generator=g)).values.tolist(), rows], dtype=torch.int32)
+    tokens = rows // 2
+    x, w = rand(tokens, k, dtype=BF16, seed=1), rand(experts, 2 * inter, k, dtype=BF16, seed=2, scale=k ** -0.5)
+    token_of = torch.randint(0, tokens, (rows,), generator=g).to(torch.int32)
+    out, both = torch.full((rows, inter), 7.0, dtype=BF16, device=DEV), torch.empty(rows, 2 * inter)
+    K.expert_swiglu(out, x.to(DEV), token_of.to(DEV), w.to(DEV), starts.to(DEV))
+    REF.expert_linear(both, x.float(), token_of, w.float(), starts, 0)
+    want = torch.nn.functional.silu(both[:, :inter]) * both[:, inter:]
+    assert K.tcgen05_status() == 0
+    close(out, want, BF16, scale=4.0)                            # (products of up to about 8, the library's form rounds twice)
