@@ -118,7 +118,7 @@ __global__ void qk_norm_rope_kv_write_kernel(T* __restrict__ q_out, const T* __r
     }
 }
 
-// The production shape, bfloat16 with head_dim = rotary_dim = 128: eight lanes share one (token, head), each holding
+// bfloat16 with head_dim 128, all of it turned (TURN) or none, with or without a bias: eight lanes share one (token, head), each holding
 // 8 values of the head's first half and the 8 it pairs with in the second half, so every access is 16 bytes wide,
 // the norm's sum takes three shuffles and nothing goes through shared memory.
 __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
@@ -145,12 +145,14 @@ template <> __device__ __forceinline__ void load_w8<float>(const float* w, float
     f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
-template <typename TW>
+// Without a turn, 2,048 tokens of 16 + 8 heads: 18.3 us in the general kernel, about 6 here.
+template <typename TW, bool TURN>
 __global__ void __launch_bounds__(256) qk_norm_rope_kv_write_d128_kernel(
         bf16* __restrict__ q_out, const bf16* __restrict__ qkv, const int32_t* __restrict__ positions,
         const float* __restrict__ table, int max_positions, const TW* __restrict__ q_weight,
         const TW* __restrict__ k_weight, float eps, float offset, bf16* __restrict__ kv,
-        const int32_t* __restrict__ write_index, int pages, int page_size, int tokens, int heads, int kv_heads) {
+        const int32_t* __restrict__ write_index, int pages, int page_size, int tokens, int heads, int kv_heads,
+        const bf16* __restrict__ bias) {
     constexpr int D = 128, HALF = 64;
     const int items = heads + (kv ? 2 * kv_heads : 0);
     const long unit = (long)blockIdx.x * 32 + (threadIdx.x >> 3);   // one (token, head) per eight lanes
@@ -180,27 +182,35 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_write_d128_kernel(
     }
     // Everything the rotation needs is asked for before the first result is used (the position first: the table row
     // hangs on it), so that a step of a few tokens pays two trips to memory instead of four.
-    int pos = live && rotate ? positions[t] : 0;
+    int pos = TURN && live && rotate ? positions[t] : 0;
     uint4 ra = make_uint4(0, 0, 0, 0), rb = ra;
     if (dst) { ra = *(const uint4*)(src + sub * 8); rb = *(const uint4*)(src + HALF + sub * 8); }
-    float wa[8], wb[8], c[8], sn[8];
+    float wa[8], wb[8], c[8], sn[8], a[8], b[8];
     if (dst && weight) {
         load_w8<TW>(weight + sub * 8, wa);
         load_w8<TW>(weight + HALF + sub * 8, wb);
     }
-    if (dst && rotate) {
+    if (TURN && dst && rotate) {
         pos = pos < 0 ? 0 : (pos >= max_positions ? max_positions - 1 : pos);
         const float* cs = table + (size_t)pos * D;
         load_w8<float>(cs + sub * 8, c);
         load_w8<float>(cs + HALF + sub * 8, sn);
     }
-    if (dst && !rotate) {                             // values: copied as they are
-        *(uint4*)(dst + sub * 8) = ra;
-        *(uint4*)(dst + HALF + sub * 8) = rb;
-    }
-    float a[8], b[8];
     unpack8(ra, a);
     unpack8(rb, b);
+    if (bias && dst) {
+        float add[8];
+        load_w8<bf16>(bias + item * D + sub * 8, add);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] += add[i];
+        load_w8<bf16>(bias + item * D + HALF + sub * 8, add);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b[i] += add[i];
+    }
+    if (dst && !rotate) {                             // values: copied as they are (to 32-bit and back is exact)
+        *(uint4*)(dst + sub * 8) = pack8(a);
+        *(uint4*)(dst + HALF + sub * 8) = pack8(b);
+    }
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) ss += a[i] * a[i] + b[i] * b[i];
@@ -219,8 +229,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_write_d128_kernel(
     float oa[8], ob[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        oa[i] = a[i] * c[i] - b[i] * sn[i];
-        ob[i] = b[i] * c[i] + a[i] * sn[i];
+        oa[i] = TURN ? a[i] * c[i] - b[i] * sn[i] : a[i];
+        ob[i] = TURN ? b[i] * c[i] + a[i] * sn[i] : b[i];
     }
     *(uint4*)(dst + sub * 8) = pack8(oa);
     *(uint4*)(dst + HALF + sub * 8) = pack8(ob);
@@ -233,12 +243,13 @@ static int launch(void* q_out, const void* qkv, const int32_t* positions, const 
                   int head_dim, const void* bias, cudaStream_t s) {
     const int items = heads + (kv ? 2 * kv_heads : 0);
     if constexpr (sizeof(T) == 2) {
-        const bool aligned = (((uintptr_t)q_out | (uintptr_t)qkv | (uintptr_t)table | (uintptr_t)qw | (uintptr_t)kw | (uintptr_t)kv) % 16) == 0;
-        if (head_dim == 128 && rotary_dim == 128 && aligned && !bias && (long)tokens * items < (1l << 31)) {
+        const bool aligned = (((uintptr_t)q_out | (uintptr_t)qkv | (uintptr_t)table | (uintptr_t)qw | (uintptr_t)kw | (uintptr_t)kv | (uintptr_t)bias) % 16) == 0;
+        if (head_dim == 128 && (rotary_dim == 128 || rotary_dim == 0) && aligned && (long)tokens * items < (1l << 31)) {
             const unsigned blocks = (unsigned)(((long)tokens * items + 31) / 32);
-            qk_norm_rope_kv_write_d128_kernel<TW><<<blocks, 256, 0, s>>>(
+            auto kernel = rotary_dim ? qk_norm_rope_kv_write_d128_kernel<TW, true> : qk_norm_rope_kv_write_d128_kernel<TW, false>;
+            kernel<<<blocks, 256, 0, s>>>(
                 (bf16*)q_out, (const bf16*)qkv, positions, table, max_positions, (const TW*)qw, (const TW*)kw, eps, offset,
-                (bf16*)kv, write_index, pages, page_size, tokens, heads, kv_heads);
+                (bf16*)kv, write_index, pages, page_size, tokens, heads, kv_heads, (const bf16*)bias);
             HB_LAUNCH_CHECK("qk_norm_rope_kv_write");
             return 0;
         }
