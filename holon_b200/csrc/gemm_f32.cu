@@ -1,266 +1,320 @@
-// out[m, n] = sum_k x[m, k] * w[n, k] in true 32-bit on CUDA cores: no tensor cores, no reduced-precision mode.
-// One order of summation for every output element, a function of k alone: k is cut into up to eight segments of equal
-// length (a multiple of 16, at least 64), each summed in ascending order with fused multiply-adds, and the segments' sums are added in
-// ascending order. So a row's result does not depend on how many other rows the batch holds, nor on which of the kernels
-// and splits below computed it (and eight shorter sums lose less than one long one).
+// out[m, n] = sum_k x[m, k] * w[n, k] in 32-bit on tcgen05 tensor cores: every operand is split exactly into three bfloat16 numbers.
+//
+// x = x1 + x2 + x3, each the nearest bfloat16 to what the ones before leave (8 + 8 + 8 bits: nothing is left), so
+// x w = x1 w1 + (x1 w2 + x2 w1) + (x1 w3 + x2 w2 + x3 w1) up to 2^-26 of |x w|. The six products of 64 columns of k are
+// accumulated by tensor cores in 32 bits, the smallest first, and that sum is added to the running one in a register with one
+// rounding: tensor cores cut sums off instead of rounding them, which 64 columns keep below a rounding error of the running sum.
+// Relative error against 64 bits (2-norm), with multiply-adds in up to eight segments before and now: 541 rows, 1,024 of k 2.1e-7 and 0.95e-7;
+// 300 rows, 3,072 of k 3.6e-7 and 1.0e-7; operands that are all positive 0.8 to 1.1e-7 and 0.9 to 0.95e-7.
+// One order of summation for every output element, a function of k alone: k is cut into up to eight segments of equal length (a multiple
+// of 64), each summed in ascending order in steps of 64, and the segments' sums are added pairwise: ((s0 + s1) + (s2 + s3)) + ((s4 + s5) +
+// (s6 + s7)). So a row's result does not depend on how many other rows the batch holds, nor on how the work was split.
+// A result that is no finite number (an infinity or a NaN among the operands, whose split is none, or an overflow) is
+// computed again with multiply-adds on the numbers as they are.
+//
+// A block takes 128 rows of w (the M side of tcgen05.mma) by up to 96 rows of x. Eight warps read 64 columns of k of both, split them and
+// write the planes to shared memory (two stages, 128-byte swizzle); two threads issue the 24 MMAs of a stage each (an MMA takes its thread some 150 cycles whatever its size); eight warps
+// (four in the form for up to 16 rows) read the sums from tensor memory (two buffers) and add them up in registers. A segment's sum waits in tensor memory
+// for its partner. Where tiles are few, the blocks of a cluster of SPLIT share a tile's segments and add them through
+// distributed shared memory. Many rows are bound by shared memory: 24 MMAs read 168 KB and the planes are written with 84 KB, 2,000 cycles for
+// 128 x 96 x 64; few rows by reading w once.
+// In us, with multiply-adds before and now (1,024 of k if not said): 541 rows, 4,096 columns 113 and 57, 6,144 161 and 76, 1,024 by 3,072 140 and
+// 43; 130 rows, 4,096 columns 54 and 19; 17 rows, 6,144 37 and 17; 8 rows 21 and 14; but 2 rows, 6,144 columns 10.4 and 14.2, 1,024 by 3,072 7.9 and 12.8:
+// up to four rows pay for a form whose sums do not depend on the rows beside them with an MMA's least time, some 100 cycles, 24 times a step.
 #include <cooperative_groups.h>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace cg = cooperative_groups;
 
-#define BM 64
-#define BN 128
-#define BK 16
-#define SEGMENTS 8
-#define SHORTEST 64                         // terms a segment holds at least: one piece of the kernel for few rows (shorter sums gain nothing)
+#define GF_BM 128                                 // rows of w a tile
+#define GF_BK 64                                  // columns of k a step
+#define GF_SEGMENTS 8
+#define GF_LOADERS 8                              // warps that load and split
+#define GF_PLANE (GF_BM * GF_BK * 2)              // bytes of a plane of w
 
 static __host__ __device__ inline int segment_length(int k) {
-    const int share = ((k + SEGMENTS - 1) / SEGMENTS + BK - 1) / BK * BK;
-    return share > SHORTEST ? share : SHORTEST;
+    return ((k + GF_SEGMENTS - 1) / GF_SEGMENTS + GF_BK - 1) / GF_BK * GF_BK;
 }
 
-// Two 32-bit multiply-adds in one instruction; each rounds as fmaf does.
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+__device__ __forceinline__ void gf_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+    tc_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ uint64_t twice(float x) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float2 halves(uint64_t v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
+__device__ __forceinline__ void gf_st16(uint32_t taddr, const float (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+                 ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+                   "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
+                 : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
 }
 
-// ---------------------------------------------------------------- many rows
-// Bound by the multiply-adds. 64 x 128 outputs a block of 128 threads, 8 x 8 a thread as packed pairs: 32 packed
-// multiply-adds for 4 wide loads from shared memory a step of k (4 x 4 a thread needed 2 for 16 and was bound by them); the
-// next 16 columns of k are fetched into registers while these are multiplied. A segment's sum goes to shared memory, so
-// that the registers hold one set of sums. Where there are too few tiles for the chip, the blocks of a cluster of SPLIT
-// share a tile's segments and add them through distributed shared memory.
-// Measured with a 28-layer model of width 1,024 in one pass over 541 rows: its 112 products of 4,096 and 6,144 columns by
-// 1,024 take 139 us on average (41 TFLOP/s), those of 1,024 columns by 2,048 and 3,072 109 us. With 64 x 64 tiles and 4 x 4
-// outputs a thread this pass and four steps of two rows took 78.7 ms in products, now 18.5. What bounds it: three wavefronts of the
-// shared-memory pipe a wide load, 12 for a step of k that multiplies for 16 cycles.
-template <bool VEC, int SPLIT>
-__global__ void __launch_bounds__(128) gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x,
-                                                       const float* __restrict__ w, int m, int n, int k, long ldx,
-                                                       long ldo, long x_batch, long o_batch) {
-    extern __shared__ float4 smem4[];
-    float (*xs)[BK][BM + 4] = reinterpret_cast<float (*)[BK][BM + 4]>(smem4);
-    float (*ws)[BK][BN + 4] = reinterpret_cast<float (*)[BK][BN + 4]>((float*)smem4 + 2 * BK * (BM + 4));
-    float* sums = (float*)smem4 + 2 * BK * (BM + BN + 8);               // [SEGMENTS / SPLIT or 1][BM][BN]
-    x += (size_t)blockIdx.z * x_batch;                                  // blockIdx.z: which of several products (w [batch, n, k])
+// Two numbers into three bfloat16 pairs.
+__device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    p1 = *(const uint32_t*)&h;
+    a -= __uint_as_float(p1 << 16);
+    b -= __uint_as_float(p1 & 0xffff0000u);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a, b);
+    p2 = *(const uint32_t*)&l;
+    a -= __uint_as_float(p2 << 16);
+    b -= __uint_as_float(p2 & 0xffff0000u);
+    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    p3 = *(const uint32_t*)&t;
+}
+
+// An element whose split gave no finite number, on the operands themselves.
+__device__ __noinline__ float gf_plain(const float* __restrict__ x, const float* __restrict__ w, int k) {
+    const int length = segment_length(k);
+    float s[GF_SEGMENTS];
+#pragma unroll
+    for (int q = 0; q < GF_SEGMENTS; ++q) {
+        s[q] = 0.f;
+        for (int i = q * length; i < min(k, (q + 1) * length); ++i) s[q] = fmaf(x[i], w[i], s[q]);
+    }
+    return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+
+// ROWS: the most rows of x a tile. rows_x: this launch's (a multiple of 16). ADDERS: warps that add up, four a half of the columns.
+template <int ROWS, int ADDERS, int SPLIT, bool VEC>
+__global__ void __launch_bounds__(32 * (GF_LOADERS + ADDERS + 2), ROWS <= 16 ? 2 : 1)
+gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, int m, int n, int k, long ldx, long ldo,
+                long x_batch, long o_batch, int rows_x) {
+    constexpr int SHARE = GF_SEGMENTS / SPLIT, GROUPS = (ROWS / 16 + ADDERS / 4 - 1) / (ADDERS / 4);   // column groups of 16 a warp adds up
+    constexpr int LEVELS = SHARE == 8 ? 3 : SHARE == 4 ? 2 : SHARE == 2 ? 1 : 0;                       // sums that wait for their partners
+    constexpr uint32_t COLS = ROWS * (2 + LEVELS) <= 32 ? 32 : ROWS * (2 + LEVELS) <= 64 ? 64 : ROWS * (2 + LEVELS) <= 128 ? 128
+                            : ROWS * (2 + LEVELS) <= 256 ? 256 : 512;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
+    float* sums = (float*)(smem_raw + (base - smem_addr(smem_raw)));         // SPLIT > 1, at the end: [rows_x][128] over the stages
+    const uint32_t plane_x = rows_x * GF_BK * 2, stage_bytes = 3 * (GF_PLANE + plane_x);
+    __shared__ __align__(8) uint64_t bars[8];
+    __shared__ uint32_t s_tmem;
+    const uint32_t full0 = smem_addr(bars), empty0 = full0 + 16, d_full0 = empty0 + 16, d_empty0 = d_full0 + 16;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    x += (size_t)blockIdx.z * x_batch;                                       // blockIdx.z: which of several products (w [batch, n, k])
     out += (size_t)blockIdx.z * o_batch;
     w += (size_t)blockIdx.z * n * k;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * BM, n0 = (blockIdx.x / SPLIT) * BN, rank = blockIdx.x % SPLIT;
-    const int length = segment_length(k), segments = (k + length - 1) / length;
-    constexpr int SHARE = SEGMENTS / SPLIT;
-    const int s_first = rank * SHARE, s_last = min(segments, s_first + SHARE);
-    const int k_first = s_first * length, k_end = min(k, s_last * length);
-    const int steps = k_end > k_first ? (k_end - k_first + BK - 1) / BK : 0, per_segment = length / BK;
+    const int n0 = ((int)blockIdx.x / SPLIT) * GF_BM, rank = (int)blockIdx.x % SPLIT, m0 = (int)blockIdx.y * rows_x;
+    const int length = segment_length(k), k_first = rank * SHARE * length, k_end = min(k, k_first + SHARE * length);
+    const int chunks = k_end > k_first ? (k_end - k_first + GF_BK - 1) / GF_BK : 0, per_segment = length / GF_BK;
 
-    // What this thread loads: 4 neighbouring k (4 lanes a row, so that a warp's load touches 8 lines and not 32: with a row a lane these
-    // loads took as much of the L1's bandwidth as all reads of shared memory) of 2 rows of x and 4 of w, 32 rows apart.
-    const int lr = tid >> 2, lk = (tid & 3) * 4;
-    float xv[2][4], wv[4][4];
-    auto fetch4 = [&](float (&v)[4], const float* p, bool there, int kk) {
-        if (VEC) {
-            const float4 f = there && kk < k ? *(const float4*)(p + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
-            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = there && kk + j < k ? p[kk + j] : 0.f;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(full0 + 8 * s, GF_LOADERS); mbar_init(empty0 + 8 * s, 1);
+            mbar_init(d_full0 + 8 * s, 1); mbar_init(d_empty0 + 8 * s, ADDERS);
         }
-    };
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) { const int r = m0 + lr + 32 * i; fetch4(xv[i], x + (size_t)(r < m ? r : 0) * ldx, r < m, k0 + lk); }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { const int r = n0 + lr + 32 * i; fetch4(wv[i], w + (size_t)(r < n ? r : 0) * k, r < n, k0 + lk); }
-    };
-    auto stage = [&](int buf) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) xs[buf][lk + j][lr + 32 * i] = xv[i][j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) ws[buf][lk + j][lr + 32 * i] = wv[i][j];
-        }
-    };
-    const int row = (warp & 1) * 32 + (lane >> 3) * 8, col = (warp >> 1) * 64 + (lane & 7) * 4;   // 8 rows; 4 columns here, 4 at + 32
-    uint64_t acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0;
-
-    if (steps) { fetch(k_first); stage(0); }
-    __syncthreads();
-    int in_segment = 0, slot = 0;
-    for (int step = 0; step < steps; ++step) {
-        const int buf = step & 1;
-        if (step + 1 < steps) fetch(k_first + (step + 1) * BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            const float4 a0 = *(const float4*)&xs[buf][kk][row], a1 = *(const float4*)&xs[buf][kk][row + 4];
-            const ulonglong2 b0 = *(const ulonglong2*)&ws[buf][kk][col], b1 = *(const ulonglong2*)&ws[buf][kk][col + 32];
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint64_t aa = twice(a[i]);
-                fma2(acc[i][0], aa, b0.x);
-                fma2(acc[i][1], aa, b0.y);
-                fma2(acc[i][2], aa, b1.x);
-                fma2(acc[i][3], aa, b1.y);
-            }
-        }
-        if (++in_segment == per_segment || step + 1 == steps) {          // the segment's end: its sum to shared memory
-            float* at = sums + (SPLIT > 1 ? (size_t)slot * BM * BN : 0);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float4* p = (float4*)&at[(row + i) * BN + col + 32 * h];
-                    const float2 u = halves(acc[i][2 * h]), v = halves(acc[i][2 * h + 1]);
-                    float4 s = make_float4(u.x, u.y, v.x, v.y);
-                    if (SPLIT == 1 && slot > 0) { const float4 t = *p; s = make_float4(t.x + s.x, t.y + s.y, t.z + s.z, t.w + s.w); }
-                    *p = s;
-                    acc[i][2 * h] = acc[i][2 * h + 1] = 0;
-                }
-            in_segment = 0;
-            ++slot;
-        }
-        if (step + 1 < steps) stage(buf ^ 1);
-        __syncthreads();
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    cg::cluster_group cluster = cg::this_cluster();
-    if (SPLIT > 1) cluster.sync();
-    constexpr int ROWS = BM / SPLIT;                                     // the tile's rows that this block adds up and writes
-    const bool wide = (n % 4 == 0) && (ldo % 4 == 0) && (o_batch % 4 == 0) && ((uintptr_t)out % 16 == 0);
-    for (int i = tid; i < ROWS * (BN / 4); i += 128) {
-        const int r = rank * ROWS + i / (BN / 4), c = i % (BN / 4) * 4;
-        if (m0 + r >= m || n0 + c >= n) continue;
-        float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (SPLIT == 1) total = *(const float4*)&sums[r * BN + c];
-        else {
-            for (int s = 0; s < segments; ++s) {
-                const float4 v = *(const float4*)(cluster.map_shared_rank(sums, s / SHARE) + (size_t)(s % SHARE) * BM * BN + r * BN + c);
-                total = s ? make_float4(total.x + v.x, total.y + v.y, total.z + v.z, total.w + v.w) : v;
+    if (warp == GF_LOADERS + ADDERS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "r"(COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    float acc[GROUPS][16];                                                   // (the adders' only)
+
+    if (warp >= ADDERS && warp < ADDERS + GF_LOADERS) {
+        // 16 lanes a row of 64 columns, two rows a warp and load, 16 rows a pass of the eight warps
+        constexpr int WP = GF_BM / 16, XP = ROWS / 16;
+        const int row = (warp - ADDERS) * 2 + (lane >> 4), kk = (lane & 15) * 4;
+        float4 v[WP + XP];
+        auto fetch = [&](int i, int chunk) {
+            const int at = k_first + chunk * GF_BK + kk, r = (i < WP ? n0 : m0) + row + 16 * (i < WP ? i : i - WP);
+            const bool there = r < (i < WP ? n : m) && (i < WP || (i - WP) * 16 < rows_x);
+            const float* p = (i < WP ? w + (size_t)r * k : x + (size_t)r * ldx) + at;
+            if (VEC) return there && at < k_end ? __ldg((const float4*)p) : make_float4(0.f, 0.f, 0.f, 0.f);   // (k and k_end are multiples of 4)
+            return make_float4(there && at < k_end ? p[0] : 0.f, there && at + 1 < k_end ? p[1] : 0.f, there && at + 2 < k_end ? p[2] : 0.f,
+                               there && at + 3 < k_end ? p[3] : 0.f);
+        };
+        if (chunks) {
+#pragma unroll
+            for (int i = 0; i < WP + XP; ++i) v[i] = fetch(i, 0);
+        }
+        bool ok = true;
+        for (int c = 0; c < chunks && ok; ++c) {
+            const int s = c & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ((c >> 1) & 1) ^ 1, 1));
+            if (!ok) break;
+            const uint32_t stage = base + s * stage_bytes;
+            const uint32_t within = (uint32_t)((((lane & 15) >> 1) ^ (row & 7)) * 16 + (lane & 1) * 8);   // (row & 7 is the same in every pass)
+#pragma unroll
+            for (int i = 0; i < WP + XP; ++i) {
+                if (i >= WP && (i - WP) * 16 >= rows_x) continue;
+                uint32_t p[3][2];
+                split2(v[i].x, v[i].y, p[0][0], p[1][0], p[2][0]);
+                split2(v[i].z, v[i].w, p[0][1], p[1][1], p[2][1]);
+                const uint32_t at = (i < WP ? stage : stage + 3 * GF_PLANE) + (row + 16 * (i < WP ? i : i - WP)) * 128 + within;
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(at + q * (i < WP ? GF_PLANE : plane_x)), "r"(p[q][0]), "r"(p[q][1]) : "memory");
+                if (c + 1 < chunks) v[i] = fetch(i, c + 1);                  // the next step's numbers are on their way while the rest is split
+            }
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full0 + 8 * s);
+        }
+    } else if (warp >= GF_LOADERS + ADDERS) {                                // a stage and buffer each
+        if (lane == 0) {
+            // kind::f16: D float32 (bit 4), A and B bfloat16 (bits 7, 10), both K-major, N / 8 at bit 17, M / 16 at bit 24
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(rows_x >> 3) << 17) | ((uint32_t)(GF_BM >> 4) << 24);
+            bool ok = true;
+            for (int c = warp - GF_LOADERS - ADDERS; c < chunks && ok; c += 2) {
+                const int s = c & 1;
+                ok = mbar_wait(d_empty0 + 8 * s, ((c >> 1) & 1) ^ 1, 4);     // the buffer's last sum has been read
+                ok = ok && mbar_wait(full0 + 8 * s, (c >> 1) & 1, 2);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t stage = base + s * stage_bytes, d = tmem + s * ROWS;
+                uint64_t a[3], b[3];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) { a[q] = tc_smem_desc(stage + q * GF_PLANE); b[q] = tc_smem_desc(stage + 3 * GF_PLANE + q * plane_x); }
+#pragma unroll
+                for (int q = 0; q < 6; ++q) {                                // w1 x3, w2 x2, w3 x1, w1 x2, w2 x1, w1 x1
+                    const int i = q < 3 ? q : q - 3 < 2 ? q - 3 : 0, j = q < 3 ? 2 - q : q < 5 ? 4 - q : 0;
+#pragma unroll
+                    for (int kk = 0; kk < GF_BK / 16; ++kk) tc_mma(d, a[i] + kk * 2, b[j] + kk * 2, idesc, (q | kk) != 0);
+                }
+                tc_commit(empty0 + 8 * s);
+                tc_commit(d_full0 + 8 * s);
             }
         }
-        float* o = out + (size_t)(m0 + r) * ldo + n0 + c;
-        if (wide) *(float4*)o = total;
-        else {
-            const float v[4] = {total.x, total.y, total.z, total.w};
+    } else {
+        const int half = warp >> 2;                                          // column groups half, half + ADDERS / 4, ...
+        const uint32_t lane_t = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        bool ok = true;
+        int c = 0;
+        for (int q = 0; q < SHARE && ok; ++q) {                              // the segments of this block
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[g][i] = 0.f;
+            for (const int until = min(chunks, c + per_segment); c < until; ++c) {
+                const int s = c & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(d_full0 + 8 * s, (c >> 1) & 1, 3));
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int g = 0; g < GROUPS; ++g) {
+                    const int col = (half + g * (ADDERS / 4)) * 16;
+                    if (col < rows_x) {
+                        float v[16];
+                        gf_ld16(lane_t + s * ROWS + col, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) acc[g][i] += v[i];
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(d_empty0 + 8 * s);
+            }
+            if constexpr (LEVELS > 0) {                                      // with its partners, or to wait for them
+#pragma unroll
+                for (int g = 0; g < GROUPS; ++g) {
+                    const int col = (half + g * (ADDERS / 4)) * 16;
+                    if (col < rows_x) {
+                        int level = 0;
+                        for (; (q >> level) & 1; ++level) {
+                            float v[16];
+                            gf_ld16(lane_t + (2 + level) * ROWS + col, v);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) acc[g][i] = v[i] + acc[g][i];
+                        }
+                        if (q < SHARE - 1) gf_st16(lane_t + (2 + level) * ROWS + col, acc[g]);
+                    }
+                }
+            }
+        }
+        const int row = (warp & 3) * 32 + lane;
+        if constexpr (SPLIT == 1) {
+            bool bad = false;
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g) {
+                const int col = (half + g * (ADDERS / 4)) * 16;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int r = m0 + col + i;
+                    if (col >= rows_x || r >= m || n0 + row >= n) continue;
+                    out[(size_t)r * ldo + n0 + row] = acc[g][i];
+                    bad |= !(fabsf(acc[g][i]) <= 3.402823466e38f);
+                }
+            }
+            if (bad)
+                for (int col = half * 16; col < rows_x; col += ADDERS * 4)
+                    for (int r = m0 + col; r < min(m, m0 + col + 16); ++r) {
+                        float* o = out + (size_t)r * ldo + n0 + row;
+                        if (!(fabsf(*o) <= 3.402823466e38f)) *o = gf_plain(x + (size_t)r * ldx, w + (size_t)(n0 + row) * k, k);
+                    }
+        }
+    }
+    if constexpr (SPLIT > 1) {
+        __syncthreads();                                                     // every stage has been read: the sums go over them
+        if (warp < ADDERS) {
+            const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g) {
+                const int col = (half + g * (ADDERS / 4)) * 16;
+                if (col < rows_x)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sums[(col + i) * GF_BM + row] = acc[g][i];
+            }
+        }
+        cg::cluster_group cluster = cg::this_cluster();
+        __syncwarp();
+        cluster.sync();
+        const int quads = rows_x * (GF_BM / 4);                              // this block's share, four columns of the output a thread
+        const bool wide = n % 4 == 0 && ldo % 4 == 0 && o_batch % 4 == 0 && (uintptr_t)out % 16 == 0;
+        for (int i = rank * (quads / SPLIT) + threadIdx.x; i < (rank + 1) * (quads / SPLIT); i += blockDim.x) {
+            const int col = i / (GF_BM / 4), row = i % (GF_BM / 4) * 4, r = m0 + col;
+            if (r >= m || n0 + row >= n) continue;
+            float4 p[SPLIT];
+#pragma unroll
+            for (int s = 0; s < SPLIT; ++s) p[s] = *(const float4*)(cluster.map_shared_rank(sums, s) + col * GF_BM + row);
+#pragma unroll
+            for (int d = 1; d < SPLIT; d *= 2)
+#pragma unroll
+                for (int s = 0; s < SPLIT; s += 2 * d)
+                    p[s] = make_float4(p[s].x + p[s + d].x, p[s].y + p[s + d].y, p[s].z + p[s + d].z, p[s].w + p[s + d].w);
+            float v[4] = {p[0].x, p[0].y, p[0].z, p[0].w};
+#pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (n0 + c + j < n) o[j] = v[j];
+                if (!(fabsf(v[j]) <= 3.402823466e38f) && n0 + row + j < n) v[j] = gf_plain(x + (size_t)r * ldx, w + (size_t)(n0 + row + j) * k, k);
+            float* o = out + (size_t)r * ldo + n0 + row;
+            if (wide) *(float4*)o = make_float4(v[0], v[1], v[2], v[3]);
+            else
+                for (int j = 0; j < 4; ++j)
+                    if (n0 + row + j < n) o[j] = v[j];
         }
+        __syncwarp();
+        cluster.sync();                                                      // nobody leaves while its sums are being read
     }
-    if (SPLIT > 1) cluster.sync();                                       // nobody leaves while its sums are being read
-}
-
-// ---------------------------------------------------------------- few rows
-// Bound by reading w once. A block of 256 threads takes 8 columns and all of k: a thread sums one segment of one column
-// for a quarter of the rows, over pieces of 64 of each segment that a ring of stages brings by cp.async: three where many
-// blocks share an SM, six where there are few blocks (the first five, all of k up to 2,560, are then on their way at once). Two rows, the same
-// model's step: 7.2 us for a product of 1,024 columns (10 with three stages), 13.2 on average for the wider ones, the head of 151,936
-// columns among them (167 us, 3.7 TB/s); as tiles of 64 rows each was a serial walk over k.
-#define FEW_COLS 8
-#define FEW_PIECE 64
-#define FEW_STRIDE (FEW_PIECE + 4)          // neighbouring (segment, column) rows then lie four banks apart
-#define FEW_ROWS 16
-
-__device__ __forceinline__ void copy16(float* dst, const float* src, bool there) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(there ? 16 : 0) : "memory");
-}
-
-template <int RT, int FEW_STAGES>           // rows a thread: 4 RT >= m
-__global__ void __launch_bounds__(256) gemm_f32_few_kernel(float* __restrict__ out, const float* __restrict__ x,
-                                                           const float* __restrict__ w, int m, int n, int k, long ldx,
-                                                           long ldo, long x_batch, long o_batch) {
-    extern __shared__ float4 smem4[];
-    x += (size_t)blockIdx.z * x_batch;
-    out += (size_t)blockIdx.z * o_batch;
-    w += (size_t)blockIdx.z * n * k;
-    const int tid = threadIdx.x, n0 = blockIdx.x * FEW_COLS;
-    const int length = segment_length(k), segments = (k + length - 1) / length, pieces = (length + FEW_PIECE - 1) / FEW_PIECE;
-    const int stage_floats = SEGMENTS * (FEW_COLS + m) * FEW_STRIDE;
-    float* base = (float*)smem4;
-    auto load = [&](int piece) {
-        float* at = base + (size_t)(piece % FEW_STAGES) * stage_floats;
-        const int total = SEGMENTS * (FEW_COLS + m) * (FEW_PIECE / 4);
-        for (int i = tid; i < total; i += 256) {
-            const int q = i % (FEW_PIECE / 4) * 4, line = i / (FEW_PIECE / 4);      // lines: [segment][column], then [segment][row]
-            const bool of_w = line < SEGMENTS * FEW_COLS;
-            const int l2 = line - SEGMENTS * FEW_COLS;
-            const int s = of_w ? line / FEW_COLS : l2 / m, c = of_w ? n0 + line % FEW_COLS : l2 % m;
-            const int in = piece * FEW_PIECE + q, kk = s * length + in;
-            const bool there = in < length && kk < k && (!of_w || c < n);
-            const float* src = of_w ? w + (size_t)c * k + kk : x + (size_t)c * ldx + kk;
-            copy16(at + line * FEW_STRIDE + q, there ? src : x, there);
-        }
-    };
-    const int column = tid & 7, s = (tid >> 3) & 7, group = tid >> 6;
-    float acc[RT];
-#pragma unroll
-    for (int r = 0; r < RT; ++r) acc[r] = 0.f;
-#pragma unroll
-    for (int p = 0; p < FEW_STAGES - 1; ++p) {
-        if (p < pieces) load(p);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    const bool busy = group * RT < m && s < segments;
-    for (int p = 0; p < pieces; ++p) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(FEW_STAGES - 2) : "memory");
-        __syncthreads();
-        if (p + FEW_STAGES - 1 < pieces) load(p + FEW_STAGES - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (busy) {
-            const float* at = base + (size_t)(p % FEW_STAGES) * stage_floats;
-            const float* wl = at + (s * FEW_COLS + column) * FEW_STRIDE;
-            const float* xl = at + (SEGMENTS * FEW_COLS + s * m) * FEW_STRIDE;
-#pragma unroll 4
-            for (int q = 0; q < FEW_PIECE; q += 4) {
-                const float4 b = *(const float4*)(wl + q);
-#pragma unroll
-                for (int r = 0; r < RT; ++r) {
-                    const float4 a = *(const float4*)(xl + min(group * RT + r, m - 1) * FEW_STRIDE + q);
-                    acc[r] = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc[r]))));
-                }
-            }
-        }
-    }
+    tc_fence_before();
     __syncthreads();
-    float* sums = base;                                                  // [row][segment][column], on the first stage
-#pragma unroll
-    for (int r = 0; r < RT; ++r)
-        if (busy && group * RT + r < m) sums[((group * RT + r) * SEGMENTS + s) * FEW_COLS + column] = acc[r];
-    __syncthreads();
-    for (int i = tid; i < m * FEW_COLS; i += 256) {
-        const int r = i / FEW_COLS, c = i % FEW_COLS;
-        if (n0 + c >= n) continue;
-        float total = sums[r * SEGMENTS * FEW_COLS + c];
-        for (int t = 1; t < segments; ++t) total += sums[(r * SEGMENTS + t) * FEW_COLS + c];
-        out[(size_t)r * ldo + n0 + c] = total;
+    if (warp == GF_LOADERS + ADDERS) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(COLS) : "memory");
     }
 }
 
 // ---------------------------------------------------------------- the choice
-template <bool VEC, int SPLIT>
-static int launch_tiles(float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx, long ldo,
-                        long x_batch, long o_batch, cudaStream_t s) {
-    const int smem = (2 * BK * (BM + BN + 8) + (SPLIT > 1 ? SEGMENTS / SPLIT : 1) * BM * BN) * (int)sizeof(float);
-    auto kernel = gemm_f32_kernel<VEC, SPLIT>;
-    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+struct GfArgs { float* out; const float* x; const float* w; int m, n, k, batch; long ldx, ldo, x_batch, o_batch; int rows_x; };
+
+template <int ROWS, int ADDERS, int SPLIT, bool VEC>
+static int launch_split(const GfArgs& a, cudaStream_t s) {
+    const int smem = 2 * 3 * (GF_PLANE + a.rows_x * GF_BK * 2) + 1024;
+    auto kernel = gemm_f32_kernel<ROWS, ADDERS, SPLIT, VEC>;
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 3 * (GF_PLANE + ROWS * GF_BK * 2) + 1024));
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3((n + BN - 1) / BN * SPLIT, (m + BM - 1) / BM, batch);
-    config.blockDim = dim3(128);
+    config.gridDim = dim3((a.n + GF_BM - 1) / GF_BM * SPLIT, (a.m + a.rows_x - 1) / a.rows_x, a.batch);
+    config.blockDim = dim3(32 * (GF_LOADERS + ADDERS + 2));
     config.dynamicSmemBytes = smem;
     config.stream = s;
     cudaLaunchAttribute attr[1];
@@ -269,55 +323,56 @@ static int launch_tiles(float* out, const float* x, const float* w, int m, int n
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     config.attrs = attr;
     config.numAttrs = SPLIT > 1 ? 1 : 0;
-    HB_CUDA(cudaLaunchKernelEx(&config, kernel, out, x, w, m, n, k, ldx, ldo, x_batch, o_batch));
+    HB_CUDA(cudaLaunchKernelEx(&config, kernel, a.out, a.x, a.w, a.m, a.n, a.k, a.ldx, a.ldo, a.x_batch, a.o_batch, a.rows_x));
     return 0;
 }
 
-template <int RT, int FEW_STAGES>
-static int launch_few_stages(float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx, long ldo,
-                      long x_batch, long o_batch, cudaStream_t s) {
-    const int smem = FEW_STAGES * SEGMENTS * (FEW_COLS + m) * FEW_STRIDE * (int)sizeof(float);
-    auto kernel = gemm_f32_few_kernel<RT, FEW_STAGES>;
-    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 FEW_STAGES * SEGMENTS * (FEW_COLS + min(FEW_ROWS, 4 * RT)) * FEW_STRIDE * (int)sizeof(float)));
-    kernel<<<dim3((n + FEW_COLS - 1) / FEW_COLS, 1, batch), 256, smem, s>>>(out, x, w, m, n, k, ldx, ldo, x_batch, o_batch);
-    return 0;
+template <int ROWS, int ADDERS>
+static int launch_rows(const GfArgs& a, bool vec, int split, cudaStream_t s) {
+#define HB_SPLIT(S) (vec ? launch_split<ROWS, ADDERS, S, true>(a, s) : launch_split<ROWS, ADDERS, S, false>(a, s))
+    return split == 8 ? HB_SPLIT(8) : split == 4 ? HB_SPLIT(4) : split == 2 ? HB_SPLIT(2) : HB_SPLIT(1);
+#undef HB_SPLIT
 }
 
-template <int RT>
-static int launch_few(float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx, long ldo,
-                      long x_batch, long o_batch, cudaStream_t s) {
-    const bool deep = (long)((n + FEW_COLS - 1) / FEW_COLS) * batch <= 296 && segment_length(k) > 3 * FEW_PIECE;
-    if constexpr (RT == 1)
-        if (deep) return launch_few_stages<RT, 6>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
-    return launch_few_stages<RT, 3>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
-}
+static int forced_split = 0;
+extern "C" int hb_gemm_f32_split(int split) { forced_split = split; return 0; }   // tests: segments shared by so many blocks (0: chosen)
 
 static int launch(const char* what, float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx,
                   long ldo, long x_batch, long o_batch, cudaStream_t s) {
     if (k <= 0) HB_REFUSE("%s: k = %d", what, k);
-    if ((m + BM - 1) / BM > 65535 || batch > 65535)
+    if ((m + 63) / 64 > 65535 || batch > 65535)
         HB_REFUSE("%s: %d rows, %d products are above the kernel's limits", what, m, batch);
     const bool vec = (k % 4 == 0) && (ldx % 4 == 0) && (x_batch % 4 == 0) && (((uintptr_t)x | (uintptr_t)w) % 16 == 0);
-    int rc;
-    // The kernel for few rows reads all of x once per 8 columns: from 9 rows on that is more than the tiles spend on their empty rows,
-    // unless there are few columns (k = 1,024 to 3,072, 16 rows: 1,024 columns 17 to 24 us against 24 to 33 as tiles, 6,144 columns 47
-    // against 37; 8 rows, 6,144 columns 23).
-    if (vec && (m <= FEW_ROWS / 2 || (m <= FEW_ROWS && n <= 2048))) {
-        if (m <= 4) rc = launch_few<1>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
-        else if (m <= 8) rc = launch_few<2>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
-        else rc = launch_few<4>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s);
-    } else {
-        // Two blocks an SM keep its multiply-adds busy: with fewer tiles than that, a tile's segments are shared out.
-        const long tiles = (long)((n + BN - 1) / BN) * ((m + BM - 1) / BM) * batch;
-        const int split = tiles * 8 <= 320 ? 8 : tiles * 4 <= 480 ? 4 : 1;
-#define HB_TILES(V, S) launch_tiles<V, S>(out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, s)
-        if (vec) rc = split == 8 ? HB_TILES(true, 8) : split == 4 ? HB_TILES(true, 4) : HB_TILES(true, 1);
-        else rc = split == 8 ? HB_TILES(false, 8) : split == 4 ? HB_TILES(false, 4) : HB_TILES(false, 1);
-#undef HB_TILES
+    const bool few = m <= 16;
+    const int parts = (m + 95) / 96, rows_x = few ? 16 : ((m + parts - 1) / parts + 15) / 16 * 16;
+    // How many blocks share a tile's segments: the launch with the least waves x (steps of 64 columns + what a block costs besides,
+    // about four steps, one more for a cluster's sums) wins. Blocks of many rows that walk all of k side by side ask for the same columns of rows
+    // whose distance is often a power of two: a step takes them 3.3 to 5 us, shared by two or more 1.8 to 2.2 (541 rows, 6,144 columns: 1,024 of k
+    // 119 us by blocks alone, 76 shared; 4,096 of k 581 and 255), so theirs count twice.
+    const long tiles = (long)((n + GF_BM - 1) / GF_BM) * ((m + rows_x - 1) / rows_x) * batch, slots = few ? 296 : 148;
+    const int steps = segment_length(k) / GF_BK, segments = (k + segment_length(k) - 1) / segment_length(k);
+    int split = 1;
+    long best = 0;
+    for (int c = 1; c <= GF_SEGMENTS; c *= 2) {
+        if (c > 1 && c >= 2 * segments) break;
+        const int share = GF_SEGMENTS / c, step = c == 1 && !few ? 2 : 1;
+        const long cost = (tiles * c + slots - 1) / slots * ((long)min(share, segments) * steps * step + 4 + (c > 1));
+        if (c == 1 || cost < best) { best = cost; split = c; }
     }
+    if (forced_split) split = forced_split;
+    const GfArgs a = {out, x, w, m, n, k, batch, ldx, ldo, x_batch, o_batch, rows_x};
+    const int rc = few ? launch_rows<16, 4>(a, vec, split, s) : launch_rows<96, 8>(a, vec, split, s);
     if (rc) return rc;
     HB_LAUNCH_CHECK(what);
+    return 0;
+}
+
+HB_DEFINE_STATUS_MIRROR(hb_gemm_f32_status_mirror)
+extern "C" int hb_gemm_f32_status(unsigned int* status) {
+    HB_CUDA(cudaDeviceSynchronize());
+    HB_CUDA(cudaMemcpyFromSymbol(status, g_tc_status, sizeof(unsigned int)));
+    const unsigned int zero = 0;
+    HB_CUDA(cudaMemcpyToSymbol(g_tc_status, &zero, sizeof(unsigned int)));
     return 0;
 }
 

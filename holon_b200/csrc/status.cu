@@ -10,6 +10,7 @@ extern "C" int hb_attention_tcgen05_status_mirror(unsigned int* word);
 extern "C" int hb_attention_maps_status_mirror(unsigned int* word);
 extern "C" int hb_latent_tcgen05_status_mirror(unsigned int* word);
 extern "C" int hb_latent_prompt_status_mirror(unsigned int* word);
+extern "C" int hb_gemm_f32_status_mirror(unsigned int* word);
 extern "C" int hb_gemm_tcgen05_status_mirror(unsigned int* word);
 extern "C" int hb_gemm_tcgen05_pair_status_mirror(unsigned int* word);
 extern "C" int hb_gemm_chain_status_mirror(unsigned int* word);
@@ -35,7 +36,7 @@ extern "C" int hb_status_word(unsigned int** host) {
             hb_gemm_tcgen05_pair_status_mirror(device) || hb_gemm_chain_status_mirror(device) ||
             hb_gemm_tickets_status_mirror(device) || hb_gemm_mid_status_mirror(device) ||
             hb_experts_tcgen05_status_mirror(device) || hb_attention_maps_status_mirror(device) || hb_latent_tcgen05_status_mirror(device) ||
-            hb_latent_prompt_status_mirror(device) ||
+            hb_latent_prompt_status_mirror(device) || hb_gemm_f32_status_mirror(device) ||
             hb_status_selftest_mirror(device))
             return HB_ERR_CUDA;
         g_word_host = word;

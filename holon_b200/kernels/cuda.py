@@ -865,7 +865,7 @@ class CudaKernels:
         out = 0
         for name in ("hb_gemm_tcgen05_status", "hb_gemm_tcgen05_pair_status", "hb_attention_tcgen05_status",
                      "hb_gemm_chain_status", "hb_gemm_tickets_status", "hb_gemm_mid_status", "hb_experts_tcgen05_status", "hb_attention_maps_status",
-                     "hb_latent_tcgen05_status", "hb_latent_prompt_status"):
+                     "hb_latent_tcgen05_status", "hb_latent_prompt_status", "hb_gemm_f32_status"):
             status = ctypes.c_uint(0)
             if getattr(self.lib, name)(ctypes.byref(status)):
                 raise KernelError(self.lib.hb_last_error().decode())
