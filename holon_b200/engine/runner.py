@@ -10,8 +10,10 @@ from collections.abc import Sequence
 
 import numpy as np
 import torch
+from torch.utils._device import DeviceContext
 
 from .batch import GroupStep, Rows, StepContext, StepEntry, Uploader
+from .recorded import Reads
 
 
 class StepError(ValueError):
@@ -19,28 +21,38 @@ class StepError(ValueError):
 
 
 class _Recorded:
-    """A step of one-token rows as a CUDA graph: its logits' buffer, the kernels it launches, and the weights it reads."""
+    """A step of one-token rows as a CUDA graph: its logits' buffer and the kernels it launches."""
 
-    __slots__ = ("graph", "logits", "launches", "weights")
+    __slots__ = ("graph", "logits", "launches")
 
-    def __init__(self, graph, logits, launches: int, weights) -> None:
-        self.graph, self.logits, self.launches, self.weights = graph, logits, launches, weights
+    def __init__(self, graph, logits, launches: int) -> None:
+        self.graph, self.logits, self.launches = graph, logits, launches
+
+
+def _watched() -> bool:
+    """Whether a mode of the caller's (torch's dispatch and function modes, but for a default device) sees each torch call of a step."""
+    modes = range(torch._C._len_torch_function_stack())
+    return torch._C._len_torch_dispatch_stack() > 0 or any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in modes)
 
 
 class Runner:
     GRAPHS = 8                                        # recorded steps a runner keeps, the last used ones
 
     def __init__(self, model, cache, build_ctx, max_step_tokens: int, cuda_graphs: bool = False) -> None:
-        """`cuda_graphs`: `step` records steps of one-token rows that come again and replays them."""
+        """`cuda_graphs`: `step` records steps of one-token rows that come again and replays them, where all that such a step
+        reads is understood (engine/recorded.py)."""
         self.model, self.cache, self.ctx = model, cache, build_ctx
-        self._use_graphs = cuda_graphs and build_ctx.device.type == "cuda"
+        self._graphs = cuda_graphs and build_ctx.device.type == "cuda"
         self._recorded: dict[tuple, _Recorded | None] = {}         # by shape and plan; None: seen once
-        self._params = self._pool = self._stream = None
+        self._pool = self._stream = None
         self.device, self.max_step_tokens = build_ctx.device, max_step_tokens
         s, t, g = cache.max_seqs + 1, max_step_tokens, len(cache.groups)
         tables = sum(s * (group.max_pages + 1) + 8 for group in cache.groups)     # every block-table row changed at once
         self.uploader = Uploader(t * (3 + g) + 16 * s + 64 + tables, self.device)
         self.vocab = model.spec.vocab
+        self._reads = Reads.of(*self._read()) if self._graphs else None
+        self._use_graphs = self._reads is not None                # whether steps may be recorded, as last looked
+        self._generation = self._wait = self._backoff = 0
 
     # ------------------------------------------------------------------ host half
     def check(self, entries: Sequence[StepEntry]) -> None:
@@ -147,40 +159,63 @@ class Runner:
         """Logits [wanted, vocab] in 32-bit, in the order of the entries and of each entry's `want`; None when
         nothing is wanted. Afterwards the cache holds the step's tokens."""
         self.check(entries)
-        if self._use_graphs and all(len(e.tokens) == 1 and tuple(e.want) == (0,) and not e.from_last for e in entries) \
-                and not torch.cuda.is_current_stream_capturing():
+        if self._graphs and all(len(e.tokens) == 1 and tuple(e.want) == (0,) and not e.from_last for e in entries) \
+                and not torch.cuda.is_current_stream_capturing() and not _watched() and self._settled():
             logits = self._single(entries)
         else:
             logits = self.model.forward(self.context(entries))
         self.commit(entries)
         return logits
 
+    def _read(self) -> tuple:
+        """What a step reads beside its own arrays."""
+        c = self.cache
+        return (self.model, c.kv_of_entry, c.slot_states, self.uploader.dev, *(g.table_device for g in c.groups))
+
+    def _settled(self) -> bool:
+        """Whether a step of this model may be recorded at all. Where something that it reads has been replaced, what was recorded
+        before is of an earlier generation and is not replayed again; whether the model may be recorded as it is now is looked at
+        a step later, and after ever more steps (the look takes about as long as a step) where it may not or where every step finds
+        something else replaced."""
+        if self._reads is not None and not self._reads.same(*self._read()):
+            self._reads, self._generation = None, self._generation + 1
+            self._wait = self._backoff = min(1023, 2 * self._backoff + 1)
+        if self._reads is None:
+            if self._wait:
+                self._wait -= 1
+            else:
+                self._reads = Reads.of(*self._read())
+                self._use_graphs = self._reads is not None
+                if self._reads is None:
+                    self._wait = self._backoff = min(1023, 2 * self._backoff + 1)
+        return self._use_graphs
+
     def _single(self, entries: Sequence[StepEntry]) -> torch.Tensor:
         """A step of one-token rows whose logits are all wanted. Enqueued kernel by kernel it is bound by the host (28 layers of
         width 1,024, five rows: 3.1 ms a step, 0.9 ms of it kernels; a trace of 2,200 tokens and six such steps takes 10.3 ms in place of 20.8), so a step whose
-        shape, plan, switches and weights have come before is recorded and from then on replayed. The first of a kind runs as it is: a
+        shape and plan have come before is recorded and from then on replayed, until anything that it reads is replaced
+        (`_settled`). The first of a kind runs as it is: a
         capture takes the host's time once more, which a step that never comes again would not earn back, and what
         kernels do for their first launch must not be captured. Both run with the plan that serves every step of the kind, so a
         step's logits do not depend on how it was run."""
         step = self.context(entries, pad_rows=0)
-        kernels = self.ctx.kernels
-        if self._params is None:
-            self._params = [p for _, p in self.model.params()]
-        weights = [p.tensor for p in self._params]
-        key = (len(entries), self.model.capture_plan(step, self.ctx.max_positions), getattr(kernels, "switches", None),
-               tuple(map(id, weights)))                # (recorded steps keep their weights: an id stands for one tensor)
+        if self._reads is None:
+            return self.model.forward(step)
+        key = (self._generation, len(entries), self.model.capture_plan(step, self.ctx.max_positions),
+               torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction)
         if key not in self._recorded:
             self._keep(key, None)
             return self.model.forward(step)
         found = self._recorded[key]
         if found is None:
-            found = self._record(step, weights)
+            found = self._record(step)
             if found is None:
                 return self.model.forward(step)
         self._keep(key, found)
+        self._backoff = 0
         found.graph.replay()
         if found.launches:
-            kernels.launches += found.launches
+            self.ctx.kernels.launches += found.launches
         return found.logits.clone()                    # (the buffer is the next replay's, too)
 
     def _keep(self, key, value) -> None:
@@ -189,7 +224,7 @@ class Runner:
         while len(self._recorded) > self.GRAPHS:
             del self._recorded[next(iter(self._recorded))]
 
-    def _record(self, step, weights) -> _Recorded | None:
+    def _record(self, step) -> _Recorded | None:
         """None, and no recording from then on, where a part does what a capture refuses (reads results on the host, say)."""
         kernels = self.ctx.kernels
         before = getattr(kernels, "launches", None)
@@ -205,7 +240,8 @@ class Runner:
                 finally:
                     graph.capture_end()
             except RuntimeError:
-                self._use_graphs, logits = False, None
+                self._graphs = self._use_graphs = False
+                logits = None
                 self._recorded.clear()
         main.wait_stream(self._stream)
         launches = 0
@@ -214,7 +250,7 @@ class Runner:
         if logits is None:
             return None
         self._pool = graph.pool()
-        return _Recorded(graph, logits, launches, weights)
+        return _Recorded(graph, logits, launches)
 
     def commit(self, entries: Sequence[StepEntry]) -> None:
         for e in entries:

@@ -80,6 +80,8 @@ class Branch:
 
 class CudaKernels:
     name = "cuda sm_100a"
+    recordable = True                         # (parts/base.py: Part.recordable) every attribute but these counts as a switch
+    counters = frozenset(("launches", "chain_launches", "chain_phases", "mid_launches", "_pending", "_side"))
 
     def __init__(self, device) -> None:
         self.device = torch.device(device)
@@ -186,14 +188,6 @@ class CudaKernels:
         self._status_word = word
 
     # ------------------------------------------------------------------ plumbing
-    @property
-    def switches(self) -> tuple:
-        """What decides, beside a call's own sizes, which kernel it launches: a recorded step serves steps under the same ones."""
-        return (self.prefill_attention, self.gemm, self.gemm_pair, self.attention_bf16, self.decode_attention, self.decode_cluster,
-                self.fused_qkv, self.fused_norm, self.mid_mode, self.mid_split, self.mid_min_rows, self.skinny32, self.decode_ctas,
-                self.latent_split, self.expert_products, self.expert_tile_rows, self.prefill_tile, self.chain, self.chain_cooperative,
-                self.branches, self.scan_parts)
-
     @property
     def mid(self) -> bool:
         """Whether steps of 17 to MID_ROWS rows keep their fused products (csrc/gemm_mid.cu)."""

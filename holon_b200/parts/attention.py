@@ -25,6 +25,8 @@ from .linear import Linear
 
 
 class GQA(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, heads: int, kv_heads: int, head_dim: int, hidden: int,
                  position: PartRef | None, qk_norm: PartRef | None = None, window: int = 0, layer: int = 0,
                  scale: float | None = None, unit_norm_eps: float | None = None, values_are_keys: bool = False,
@@ -139,6 +141,8 @@ class TalkingAttention(Part):
     The cache keeps per token and kv head one row [key | value] (`PagedRows`). `forward_biased` returns the output
     projection's product and its bias apart, for a block that adds the bias in its own sum."""
 
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, heads: int, kv_heads: int, key_dim: int, value_dim: int, hidden: int,
                  scale: float, position: PartRef | None = None, qk_eps: float | None = None, chunk: int = 0,
                  window: int = 0, talking: bool = True, head_temperature: bool = True, biases: bool | str = True,
@@ -236,6 +240,8 @@ class MapAttention(Part):
 
     q, k, v and g are one merged product. The cache keeps per token and kv head one row [key of map 1 | key of map 2 | value]
     (`PagedRows`)."""
+
+    recordable = True
 
     def __init__(self, ctx: BuildContext, *, heads: int, kv_heads: int, key_dim: int, value_dim: int, hidden: int, scale: float,
                  eps: float, maps: int = 1, diff: float | None = None, softcap: float | None = None, window: int = 0,

@@ -39,6 +39,11 @@ class Param:
 
 
 class Part:
+    #: A class that sets this to True of itself (it is not inherited) says: apart from what it enqueues on the device, `forward` does
+    #: nothing that outlives the step, and what it enqueues follows from the step's shape and plan and from the attributes of the part
+    #: and of what it holds. A step of such parts alone may be recorded and replayed without running them (engine/recorded.py).
+    recordable = False
+
     def __init__(self) -> None:
         self._params: dict[str, Param] = {}
         self._children: dict[str, "Part"] = {}
@@ -157,6 +162,8 @@ def unregister_part(kind: str, name: str) -> None:
 
 class BuildContext:
     """What parts see while they are built: device, dtype, the kernel table and the engine's limits."""
+
+    recordable = True
 
     def __init__(self, device, dtype: torch.dtype, kernels, max_positions: int, max_step_tokens: int = 0) -> None:
         self.device, self.dtype, self.kernels = torch.device(device), dtype, kernels

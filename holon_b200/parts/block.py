@@ -26,6 +26,8 @@ from .base import BuildContext, Link, NormedPair, Part, Residual, SlotState
 
 
 class PreNorm(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, layer: int, hidden: int, mixer: PartRef, ffn: PartRef | None,
                  norm: PartRef, residual_mult: float = 1.0) -> None:
         super().__init__()
@@ -71,6 +73,8 @@ class PreNorm(Part):
 class OutNorm(Part):
     """`average`: how many results this block averages (its own included; None: no averaging). `results`: how many the
     step's blocks leave in all, the embedding's rows included (the first block of a step makes room for them)."""
+
+    recordable = True
 
     KEY = "outnorm"                # step.shared: {"x": the stream's rows as the sublayers read them, "hist", "n"}
 
@@ -169,6 +173,8 @@ class OutNorm(Part):
 
 class Sandwich(Part):
     """Its norms offer `add`, `add_shifted`, `add_then` and `gather` (parts/norm.py: DynamicTanh)."""
+
+    recordable = True
 
     def __init__(self, ctx: BuildContext, *, layer: int, hidden: int, mixer: PartRef, ffn: PartRef | None, norm: PartRef,
                  shift: bool = False) -> None:

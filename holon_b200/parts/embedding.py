@@ -8,6 +8,8 @@ from .base import BuildContext, Part, Residual, SlotState
 
 
 class Embedding(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, vocab: int, hidden: int) -> None:
         super().__init__()
         self.ctx, self.vocab, self.hidden = ctx, vocab, hidden
@@ -24,6 +26,8 @@ class PairEmbedding(Embedding):
     (previous · mul_prev + token · mul_cur) mod buckets, and the table's last row (number `buckets`) for a sequence's
     first token. The previous token of a request's next step is part of its state: one int32 per slot, which the
     kernel reads for a row's first token and sets to the row's last. `buckets` None: no second table."""
+
+    recordable = True
 
     wants_step = True
 
@@ -46,6 +50,8 @@ class PairEmbedding(Embedding):
 
 
 class Head(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, vocab: int, hidden: int, tied: bool, embed: Embedding | None,
                  softcap: float | None = None) -> None:
         super().__init__()

@@ -43,6 +43,8 @@ EXPERT_ACTIVATIONS = ("relu2", "silu", "gelu_tanh")      # what the experts' pro
 
 
 class Experts(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, experts: int, top: int, scale: float, inter: int, hidden: int,
                  shared_inter: int | None = None, activation: str = "relu2", renormalize: bool = False,
                  gated: bool = False, router_bias: bool = False, identity: int = 0, groups: int = 1, keep_groups: int = 1,

@@ -17,6 +17,8 @@ from .linear import Linear
 
 
 class SwiGLU(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, inter: int, hidden: int, layer: int = 0) -> None:
         super().__init__()
         self.ctx, self.inter = ctx, inter
@@ -37,6 +39,8 @@ class SwiGLU(Part):
 
 
 class ClampedGLU(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, inter: int, hidden: int, limit: float, alpha: float = 1.702,
                  layer: int = 0) -> None:
         super().__init__()
@@ -67,6 +71,8 @@ class ClampedGLU(Part):
 
 
 class MLP(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, inter: int, hidden: int, activation: str = "gelu_tanh", layer: int = 0) -> None:
         super().__init__()
         from .experts import ACTIVATIONS

@@ -52,6 +52,8 @@ class Streams(Residual):
 
 
 class Hyper(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, streams: int, layer: int, hidden: int, mixer: PartRef,
                  ffn: PartRef | None, norm: PartRef) -> None:
         super().__init__()

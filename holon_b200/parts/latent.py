@@ -34,6 +34,8 @@ from .linear import Linear
 
 
 class LatentAttention(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, heads: int, dim: int, rot_dim: int, vdim: int, rank: int, scale: float,
                  hidden: int, norm: PartRef, position: PartRef | None, own_latent: bool = True, window: int = 0,
                  q_rank: int | None = None, gate: bool = True, sink: bool = False, layer: int = 0) -> None:

@@ -8,6 +8,8 @@ from .base import BuildContext, Part
 
 
 class Linear(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, name: str, width_in: int, pieces: dict[str, int], spare: int = 0) -> None:
         """`pieces`: loadable name -> rows, in the order they are stacked. `spare`: so many rows more behind them that
         no stored tensor fills; the part that asked for them writes them in its `finalize()`."""

@@ -35,6 +35,8 @@ class LayerCache:
 
 
 class Model(Part):
+    recordable = True
+
     def __init__(self, spec: ModelSpec, ctx: BuildContext) -> None:
         super().__init__()
         self.spec, self.ctx = spec, ctx

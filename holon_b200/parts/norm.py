@@ -12,6 +12,8 @@ from .base import BuildContext, PairRows, Part, Residual
 
 
 class RMSNorm(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, eps: float, dim: int, offset: float = 0.0) -> None:
         super().__init__()
         self.ctx, self.eps, self.dim, self.offset = ctx, float(eps), dim, float(offset)
@@ -48,6 +50,8 @@ class RMSNorm(Part):
 class LayerNorm(Part):
     """`takes_pairs`: a pending output may still be rows of (token, choice) pairs (base.PairRows) and may carry a factor
     (`Residual.delta_scale`); the kernel that norms the sum does both."""
+
+    recordable = True
 
     takes_pairs = True
     links = False                            # its statistics need the whole row: no product leaves its rows behind (base.Link)
@@ -89,6 +93,8 @@ class DynamicTanh(Part):
     `alpha`; 32-bit arithmetic, one rounding at the end. A block may leave a part's output pending on the stream
     together with the norm it passes before it is added (`Residual.delta`, `Residual.delta_by`); `add` and `gather`
     fold both in."""
+
+    recordable = True
 
     def __init__(self, ctx: BuildContext, *, dim: int, eps: float = 0.0) -> None:
         super().__init__()

@@ -23,6 +23,8 @@ from .model import LayerCache
 
 
 class SideBySide(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, left: PartRef, right: PartRef, left_scale: float, right_scale: float,
                  hidden: int, layer: int = 0, out_eps: float | None = None) -> None:
         super().__init__()
@@ -91,6 +93,8 @@ class SideBySide(Part):
 
 
 class ParallelBlock(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, layer: int, hidden: int, mixer: PartRef, ffn: PartRef | None,
                  norm: PartRef) -> None:
         super().__init__()

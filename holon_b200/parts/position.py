@@ -21,6 +21,8 @@ from .base import BuildContext, Part
 
 
 class Rope(Part):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, theta: float, rotary_dim: int, head_dim: int, interleaved: bool = False,
                  factor: float = 1.0, yarn: tuple[float, float, float, float] | None = None) -> None:
         super().__init__()

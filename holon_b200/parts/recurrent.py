@@ -78,6 +78,8 @@ class _MatrixState(Part):
 
 
 class Retention(_MatrixState):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, heads: int, dim: int, vdim: int, decay: tuple[float, ...], eps: float,
                  hidden: int, position: PartRef | None, layer: int = 0) -> None:
         super().__init__()
@@ -116,6 +118,8 @@ class Retention(_MatrixState):
 
 
 class Lightning(_MatrixState):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, heads: int, dim: int, vdim: int, decay: tuple[float, ...], eps: float,
                  hidden: int, layer: int = 0) -> None:
         super().__init__()
@@ -152,6 +156,7 @@ class Lightning(_MatrixState):
 
 
 class GatedDelta(_MatrixState):
+    recordable = True
     UNIT_EPS = 1e-6                       # inside the root of the unit vectors
 
     def __init__(self, ctx: BuildContext, *, heads: int, kv_heads: int, dim: int, vdim: int, taps: int, decay_rank: int,
@@ -215,6 +220,7 @@ class GatedDelta(_MatrixState):
 
 
 class MLSTM(_MatrixState):
+    recordable = True
     TINY = 1e-6                           # added to the denominator of the read-out
 
     def __init__(self, ctx: BuildContext, *, heads: int, dim: int, vdim: int, gate_cap: float, eps: float, hidden: int,
@@ -252,6 +258,8 @@ class MLSTM(_MatrixState):
 
 
 class GeneralDelta(_MatrixState):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, heads: int, dim: int, decay_rank: int, eps: float, hidden: int,
                  decay_scale: float = 0.6065306597126334, unit_eps: float = 1e-6, layer: int = 0) -> None:
         super().__init__()
@@ -290,6 +298,8 @@ class GeneralDelta(_MatrixState):
 
 
 class StateSpace(_MatrixState):
+    recordable = True
+
     def __init__(self, ctx: BuildContext, *, heads: int, vdim: int, state: int, groups: int, taps: int, norm_groups: int, eps: float,
                  hidden: int, layer: int = 0) -> None:
         super().__init__()

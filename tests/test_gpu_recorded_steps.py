@@ -3,8 +3,10 @@ between the steps of a kind, and no recording where a part cannot be captured.""
 import pytest
 import torch
 
+from rulorax_tools import CONFIGS as RULORAX
+
 from holon_b200.engine import StepEntry, build
-from holon_b200.weights import RandomSource
+from holon_b200.weights import RandomSource, load_weights
 
 pytestmark = pytest.mark.gpu
 CONFIG = dict(architectures=["Qwen3ForCausalLM"], num_hidden_layers=2, hidden_size=128, num_attention_heads=4, num_key_value_heads=2, head_dim=32,
@@ -19,7 +21,7 @@ def made(dtype="bfloat16", graphs=True):
 
 def trace(built, lengths, steps, seed=1, between=None):
     g = torch.Generator().manual_seed(seed)
-    ids = [torch.randint(0, 331, (n + steps,), generator=g).tolist() for n in lengths]
+    ids = [torch.randint(0, built.model.spec.vocab, (n + steps,), generator=g).tolist() for n in lengths]
     out, cache = [], built.cache
     with torch.inference_mode():
         slots = [cache.admit() for _ in ids]
@@ -96,3 +98,85 @@ def test_a_part_that_cannot_be_captured():
     a, b = trace(built, [9, 30], 6), trace(plain, [9, 30], 6)
     assert not built.runner._use_graphs and len(seen) >= 7
     assert all(torch.linalg.norm(x - y) <= 2e-2 * torch.linalg.norm(y) for x, y in zip(a, b))
+
+
+def latent(graphs=True, seed=5):
+    with torch.inference_mode():
+        return build(RandomSource(RULORAX["a"], seed=seed, device="cuda:0", dtype=torch.float32), dtype="float32", device="cuda:0", page_size=16, max_seqs=4,
+                     max_model_len=256, max_step_tokens=256, pages=64, cuda_graphs=graphs)
+
+
+def replayed(built):
+    return sum(r is not None for key, r in built.runner._recorded.items() if key[0] == built.runner._generation)
+
+
+def close(a, b):
+    return all(torch.linalg.norm(x - y) <= 1e-5 * torch.linalg.norm(y) for x, y in zip(a, b, strict=True))
+
+
+def test_weights_that_are_loaded_again():
+    """The same tensors with other numbers: what latent attention derives from them is another tensor."""
+    built, plain = latent(), latent(graphs=False, seed=6)
+    trace(built, [9, 30], 5)
+    assert replayed(built) == 1
+    with torch.inference_mode():
+        load_weights(built.model, built.model.spec, RandomSource(RULORAX["a"], seed=6, device="cuda:0", dtype=torch.float32).tensors(), torch.float32, "cuda:0")
+        torch.cuda.empty_cache()
+    want = trace(plain, [9, 30], 6)
+    assert close(trace(built, [9, 30], 6), want) and close(trace(built, [9, 30], 6), want) and replayed(built) == 1
+
+
+def test_weights_swapped_and_swapped_back():
+    built, plain = latent(), latent(graphs=False)
+    want = trace(plain, [9, 30], 6)
+    assert close(trace(built, [9, 30], 6), want)
+    own = {n: p.tensor for n, p in built.model.params()}
+    for other in (True, False):
+        for n, p in built.model.params():
+            p.tensor = own[n] * 0.5 if other and own[n].is_floating_point() else own[n]
+        with torch.inference_mode():
+            built.model.finalize()
+        got = [trace(built, [9, 30], 6) for _ in range(3)]
+        assert all(close(x, want) != other for x in got) and all(torch.equal(a, b) for x in got for a, b in zip(x, got[0]))
+
+
+def test_storage_behind_a_parameter_and_a_number_of_a_part():
+    built, plain = latent(), latent(graphs=False)
+    trace(built, [9, 30], 4)
+    for b in (built, plain):
+        with torch.inference_mode():
+            p = next(p for n, p in b.model.params() if n.endswith("out.weight"))
+            p.tensor.data = p.tensor.data * 3.0
+    want = trace(plain, [9, 30], 6)
+    assert close(trace(built, [9, 30], 6), want) and close(trace(built, [9, 30], 6), want)
+    for b in (built, plain):
+        b.model.layers[0].mixer.scale *= 2.0
+    other = trace(plain, [9, 30], 6)
+    assert not close(other, want) and close(trace(built, [9, 30], 6), other) and close(trace(built, [9, 30], 6), other) and replayed(built)
+
+
+def test_a_part_with_python_of_its_own_runs_in_every_step():
+    """A wrapped `forward`, set before or after steps were recorded, and a part of a class that does not declare itself."""
+    built, plain = made("float32"), made("float32", graphs=False)
+    want = trace(plain, [9, 30], 6)
+    trace(built, [9, 30], 4)
+    assert replayed(built) == 1
+    forward, kept = built.model.head.forward, []
+
+    def watching(rows):
+        kept.append(rows.clone())
+        return forward(rows)
+
+    built.model.head.forward = watching
+    assert close(trace(built, [9, 30], 6), want) and len(kept) == 7 and all(len(x) for x in kept) and len({x.data_ptr() for x in kept}) == 7
+    del built.model.head.forward
+    other = made("float32")
+    seen = []
+
+    class Head(type(other.model.head)):
+        def forward(self, rows):
+            seen.append(rows.shape[0])
+            return super().forward(rows)
+
+    other.model.head.__class__ = Head
+    assert close(trace(other, [9, 30], 6), want) and close(trace(other, [9, 30], 6), want) and seen == [2] * 14 and not any(other.runner._recorded.values())
