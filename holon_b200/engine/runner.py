@@ -6,6 +6,7 @@ admitted the requests and reserved their pages; the step checks that and fails b
 """
 from __future__ import annotations
 
+import warnings
 from collections.abc import Sequence
 
 import numpy as np
@@ -37,14 +38,16 @@ def _watched() -> bool:
 
 class Runner:
     GRAPHS = 8                                        # recorded steps a runner keeps, the last used ones
+    SEEN = 64                                         # kinds of steps it remembers to have run once
 
     def __init__(self, model, cache, build_ctx, max_step_tokens: int, cuda_graphs: bool = False) -> None:
         """`cuda_graphs`: `step` records steps of one-token rows that come again and replays them, where all that such a step
         reads is understood (engine/recorded.py)."""
         self.model, self.cache, self.ctx = model, cache, build_ctx
         self._graphs = cuda_graphs and build_ctx.device.type == "cuda"
-        self._recorded: dict[tuple, _Recorded | None] = {}         # by shape and plan; None: seen once
-        self._pool = self._stream = None
+        self._recorded: dict[tuple, _Recorded] = {}                # by shape and plan
+        self._seen: dict[tuple, None] = {}                         # kinds that came once
+        self._pool = self._stream = None                           # the recordings' memory (None: there are none)
         self.device, self.max_step_tokens = build_ctx.device, max_step_tokens
         s, t, g = cache.max_seqs + 1, max_step_tokens, len(cache.groups)
         tables = sum(s * (group.max_pages + 1) + 8 for group in cache.groups)     # every block-table row changed at once
@@ -203,35 +206,38 @@ class Runner:
             return self.model.forward(step)
         key = (self._generation, len(entries), self.model.capture_plan(step, self.ctx.max_positions),
                torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction)
-        if key not in self._recorded:
-            self._keep(key, None)
-            return self.model.forward(step)
-        found = self._recorded[key]
-        if found is None:
+        found = self._recorded.get(key)
+        if found is None and key in self._seen:
+            del self._seen[key]
             found = self._record(step)
-            if found is None:
-                return self.model.forward(step)
-        self._keep(key, found)
+        elif found is None:
+            self._keep(self._seen, key, None, self.SEEN)
+        if found is None:
+            return self.model.forward(step)
+        self._keep(self._recorded, key, found, self.GRAPHS)
         self._backoff = 0
         found.graph.replay()
         if found.launches:
             self.ctx.kernels.launches += found.launches
         return found.logits.clone()                    # (the buffer is the next replay's, too)
 
-    def _keep(self, key, value) -> None:
-        self._recorded.pop(key, None)
-        self._recorded[key] = value
-        while len(self._recorded) > self.GRAPHS:
-            del self._recorded[next(iter(self._recorded))]
+    @staticmethod
+    def _keep(kept: dict, key, value, most: int) -> None:
+        kept.pop(key, None)
+        kept[key] = value
+        while len(kept) > most:
+            del kept[next(iter(kept))]
 
     def _record(self, step) -> _Recorded | None:
-        """None, and no recording from then on, where a part does what a capture refuses (reads results on the host, say)."""
+        """None where it did not work: for want of memory (the step is recorded another time), or, and then nothing is recorded from then on,
+        where a part does what a capture refuses (reads results on the host, say) although it says that it may be recorded."""
         kernels = self.ctx.kernels
         before = getattr(kernels, "launches", None)
         graph, main = torch.cuda.CUDAGraph(), torch.cuda.current_stream(self.device)
         if self._stream is None:
             self._stream = torch.cuda.Stream(self.device)
         self._stream.wait_stream(main)
+        logits = error = None
         with torch.cuda.stream(self._stream):
             try:
                 graph.capture_begin(pool=self._pool, capture_error_mode="thread_local")
@@ -239,18 +245,26 @@ class Runner:
                     logits = self.model.forward(step)
                 finally:
                     graph.capture_end()
-            except RuntimeError:
-                self._graphs = self._use_graphs = False
-                logits = None
-                self._recorded.clear()
+            except RuntimeError as e:
+                error = e.__context__ or e             # (the capture's end fails, too, once something in it has failed)
         main.wait_stream(self._stream)
         launches = 0
         if before is not None:
             launches, kernels.launches = kernels.launches - before, before
-        if logits is None:
+        if error is None:
+            self._pool = graph.pool()
+            return _Recorded(graph, logits, launches)
+        if getattr(kernels, "_pending", None):         # (queued for a launch that was to be recorded)
+            kernels._pending.clear()
+        if isinstance(error, torch.OutOfMemoryError):
             return None
-        self._pool = graph.pool()
-        return _Recorded(graph, logits, launches)
+        if "captur" not in str(error):
+            raise error
+        warnings.warn(f"steps of one-token rows run kernel by kernel from here on: {error}")
+        self._graphs = self._use_graphs = False
+        self._recorded.clear()
+        self._pool = None                              # (a pool without a graph is given back: its name stands for nothing)
+        return None
 
     def commit(self, entries: Sequence[StepEntry]) -> None:
         for e in entries:

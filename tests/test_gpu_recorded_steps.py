@@ -107,7 +107,7 @@ def latent(graphs=True, seed=5):
 
 
 def replayed(built):
-    return sum(r is not None for key, r in built.runner._recorded.items() if key[0] == built.runner._generation)
+    return sum(key[0] == built.runner._generation for key in built.runner._recorded)
 
 
 def close(a, b):
@@ -179,4 +179,70 @@ def test_a_part_with_python_of_its_own_runs_in_every_step():
             return super().forward(rows)
 
     other.model.head.__class__ = Head
-    assert close(trace(other, [9, 30], 6), want) and close(trace(other, [9, 30], 6), want) and seen == [2] * 14 and not any(other.runner._recorded.values())
+    assert close(trace(other, [9, 30], 6), want) and close(trace(other, [9, 30], 6), want) and seen == [2] * 14 and not other.runner._recorded
+
+
+def test_kinds_that_come_once_take_no_recordings_place():
+    built = made()
+    built.runner.GRAPHS = 2
+    trace(built, [5], 3)
+    graph = next(iter(built.runner._recorded.values()))
+    for rows in (2, 3, 4):
+        trace(built, [5] * rows, 1)
+    assert list(built.runner._recorded.values()) == [graph] and len(built.runner._seen) == 3
+    trace(built, [5] * 2, 1)
+    assert replayed(built) == 2 and built.runner._use_graphs and len(built.runner._seen) == 2
+    built.runner.SEEN = 1
+    trace(built, [500] * 2, 1)
+    trace(built, [600] * 1, 1)
+    assert len(built.runner._seen) == 1
+
+
+def declared(built, before):
+    """`before()` in every pass of a head that says it may be recorded."""
+    class Head(type(built.model.head)):
+        recordable = True
+
+        def forward(self, rows):
+            before(rows)
+            return super().forward(rows)
+
+    built.model.head.__class__ = Head
+
+
+def test_a_capture_without_memory_is_tried_again():
+    built, plain = made("float32"), made("float32", graphs=False)
+    failed = []
+
+    def before(rows):
+        if torch.cuda.is_current_stream_capturing() and len(failed) < 2:
+            failed.append(rows.shape)
+            raise torch.OutOfMemoryError("CUDA out of memory")
+
+    declared(built, before)
+    assert close(trace(built, [9, 30], 12), trace(plain, [9, 30], 12))
+    assert len(failed) == 2 and replayed(built) == 1 and built.runner._use_graphs
+    assert close(trace(built, [9, 30], 3), trace(plain, [9, 30], 3))
+
+
+def test_a_part_that_says_so_and_cannot_be_captured():
+    built, plain = made("float32"), made("float32", graphs=False)
+    seen = []
+    declared(built, lambda rows: seen.append(float(rows.float().sum().item())))
+    with pytest.warns(UserWarning, match="kernel by kernel"):
+        a = trace(built, [9, 30], 8)
+    assert close(a, trace(plain, [9, 30], 8)) and not built.runner._use_graphs and not built.runner._recorded and built.runner._pool is None
+    assert len(seen) == 9                                  # (the capture ended ahead of its number)
+
+
+def test_an_error_of_a_part_stays_its_own():
+    built = made("float32")
+
+    def before(rows):
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("a fault of its own")
+
+    declared(built, before)
+    with pytest.raises(RuntimeError, match="a fault of its own"):
+        trace(built, [9, 30], 8)
+    assert built.runner._use_graphs and torch.cuda.current_stream().query() in (True, False)
