@@ -21,7 +21,7 @@ TORCH_DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
 @dataclasses.dataclass
 class Memory:
     """Bytes of device memory, as found when the engine was built. `activations` and `graphs` are measured (the peak
-    of a worst-case step, and of the largest step that is replayed from a graph) when the cache's size follows from
+    of a worst-case step, and of the largest step that is replayed from a graph; `_measure`) when the cache's size follows from
     `memory_fraction`; with a size given by the caller nothing is run and they are None."""
 
     weights: int
@@ -78,10 +78,12 @@ def _cuts(tokens: int, rows: int, longest: int, lengths=()) -> list[list[int]]:
 
 def _measure(model, ctx, entries, *, page_size: int, max_seqs: int, max_model_len: int, max_step_tokens: int,
              chunk_with_decode: int, dtype, device) -> tuple[int, int]:
-    """The activation peaks of (1) the largest step the scheduler can make: `max_step_tokens` prompt tokens in as
+    """Bytes for the activations of (1) the largest step the scheduler can make: `max_step_tokens` prompt tokens in as
     many rows as may end a prompt in one step, every row sampled, and the same tokens in other cuts, since scratch may grow
-    with a row's length (`costly_rows` of a kernel table: the lengths at which it is largest for the tokens); (2) the largest step replayed from a CUDA graph:
-    one token for every sequence beside `chunk_with_decode` prompt tokens. Both run through the engine's own step
+    with a row's length (`costly_rows` of a kernel table: the lengths at which it is largest for the tokens), and the scratch that tokens before them in the cache
+    may cost besides (`Part.context_scratch`: such steps are not run here); (2) the largest step replayed from a CUDA graph:
+    one token for every sequence beside `chunk_with_decode` prompt tokens, laid out and planned as one that is
+    recorded, and the logits that a runner's recorded steps leave in a place of their own. Steps run through the engine's own step
     function on pools just large enough to hold them, which are freed again (executor.py:208-234 does the same on
     minimum-size pools)."""
     from ..sampling import Sampler, SamplingParams, sampling_arrays
@@ -95,7 +97,7 @@ def _measure(model, ctx, entries, *, page_size: int, max_seqs: int, max_model_le
     runner, sampler = Runner(model, cache, ctx, max_step_tokens), Sampler(ctx.kernels, device)
     params = SamplingParams(temperature=1.0)
 
-    def step(counts) -> None:
+    def step(counts, graph=False) -> None:
         batch = []
         for n in counts:
             slot = cache.admit()
@@ -103,7 +105,9 @@ def _measure(model, ctx, entries, *, page_size: int, max_seqs: int, max_model_le
             batch.append(StepEntry(slot, [0] * n, 0, (n - 1,)))
         arrays = sampling_arrays([(params, 1, n) for n in counts])
         arrays["sample_slot"] = np.array([e.slot for e in batch], dtype=np.int32)
-        ctx_ = runner.context(batch, extra=arrays)
+        ctx_ = runner.context(batch, pad_rows=0 if graph else None, extra=arrays)
+        if graph:
+            model.capture_plan(ctx_, max_model_len)
         logits = model.forward(ctx_)
         sampler.sample(logits, ctx_.extra, False)
         for e in batch:
@@ -111,7 +115,8 @@ def _measure(model, ctx, entries, *, page_size: int, max_seqs: int, max_model_le
 
     cuts = _cuts(tokens, rows, max_model_len - 1, getattr(ctx.kernels, "costly_rows", ()))
     largest = max(_peak_of(device, lambda counts=counts: step(counts)) for counts in cuts)
-    graphed = _peak_of(device, lambda: step(ones + [n for n in portion if n > 0]))
+    largest += model.context_scratch(tokens, rows, max_model_len)
+    graphed = _peak_of(device, lambda: step(ones + [n for n in portion if n > 0], graph=True)) + 4 * max_seqs * model.spec.vocab
     del runner, cache
     torch.cuda.empty_cache()
     return largest, graphed

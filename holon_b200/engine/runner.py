@@ -22,7 +22,7 @@ class StepError(ValueError):
 
 
 class _Recorded:
-    """A step of one-token rows as a CUDA graph: its logits' buffer and the kernels it launches."""
+    """A step of one-token rows as a CUDA graph that leaves its logits in `logits`, and the kernels it launches."""
 
     __slots__ = ("graph", "logits", "launches")
 
@@ -48,6 +48,7 @@ class Runner:
         self._recorded: dict[tuple, _Recorded] = {}                # by shape and plan
         self._seen: dict[tuple, None] = {}                         # kinds that came once
         self._pool = self._stream = None                           # the recordings' memory (None: there are none)
+        self._logits = None                                        # [max_seqs, vocab]: where all of them leave their logits
         self.device, self.max_step_tokens = build_ctx.device, max_step_tokens
         s, t, g = cache.max_seqs + 1, max_step_tokens, len(cache.groups)
         tables = sum(s * (group.max_pages + 1) + 8 for group in cache.groups)     # every block-table row changed at once
@@ -219,7 +220,7 @@ class Runner:
         found.graph.replay()
         if found.launches:
             self.ctx.kernels.launches += found.launches
-        return found.logits.clone()                    # (the buffer is the next replay's, too)
+        return found.logits.clone()                    # (the place is the next replay's, too)
 
     @staticmethod
     def _keep(kept: dict, key, value, most: int) -> None:
@@ -237,12 +238,19 @@ class Runner:
         if self._stream is None:
             self._stream = torch.cuda.Stream(self.device)
         self._stream.wait_stream(main)
-        logits = error = None
+        error = None
+        try:
+            if self._logits is None:
+                with torch.inference_mode(False):      # (steps in and out of that mode write it)
+                    self._logits = torch.empty(self.cache.max_seqs, self.vocab, dtype=torch.float32, device=self.device)
+        except torch.OutOfMemoryError:
+            return None
+        logits = self._logits[:len(step.logits_index)]
         with torch.cuda.stream(self._stream):
             try:
                 graph.capture_begin(pool=self._pool, capture_error_mode="thread_local")
                 try:
-                    logits = self.model.forward(step)
+                    logits.copy_(self.model.forward(step))      # (a step's own logits are the pool's, as all it makes)
                 finally:
                     graph.capture_end()
             except RuntimeError as e:

@@ -1020,12 +1020,23 @@ class CudaKernels:
                 or self.prefill_attention != "tcgen05" or self.attention_bf16 != "fast" or not scale > 0 \
                 or any(t.dtype != torch.bfloat16 or t.data_ptr() % 16 or t.stride(0) % 8 for t in tensors):
             return False
-        key = ("latent prompt", dim, rot, vdim, rank)
-        if key not in self._splits:
-            self._splits[key] = int(self.lib.hb_latent_prompt_takes(dim, rot, vdim, rank))
         total = self._latent_rows(rows, window)
-        return bool(self._splits[key]) and total <= self.LATENT_KEYS * (rows.n_tokens - rows.n_decode) + 64 * (rows.n_rows - rows.n_decode) \
+        return self._latent_prompt_takes(dim, rot, vdim, rank) and total <= self.LATENT_KEYS * (rows.n_tokens - rows.n_decode) + 64 * (rows.n_rows - rows.n_decode) \
             and 2 * total * (heads * (dim + vdim) + rank + rot) <= self.LATENT_SCRATCH and self._query_tiles(rows, 128) <= 65535
+
+    def latent_scratch(self, tokens, rows, longest, heads, dim, rot, vdim, rank) -> int:
+        """The most bytes that `latent_prompt` takes for portions of `tokens` tokens in up to `rows` rows, whatever they see of up to `longest`
+        cache rows each: what `latent_expands` allows."""
+        if not self._latent_prompt_takes(dim, rot, vdim, rank):
+            return 0
+        seen = min(self.LATENT_KEYS * tokens + 64 * rows, rows * -(-longest // 64) * 64)
+        return min(self.LATENT_SCRATCH, 2 * seen * (heads * (dim + vdim) + rank + rot))
+
+    def _latent_prompt_takes(self, *sizes: int) -> bool:
+        key = ("latent prompt", *sizes)
+        if key not in self._splits:
+            self._splits[key] = int(self.lib.hb_latent_prompt_takes(*sizes))
+        return bool(self._splits[key])
 
     @staticmethod
     def _latent_rows(rows, window: int) -> int:

@@ -72,6 +72,11 @@ class Part:
         for name, child in self._children.items():
             yield from child.loadables(f"{prefix}{name}.")
 
+    def context_scratch(self, tokens: int, rows: int, longest: int) -> int:
+        """Bytes of scratch that a step of `tokens` prompt tokens in up to `rows` rows may take at most because of what lies before them in
+        the cache (a request holds up to `longest` tokens). What the new tokens alone ask for is measured; this is added to it."""
+        return max((child.context_scratch(tokens, rows, longest) for child in self._children.values()), default=0)
+
     def finalize(self) -> None:
         """Called once after every parameter holds its tensor. What needs the tensors, the device or the kernel table
         (derived tensors, a library of the part's own: `ctx.kernels.extension`) is done here, not in the constructor:

@@ -76,6 +76,12 @@ class LatentAttention(Part):
         if self.ukv.tensor is not None:
             self.uk_t = self.ukv.tensor[:self.heads * self.dim].view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
 
+    def context_scratch(self, tokens: int, rows: int, longest: int) -> int:
+        scratch = getattr(self.ctx.kernels, "latent_scratch", None)
+        if scratch is None or self.ctx.dtype != torch.bfloat16:
+            return 0
+        return scratch(tokens, rows, longest, self.heads, self.dim, self.rot_dim, self.vdim, self.rank)
+
     def cache(self) -> PagedLatent:
         return PagedLatent(self.rank, self.rot_dim, self.window)
 

@@ -426,3 +426,38 @@ def test_the_measured_peak_covers_one_long_prompt():
 
         for counts in ([4096], [2000, 2096], [129] * 31, [200] * 20):
             assert _peak_of(built.ctx.device, lambda: step(counts)) <= built.memory.activations + (2 << 20), counts
+
+
+def test_the_account_covers_portions_behind_a_context_and_steps_as_graphs_run_them():
+    """Latent attention makes keys and values of all that a prompt's portion sees, and not where a graph serves every cut of its tokens:
+    neither needs more than the account says, although neither is the largest step from an empty cache."""
+    import torch
+    from holon_b200.engine import StepEntry, build
+    from holon_b200.engine.build import _peak_of
+    from holon_b200.weights import RandomSource
+    mixer = {"heads": 16, "dim": 128, "rot_dim": 64, "vdim": 128, "kv_rank": 512, "rot": {"base": 10000.0, "dims": 64}, "scale": 192 ** -0.5}
+    config = {"architecture": "Rulorax", "width": 256, "vocab": 1024, "norm": {"eps": 1e-6}, "streams": 1,
+              "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": {"kind": "dense", "ff": 256}}]}
+    with torch.inference_mode():
+        built = build(RandomSource(config, seed=1, device="cuda:0", dtype=torch.bfloat16), dtype="bfloat16", device="cuda:0", page_size=64,
+                      max_seqs=4, max_model_len=8192, max_step_tokens=1024, memory_fraction=0.05, chunk_with_decode=1000)
+        cache, runner, slack = built.cache, built.runner, 2 << 20
+        slot = cache.admit()
+        assert cache.reserve(slot, 8190)
+        for start in range(0, 6900, 1024):
+            runner.step([StepEntry(slot, [5] * min(1024, 6900 - start), start, [])])
+        peak = _peak_of(built.ctx.device, lambda: runner.step([StepEntry(slot, [5] * 1000, 6900, [999])]))
+        assert 2 * 7936 * (16 * 256 + 576) <= peak <= built.memory.activations + slack
+        cache.release(slot)
+
+        def graphed():
+            slots = [cache.admit() for _ in range(4)]
+            entries = [StepEntry(s, [5] * n, 0, [n - 1]) for s, n in zip(slots, (1, 1, 1, 1000))]
+            assert all(cache.reserve(e.slot, len(e.tokens)) for e in entries)
+            step = runner.context(entries, pad_rows=0)
+            built.model.capture_plan(step, 8192)
+            built.model.forward(step)
+            for s in slots:
+                cache.release(s)
+
+        assert _peak_of(built.ctx.device, graphed) <= built.memory.graphs + slack

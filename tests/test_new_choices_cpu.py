@@ -58,6 +58,28 @@ def test_rows_seen_and_scratch():
     assert expands(table(), rows([30_000], [30_000])) and not expands(table(), rows([70_000], [70_000]), heads=32)
 
 
+def test_the_account_covers_what_portions_may_take():
+    """Whatever portions of a step's tokens see: where they take the form that makes keys and values, its scratch is in the account."""
+    import random
+    k, rng, most = table(), random.Random(7), 0
+    heads, dim, rot, vdim, rank = 16, 128, 64, 128, 512
+    for _ in range(400):
+        tokens, seqs, longest = rng.choice([64, 512, 4096]), rng.choice([1, 3, 16]), rng.choice([300, 2048, 8192])
+        new, left = [], tokens
+        while left > 1 and len(new) < seqs:
+            new.append(min(left, longest, max(2, left if rng.random() < 0.3 else rng.randrange(2, left + 1))))
+            left -= new[-1]
+        lens = [min(longest, n + int(rng.choice([0, 1, 7, 9]) * n * rng.random() * 1.2)) for n in new]
+        r, window = rows(new, lens), rng.choice([0, 0, 100])
+        if expands(k, r, window=window):
+            taken = 2 * k._latent_rows(r, window) * (heads * (dim + vdim) + rank + rot)
+            bound = k.latent_scratch(tokens, seqs, longest, heads, dim, rot, vdim, rank)
+            assert taken <= bound <= k.LATENT_SCRATCH
+            most = max(most, taken / bound)
+    assert most > 0.9
+    assert k.latent_scratch(512, 2, 4096, heads, dim, 32, vdim, rank) == 0            # (sizes that keep the folded form)
+
+
 def test_tensors_that_do_not_fit_sixteen_bytes():
     wide = torch.zeros(64, 40, dtype=BF16)
     assert expands(table(), rows([300], [300]), tensors=(wide, wide[:, :16]))
