@@ -66,3 +66,19 @@ def test_more_experts_than_the_kernel_counts(K):
         REF.expert_linear(want, x, None, w, starts, 0)
         close(out, want, torch.bfloat16, scale=2.0)
     K.expert_products = "tcgen05"
+
+
+@pytest.mark.parametrize("clamped", [False, True])
+def test_gates_far_below_zero(K, clamped):
+    """silu(-88) is -5.3e-37: no zero, although what it is divided by is beyond 2^126."""
+    rows, k, inter = 300, 64, 8
+    x, w = torch.zeros(rows, k, dtype=torch.bfloat16), torch.zeros(1, 2 * inter, k, dtype=torch.bfloat16)
+    x[:, 3], w[0, :inter, 3], w[0, inter:, 3] = 1.0, torch.linspace(-88.5, -86.5, inter), 2.0
+    starts, out = torch.tensor([0, rows], dtype=torch.int32), torch.empty(rows, inter, dtype=torch.bfloat16, device=DEV)
+    if clamped:
+        K.expert_glu(out, x.to(DEV), None, w.to(DEV), starts.to(DEV), 100.0, 1.0, None)
+    else:
+        K.expert_swiglu(out, x.to(DEV), None, w.to(DEV), starts.to(DEV))
+    gate, up = w[0, :inter, 3].double(), 2.0
+    want = (gate * torch.sigmoid(gate) * (up + 1.0 if clamped else up)).expand(rows, inter)
+    assert ((out.cpu().double() - want).abs() <= 2.0 ** -8 * want.abs()).all()           # (a bfloat16 rounding, and 88 log2(e) to 2^-17)
