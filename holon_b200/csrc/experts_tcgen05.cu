@@ -40,6 +40,7 @@ __global__ void gather_rows_kernel(bf16* __restrict__ out, const bf16* __restric
 __device__ __forceinline__ float xt_act(float v, int act) {
     if (act == 1) { v = fmaxf(v, 0.f); return v * v; }
     if (act == 2) return v / (1.f + __expf(-v));
+    if (act == 3) return 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));   // gelu, tanh form
     return v;
 }
 

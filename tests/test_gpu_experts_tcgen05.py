@@ -82,3 +82,19 @@ def test_gates_far_below_zero(K, clamped):
     gate, up = w[0, :inter, 3].double(), 2.0
     want = (gate * torch.sigmoid(gate) * (up + 1.0 if clamped else up)).expand(rows, inter)
     assert ((out.cpu().double() - want).abs() <= 2.0 ** -8 * want.abs()).all()           # (a bfloat16 rounding, and 88 log2(e) to 2^-17)
+
+
+@pytest.mark.parametrize("act", [1, 2, 3])
+@pytest.mark.parametrize("n,k", [(136, 72), (520, 320)])
+def test_activations(K, act, n, k):
+    """Each that experts may have (parts/experts.py: EXPERT_ACTIVATIONS), as the kernels for fewer rows apply it."""
+    rows, starts, _, x, w = case(COUNTS, n, k, False)
+    out, want = torch.full((rows, n), 7.0, dtype=torch.bfloat16, device=DEV), torch.empty(rows, n, dtype=torch.bfloat16)
+    K.expert_linear(out, x.to(DEV), None, w.to(DEV), starts.to(DEV), act)
+    REF.expert_linear(want, x, None, w, starts, act)
+    close(out, want, torch.bfloat16, scale=4.0)
+    K.expert_products = "mma"
+    other = torch.empty_like(out)
+    K.expert_linear(other, x.to(DEV), None, w.to(DEV), starts.to(DEV), act)
+    K.expert_products = "tcgen05"
+    close(out, other.cpu(), torch.bfloat16, scale=4.0)
