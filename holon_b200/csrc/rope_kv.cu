@@ -207,9 +207,9 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kv_write_d128_kernel(
 #pragma unroll
         for (int i = 0; i < 8; ++i) b[i] += add[i];
     }
-    if (dst && !rotate) {                             // values: copied as they are (to 32-bit and back is exact)
-        *(uint4*)(dst + sub * 8) = pack8(a);
-        *(uint4*)(dst + HALF + sub * 8) = pack8(b);
+    if (dst && !rotate) {                             // values: copied as they are, bit for bit
+        *(uint4*)(dst + sub * 8) = bias ? pack8(a) : ra;
+        *(uint4*)(dst + HALF + sub * 8) = bias ? pack8(b) : rb;
     }
     float ss = 0.f;
 #pragma unroll

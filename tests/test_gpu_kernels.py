@@ -245,6 +245,35 @@ def test_qk_norm_rope_kv_write(K, dtype, heads, kv_heads, head_dim, rotary, page
     assert torch.equal(qg2, qg)
 
 
+@pytest.mark.parametrize("rotary", [0, 128])
+@pytest.mark.parametrize("gains", [None, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("biased", [False, True])
+@pytest.mark.parametrize("t,heads,kv_heads", [(1, 1, 1), (11, 5, 3), (300, 4, 1)])
+def test_qk_norm_rope_kv_write_of_bfloat16_heads_of_128(K, rotary, gains, biased, t, heads, kv_heads):
+    """With and without a turn, a norm (its gains in either dtype) and biases; the last block's units partly empty; tokens that are not stored."""
+    page, pages, dt, width = 16, 24, torch.bfloat16, (heads + 2 * kv_heads) * 128
+    qkv, bias = rand(t, width, dtype=dt, seed=5), rand(width, dtype=dt, seed=2, scale=0.5) if biased else None
+    positions = (torch.arange(t) * 7 % 310).to(torch.int32)                             # (some behind the table's end)
+    ang = torch.arange(300, dtype=torch.float32)[:, None] * (1.0 / (1e4 ** (torch.arange(0, 128, 2, dtype=torch.float32) / 128)))[None]
+    table = torch.cat((ang.cos(), ang.sin()), -1).contiguous() if rotary else None
+    qw, kw = ((1 + rand(128, seed=s) * 0.1).to(gains) for s in (6, 7)) if gains else (None, None)
+    write = torch.randperm(pages * page, generator=torch.Generator().manual_seed(8))[:t].to(torch.int32)
+    write[2::5] = -1
+    qkv.view(torch.int16)[0, -3] = 0x7fc1                                                # a NaN among the values keeps its bits
+    kv = rand(pages, 2, kv_heads, page, 128, dtype=dt, seed=9)
+    g = lambda x: x.to(DEV) if x is not None else None                                   # noqa: E731
+    kvg, q, qg = kv.clone().to(DEV), torch.empty(t, heads, 128, dtype=dt), torch.full((t, heads, 128), 7.0, dtype=dt, device=DEV)
+    K.qk_norm_rope_kv_write(qg, qkv.to(DEV), positions.to(DEV), g(table), rotary, g(qw), g(kw), 1e-6, 0.0, kvg, write.to(DEV), heads, kv_heads, 128,
+                            bias=g(bias))
+    REF.qk_norm_rope_kv_write(q, qkv, positions.clamp(max=299), table, rotary, qw, kw, 1e-6, 0.0, kv, write, heads, kv_heads, 128, bias=bias)
+    close(qg, q, dt, scale=4.0)
+    close(kvg.nan_to_num(50.0), kv.nan_to_num(50.0), dt, scale=4.0)
+    assert biased or torch.equal(kvg.cpu()[:, 1].view(torch.int16), kv[:, 1].view(torch.int16))
+    read = torch.full((t, heads, 128), 7.0, dtype=dt, device=DEV)                        # a run that only reads the cache
+    K.qk_norm_rope_kv_write(read, qkv.to(DEV), positions.to(DEV), g(table), rotary, g(qw), g(kw), 1e-6, 0.0, None, None, heads, kv_heads, 128, bias=g(bias))
+    assert torch.equal(read, qg)
+
+
 def paged_case(heads, kv_heads, head_dim, page, rows_spec, dtype, seed=0, window=0):
     """rows_spec: (tokens held before the step, new tokens) per row. Pages are handed out in a shuffled order."""
     g = torch.Generator().manual_seed(seed)
