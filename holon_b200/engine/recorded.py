@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import dataclasses
 import operator
+import types
 import weakref
 from itertools import chain
 
@@ -28,6 +29,11 @@ class _NotUnderstood(Exception):
 
 def _dead() -> None:
     return None
+
+
+def _own_method(v, name: str, x) -> bool:
+    """Whether `x` is nothing but the method `name` that `v` has from its class (who watches a method and puts it back may leave it on the object)."""
+    return isinstance(x, types.MethodType) and x.__self__ is v and x.__func__ is getattr(type(v), name, None)
 
 
 class Reads:
@@ -112,10 +118,11 @@ class Reads:
             for name, x in vars(v).items():
                 if isinstance(v, Part) and name in ("_params", "_children"):
                     continue                         # (what a step reads of them it reads by their own names)
-                self._look(x)
+                if not _own_method(v, name, x):
+                    self._look(x)
             return
         # A kernel table: what it holds decides which kernels it launches, except its counters; nothing in it is walked into
-        if any(callable(getattr(type(v), name, None)) for name in vars(v)):
+        if any(callable(getattr(type(v), name, None)) and not _own_method(v, name, x) for name, x in vars(v).items()):
             raise _NotUnderstood
         names = tuple(name for name in vars(v) if name not in counters)
         self.tables.append((vars(v), names, len(vars(v)), tuple(vars(v)[name] for name in names)))

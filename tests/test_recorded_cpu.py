@@ -152,6 +152,18 @@ def test_a_method_set_on_a_class(monkeypatch):
     assert same(built, reads)
 
 
+def test_a_method_that_was_watched_and_put_back():
+    built, reads = made()
+    k, head = built.ctx.kernels, built.model.head
+    own = k.linear, head.forward
+    k.linear, head.forward = (lambda *a: own[0](*a)), (lambda x: own[1](x))
+    assert not same(built, reads) and Reads.of(*built.runner._read()) is None
+    k.linear, head.forward = own
+    assert not same(built, reads) and Reads.of(*built.runner._read()) is not None
+    k.linear = head.forward                               # (somebody else's)
+    assert Reads.of(*built.runner._read()) is None
+
+
 def test_what_is_not_understood_is_not_recorded():
     built, _ = made()
 
