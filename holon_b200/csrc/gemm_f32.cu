@@ -1,26 +1,28 @@
-// out[m, n] = sum_k x[m, k] * w[n, k] in 32-bit on tcgen05 tensor cores: every operand is split exactly into three bfloat16 numbers.
+// out[m, n] = sum_k x[m, k] * w[n, k] in 32-bit on tcgen05 tensor cores: every operand is split into three bfloat16 numbers.
 //
-// x = x1 + x2 + x3, each the nearest bfloat16 to what the ones before leave (8 + 8 + 8 bits: nothing is left), so
+// x = x1 + x2 + x3, each the nearest bfloat16 to what the ones before leave (8 + 8 + 8 bits: nothing is left of numbers from 2^-103 on), so
 // x w = x1 w1 + (x1 w2 + x2 w1) + (x1 w3 + x2 w2 + x3 w1) up to 2^-26 of |x w|. The six products of 64 columns of k are
 // accumulated by tensor cores in 32 bits, the smallest first, and that sum is added to the running one in a register with one
-// rounding: tensor cores cut sums off instead of rounding them, which 64 columns keep below a rounding error of the running sum.
+// rounding. Tensor cores cut sums off instead of rounding them, by up to 2^-23 of a step's sum; steps are short so that this does not grow with
+// k (up to 512 of k a segment is one step, and it is the whole error).
 // Relative error against 64 bits (2-norm), with multiply-adds in up to eight segments before and now: 541 rows, 1,024 of k 2.1e-7 and 0.95e-7;
 // 300 rows, 3,072 of k 3.6e-7 and 1.0e-7; operands that are all positive 0.8 to 1.1e-7 and 0.9 to 0.95e-7.
 // One order of summation for every output element, a function of k alone: k is cut into up to eight segments of equal length (a multiple
 // of 64), each summed in ascending order in steps of 64, and the segments' sums are added pairwise: ((s0 + s1) + (s2 + s3)) + ((s4 + s5) +
 // (s6 + s7)). So a row's result does not depend on how many other rows the batch holds, nor on how the work was split.
-// A result that is no finite number (an infinity or a NaN among the operands, whose split is none, or an overflow) is
-// computed again with multiply-adds on the numbers as they are.
+// A result that is no finite number (an infinity or a NaN among the operands, whose split is none, or an overflow), or so small beside
+// its operands that parts below bfloat16's smallest number may be missing from it (GF_TINY), is computed again with multiply-adds on the numbers as they are.
 //
 // A block takes 128 rows of w (the M side of tcgen05.mma) by up to 96 rows of x. Eight warps read 64 columns of k of both, split them and
-// write the planes to shared memory (two stages, 128-byte swizzle); two threads issue the 24 MMAs of a stage each (an MMA takes its thread some 150 cycles whatever its size); eight warps
+// write the planes to shared memory (two stages, 128-byte swizzle); two threads issue the 24 MMAs of a stage each (an MMA keeps its thread for 100 cycles at least, 160 with 96 rows, as far as whole kernels tell); eight warps
 // (four in the form for up to 16 rows) read the sums from tensor memory (two buffers) and add them up in registers. A segment's sum waits in tensor memory
 // for its partner. Where tiles are few, the blocks of a cluster of SPLIT share a tile's segments and add them through
 // distributed shared memory. Many rows are bound by shared memory: 24 MMAs read 168 KB and the planes are written with 84 KB, 2,000 cycles for
 // 128 x 96 x 64; few rows by reading w once.
-// In us, with multiply-adds before and now (1,024 of k if not said): 541 rows, 4,096 columns 113 and 57, 6,144 161 and 76, 1,024 by 3,072 140 and
-// 43; 130 rows, 4,096 columns 54 and 19; 17 rows, 6,144 37 and 17; 8 rows 21 and 14; but 2 rows, 6,144 columns 10.4 and 14.2, 1,024 by 3,072 7.9 and 12.8:
-// up to four rows pay for a form whose sums do not depend on the rows beside them with an MMA's least time, some 100 cycles, 24 times a step.
+// In us, with multiply-adds and now (1,024 of k if not said): 541 rows, 4,096 columns 113 and 58, 6,144 161 and 78, 1,024 by 3,072 140 and 45; 130 rows,
+// 4,096 columns 54 and 19.5; 17 rows, 6,144 37 and 17; 8 rows, 4,096 21 and 11; 2 rows, 151,936 columns 167 and 164; but 2 rows, 6,144 columns 10.4 and 13.8, 1,024 by
+// 3,072 7.9 and 13.1: up to four rows pay for a form whose sums do not depend on the rows beside them with the least time of 24 MMAs a step.
+// Looking for the largest number and holding the outputs against it takes 2 to 5 % of that (541 rows: 55.3, 74.5 and 42.4 us without).
 #include <cooperative_groups.h>
 
 #include "tcgen05.cuh"
@@ -55,21 +57,29 @@ __device__ __forceinline__ void gf_st16(uint32_t taddr, const float (&v)[16]) {
     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
 }
 
-// Two numbers into three bfloat16 pairs.
-__device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+// Two numbers into three bfloat16 pairs (packed subtractions: what a loading warp issues is what bounds a step of many rows).
+__device__ __forceinline__ void split2(uint64_t v, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    const uint64_t minus = pack2(-1.f, -1.f);
+    float a, b;
+    unpack2(v, a, b);
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     p1 = *(const uint32_t*)&h;
-    a -= __uint_as_float(p1 << 16);
-    b -= __uint_as_float(p1 & 0xffff0000u);
+    v = fma2(pack2(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u)), minus, v);
+    unpack2(v, a, b);
     const __nv_bfloat162 l = __floats2bfloat162_rn(a, b);
     p2 = *(const uint32_t*)&l;
-    a -= __uint_as_float(p2 << 16);
-    b -= __uint_as_float(p2 & 0xffff0000u);
+    v = fma2(pack2(__uint_as_float(p2 << 16), __uint_as_float(p2 & 0xffff0000u)), minus, v);
+    unpack2(v, a, b);
     const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
     p3 = *(const uint32_t*)&t;
 }
 
-// An element whose split gave no finite number, on the operands themselves.
+// Outputs below this times k times the largest number of their rows of x and w (or one) may miss bits: parts of numbers below 2^-103, and parts'
+// products, may lie under 2^-126, from where on nothing is taken for granted. That is 2^-125 k of the larger row in all, 2^-24 of such an
+// output. It is 1e-27 for 1,024 of k and ordinary rows; only zeros lie below.
+#define GF_TINY 0x1p-99f
+
+// An element whose parts gave no finite number or may have lost bits, on the operands themselves.
 __device__ __noinline__ float gf_plain(const float* __restrict__ x, const float* __restrict__ w, int k) {
     const int length = segment_length(k);
     float s[GF_SEGMENTS];
@@ -79,6 +89,39 @@ __device__ __noinline__ float gf_plain(const float* __restrict__ x, const float*
         for (int i = q * length; i < min(k, (q + 1) * length); ++i) s[q] = fmaf(x[i], w[i], s[q]);
     }
     return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+
+__device__ __forceinline__ float largest(float a, float b, float c) {   // of three sizes, in one instruction
+    asm("max.abs.f32 %0, %0, %1, %2;" : "+f"(a) : "f"(b), "f"(c));
+    return a;
+}
+__device__ __forceinline__ bool gf_infinite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
+
+// Rows row0 .. row1 - 1 of x by this block's columns of the output, which have been written: what the parts of the operands cannot give is made again. Which
+// elements those are follows from the element, its row of x and its row of w alone (not from the rows beside them, which only
+// decide whether the block looks). `tops` [GF_BM]: room for the largest number of each row of w.
+__device__ __noinline__ void gf_repair(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, int n, int k, long ldx, long ldo,
+                                       int n0, int row0, int row1, float* tops) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, columns = min(GF_BM, n - n0);
+    for (int c = warp; c < columns; c += warps) {
+        float top = 0.f;
+        for (int i = lane; i < k; i += 32) top = fmaxf(top, fabsf(w[(size_t)(n0 + c) * k + i]));
+        top = warp_max(top);
+        if (lane == 0) tops[c] = top;
+    }
+    __syncthreads();
+    for (int r = row0 + warp; r < row1; r += warps) {
+        const float* xr = x + (size_t)r * ldx;
+        float top = 0.f;
+        for (int i = lane; i < k; i += 32) top = fmaxf(top, fabsf(xr[i]));
+        top = warp_max(top);
+        for (int c = lane; c < columns; c += 32) {
+            float* o = out + (size_t)r * ldo + n0 + c;
+            const float v = *o, other = tops[c];
+            const bool small = fabsf(v) < fmaxf(fmaxf(top, other), 1.f) * (GF_TINY * (float)k) && top > 0.f && other > 0.f;
+            if (gf_infinite(v) || small) *o = gf_plain(xr, w + (size_t)(n0 + c) * k, k);
+        }
+    }
 }
 
 // ROWS: the most rows of x a tile. rows_x: this launch's (a multiple of 16). ADDERS: warps that add up, four a half of the columns.
@@ -96,6 +139,8 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
     const uint32_t plane_x = rows_x * GF_BK * 2, stage_bytes = 3 * (GF_PLANE + plane_x);
     __shared__ __align__(8) uint64_t bars[8];
     __shared__ uint32_t s_tmem;
+    __shared__ float s_top;
+    __shared__ float tops[GF_BM];
     const uint32_t full0 = smem_addr(bars), empty0 = full0 + 16, d_full0 = empty0 + 16, d_empty0 = d_full0 + 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     x += (size_t)blockIdx.z * x_batch;                                       // blockIdx.z: which of several products (w [batch, n, k])
@@ -106,6 +151,7 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
     const int chunks = k_end > k_first ? (k_end - k_first + GF_BK - 1) / GF_BK : 0, per_segment = length / GF_BK;
 
     if (threadIdx.x == 0) {
+        s_top = 0.f;
         for (int s = 0; s < 2; ++s) {
             mbar_init(full0 + 8 * s, GF_LOADERS); mbar_init(empty0 + 8 * s, 1);
             mbar_init(d_full0 + 8 * s, 1); mbar_init(d_empty0 + 8 * s, ADDERS);
@@ -120,6 +166,10 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    if constexpr (SPLIT > 1) {                                               // s_top is there
+        __syncwarp();
+        cluster_arrive();
+    }
     float acc[GROUPS][16];                                                   // (the adders' only)
 
     if (warp >= ADDERS && warp < ADDERS + GF_LOADERS) {
@@ -140,6 +190,7 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
             for (int i = 0; i < WP + XP; ++i) v[i] = fetch(i, 0);
         }
         bool ok = true;
+        float top = 0.f;                                                     // the largest number (a NaN is none)
         for (int c = 0; c < chunks && ok; ++c) {
             const int s = c & 1;
             ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ((c >> 1) & 1) ^ 1, 1));
@@ -150,8 +201,10 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
             for (int i = 0; i < WP + XP; ++i) {
                 if (i >= WP && (i - WP) * 16 >= rows_x) continue;
                 uint32_t p[3][2];
-                split2(v[i].x, v[i].y, p[0][0], p[1][0], p[2][0]);
-                split2(v[i].z, v[i].w, p[0][1], p[1][1], p[2][1]);
+                const uint64_t lo = pack2(v[i].x, v[i].y), hi = pack2(v[i].z, v[i].w);
+                split2(lo, p[0][0], p[1][0], p[2][0]);
+                split2(hi, p[0][1], p[1][1], p[2][1]);
+                top = largest(largest(top, v[i].x, v[i].y), v[i].z, v[i].w);
                 const uint32_t at = (i < WP ? stage : stage + 3 * GF_PLANE) + (row + 16 * (i < WP ? i : i - WP)) * 128 + within;
 #pragma unroll
                 for (int q = 0; q < 3; ++q)
@@ -161,6 +214,14 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
             fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(full0 + 8 * s);
+        }
+        const unsigned most = __reduce_max_sync(0xffffffffu, __float_as_uint(top));   // (numbers from 0 on are ordered as their bits)
+        if constexpr (SPLIT > 1) {                                           // in every block of the cluster, once all have set theirs to zero
+            __syncwarp();
+            cluster_wait();
+            if (lane < SPLIT) atomicMax((unsigned*)cg::this_cluster().map_shared_rank(&s_top, lane), most);
+        } else if (lane == 0) {
+            atomicMax((unsigned*)&s_top, most);
         }
     } else if (warp >= GF_LOADERS + ADDERS) {                                // a stage and buffer each
         if (lane == 0) {
@@ -233,9 +294,20 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
                 }
             }
         }
-        const int row = (warp & 3) * 32 + lane;
-        if constexpr (SPLIT == 1) {
-            bool bad = false;
+    }
+    if constexpr (SPLIT > 1) {
+        if (warp < ADDERS || warp >= ADDERS + GF_LOADERS) {
+            __syncwarp();
+            cluster_wait();
+        }
+    }
+    __syncthreads();                                                         // every stage has been read; alone: s_top is whole
+    const float unsafe = GF_TINY * (float)k;
+    bool bad = false;
+    if constexpr (SPLIT == 1) {
+        const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+        const float small = fmaxf(s_top, 1.f) * unsafe;
+        if (warp < ADDERS) {
 #pragma unroll
             for (int g = 0; g < GROUPS; ++g) {
                 const int col = (half + g * (ADDERS / 4)) * 16;
@@ -244,19 +316,12 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
                     const int r = m0 + col + i;
                     if (col >= rows_x || r >= m || n0 + row >= n) continue;
                     out[(size_t)r * ldo + n0 + row] = acc[g][i];
-                    bad |= !(fabsf(acc[g][i]) <= 3.402823466e38f);
+                    bad |= gf_infinite(acc[g][i]) || fabsf(acc[g][i]) < small;
                 }
             }
-            if (bad)
-                for (int col = half * 16; col < rows_x; col += ADDERS * 4)
-                    for (int r = m0 + col; r < min(m, m0 + col + 16); ++r) {
-                        float* o = out + (size_t)r * ldo + n0 + row;
-                        if (!(fabsf(*o) <= 3.402823466e38f)) *o = gf_plain(x + (size_t)r * ldx, w + (size_t)(n0 + row) * k, k);
-                    }
         }
     }
-    if constexpr (SPLIT > 1) {
-        __syncthreads();                                                     // every stage has been read: the sums go over them
+    if constexpr (SPLIT > 1) {                                               // the sums go over the stages
         if (warp < ADDERS) {
             const int half = warp >> 2, row = (warp & 3) * 32 + lane;
 #pragma unroll
@@ -270,6 +335,7 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
         cg::cluster_group cluster = cg::this_cluster();
         __syncwarp();
         cluster.sync();
+        const float small = fmaxf(s_top, 1.f) * unsafe;
         const int quads = rows_x * (GF_BM / 4);                              // this block's share, four columns of the output a thread
         const bool wide = n % 4 == 0 && ldo % 4 == 0 && o_batch % 4 == 0 && (uintptr_t)out % 16 == 0;
         for (int i = rank * (quads / SPLIT) + threadIdx.x; i < (rank + 1) * (quads / SPLIT); i += blockDim.x) {
@@ -285,8 +351,7 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
                     p[s] = make_float4(p[s].x + p[s + d].x, p[s].y + p[s + d].y, p[s].z + p[s + d].z, p[s].w + p[s + d].w);
             float v[4] = {p[0].x, p[0].y, p[0].z, p[0].w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (!(fabsf(v[j]) <= 3.402823466e38f) && n0 + row + j < n) v[j] = gf_plain(x + (size_t)r * ldx, w + (size_t)(n0 + row + j) * k, k);
+            for (int j = 0; j < 4; ++j) bad |= n0 + row + j < n && (gf_infinite(v[j]) || fabsf(v[j]) < small);
             float* o = out + (size_t)r * ldo + n0 + row;
             if (wide) *(float4*)o = make_float4(v[0], v[1], v[2], v[3]);
             else
@@ -296,6 +361,7 @@ gemm_f32_kernel(float* __restrict__ out, const float* __restrict__ x, const floa
         __syncwarp();
         cluster.sync();                                                      // nobody leaves while its sums are being read
     }
+    if (__syncthreads_or(bad)) gf_repair(out, x, w, n, k, ldx, ldo, n0, m0 + rank * (rows_x / SPLIT), min(m, m0 + (rank + 1) * (rows_x / SPLIT)), tops);
     tc_fence_before();
     __syncthreads();
     if (warp == GF_LOADERS + ADDERS) {
