@@ -128,7 +128,7 @@ int hb_attention_tcgen05_status(unsigned int* status);
 
 // out[m, n] = sum_k x[m, k] * w[n, k], all float32, sums in a fixed order that does not depend on m's neighbours.
 int hb_gemm_f32(float* out, const float* x, const float* w, int m, int n, int k, hb_stream stream);
-int hb_gemm_f32_split(int split);                   // tests: so many blocks (1, 2, 4 or 8) share a tile's segments (0: chosen per launch)
+int hb_gemm_f32_split(int split);                   // tests: so many blocks (1, 2, 4 or 8) share a tile's segments (0: chosen per launch) in the calling thread's launches
 int hb_gemm_f32_status(unsigned int* status);       // as hb_gemm_tcgen05_status
 
 // `batch` float32 products at once, one per head: out[t, b, :] = x[t, b, :] · w[b]ᵀ with w [batch, n, k]; row t of

@@ -400,7 +400,7 @@ static int launch_rows(const GfArgs& a, bool vec, int split, cudaStream_t s) {
 #undef HB_SPLIT
 }
 
-static int forced_split = 0;
+static thread_local int forced_split = 0;
 extern "C" int hb_gemm_f32_split(int split) { forced_split = split; return 0; }   // tests: segments shared by so many blocks (0: chosen)
 
 static int launch(const char* what, float* out, const float* x, const float* w, int m, int n, int k, int batch, long ldx,
