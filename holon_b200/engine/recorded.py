@@ -20,7 +20,7 @@ import torch
 
 from ..parts.base import Param, Part
 
-_PLAIN = (type(None), bool, int, float, complex, str, bytes, torch.dtype, torch.device, torch.Size)
+_PLAIN = frozenset((type(None), bool, int, float, complex, str, bytes, torch.dtype, torch.device, torch.Size))
 
 
 class _NotUnderstood(Exception):
@@ -45,7 +45,7 @@ class Reads:
         self.views, self.values, self.params, self.weak, self.tensors, self.pointers = [], [], [], [], [], []
         self.tables: list[tuple] = []                # (vars, names, how many in all, values) of objects with counters
         self.objects, self.types = [], []            # what declares itself, and the classes it was of
-        self.classes: list[type] = []                # these and their bases
+        self.classes: dict[type, None] = {}          # these and their bases
         self._seen: dict[int, object] = {}
 
     @classmethod
@@ -65,6 +65,11 @@ class Reads:
         reads._seen = {}
         return reads
 
+    @staticmethod
+    def declared(part: Part) -> bool:
+        """Whether every part below this one is of a class that says it may be recorded: what can be told without looking further."""
+        return vars(type(part)).get("recordable") is True and all(map(Reads.declared, part._children.values()))
+
     def same(self, *roots) -> bool:
         """Whether these are the roots it was made of and all that they read is as it was."""
         return len(roots) == len(self.roots) and all(map(operator.is_, roots, self.roots)) \
@@ -79,47 +84,44 @@ class Reads:
         return [t.data_ptr() for t in self.tensors] + [p.tensor.data_ptr() for p in self.params if p.tensor is not None]
 
     def _look(self, v) -> None:
-        if isinstance(v, _PLAIN) or id(v) in self._seen:
+        t = type(v)
+        if t in _PLAIN or id(v) in self._seen:
             return
         self._seen[id(v)] = v
-        if type(v) is torch.Tensor:
-            self.tensors.append(v)
-        elif type(v) is Param:
+        if t is tuple:
+            for x in v:
+                self._look(x)
+        elif t is Param:
             if v.tensor is not None and type(v.tensor) is not torch.Tensor:
                 raise _NotUnderstood
             self.params.append(v)
-        elif type(v) is tuple:
-            for x in v:
-                self._look(x)
-        elif type(v) is list:
+        elif t is torch.Tensor:
+            self.tensors.append(v)
+        elif vars(t).get("recordable") is True:
+            self._look_at_object(v)
+        elif t is list:
             self.views.append(v)
             for x in v:
                 self._look(x)
-        elif type(v) is dict:
+        elif t is dict:
             self.views.append(v.values())
             for x in v.values():
                 self._look(x)
-        elif dataclasses.is_dataclass(v) and not isinstance(v, type) and type(v).__dataclass_params__.frozen:
-            pass                                     # (it cannot change; its holder is asked whether it is still the same)
-        elif vars(type(v)).get("recordable") is True:
-            self._look_at_object(v)
-        else:
-            raise _NotUnderstood
+        elif not (dataclasses.is_dataclass(t) and t.__dataclass_params__.frozen):    # (such an object cannot change; its holder is asked
+            raise _NotUnderstood                                                     # whether it is still the same)
 
     def _look_at_object(self, v) -> None:
         self.objects.append(v)
         self.types.append(type(v))
-        for c in type(v).__mro__[:-1]:
-            if c not in self.classes:
-                self.classes.append(c)
+        if type(v) not in self.classes:
+            self.classes.update(dict.fromkeys(type(v).__mro__[:-1]))
         counters = getattr(type(v), "counters", None)
         if counters is None:
-            self.views.append(vars(v).values())
-            for name, x in vars(v).items():
-                if isinstance(v, Part) and name in ("_params", "_children"):
-                    continue                         # (what a step reads of them it reads by their own names)
-                if not _own_method(v, name, x):
-                    self._look(x)
+            held, part = vars(v), isinstance(v, Part)
+            self.views.append(held.values())
+            for name, x in held.items():
+                if type(x) not in _PLAIN and not (part and name in ("_params", "_children")) and not _own_method(v, name, x):
+                    self._look(x)                    # (what a step reads of those two it reads by their own names)
             return
         # A kernel table: what it holds decides which kernels it launches, except its counters; nothing in it is walked into
         if any(callable(getattr(type(v), name, None)) and not _own_method(v, name, x) for name, x in vars(v).items()):

@@ -54,8 +54,8 @@ class Runner:
         tables = sum(s * (group.max_pages + 1) + 8 for group in cache.groups)     # every block-table row changed at once
         self.uploader = Uploader(t * (3 + g) + 16 * s + 64 + tables, self.device)
         self.vocab = model.spec.vocab
-        self._reads = Reads.of(*self._read()) if self._graphs else None
-        self._use_graphs = self._reads is not None                # whether steps may be recorded, as last looked
+        self._reads = None                                        # what recorded steps read (None: not looked at)
+        self._use_graphs = self._graphs and Reads.declared(model) # whether steps may be recorded, as far as known
         self._generation = self._wait = self._backoff = 0
 
     # ------------------------------------------------------------------ host half
@@ -177,22 +177,27 @@ class Runner:
         return (self.model, c.kv_of_entry, c.slot_states, self.uploader.dev, *(g.table_device for g in c.groups))
 
     def _settled(self) -> bool:
-        """Whether a step of this model may be recorded at all. Where something that it reads has been replaced, what was recorded
-        before is of an earlier generation and is not replayed again; whether the model may be recorded as it is now is looked at
-        a step later, and after ever more steps (the look takes about as long as a step) where it may not or where every step finds
-        something else replaced."""
+        """Whether a step of this model may be recorded at all, as far as known. Where something that steps read has been replaced, what was
+        recorded before is of an earlier generation and is not replayed again. What the model reads now is looked at
+        a step later, and after ever more steps where it may not be recorded or where every step finds something else replaced (the
+        look takes as long as a step of few layers)."""
         if self._reads is not None and not self._reads.same(*self._read()):
             self._reads, self._generation = None, self._generation + 1
-            self._wait = self._backoff = min(1023, 2 * self._backoff + 1)
-        if self._reads is None:
-            if self._wait:
-                self._wait -= 1
-            else:
-                self._reads = Reads.of(*self._read())
-                self._use_graphs = self._reads is not None
-                if self._reads is None:
-                    self._wait = self._backoff = min(1023, 2 * self._backoff + 1)
+            self._rest()
+        elif self._wait:
+            self._wait -= 1
+        elif not self._use_graphs:
+            self._look()
         return self._use_graphs
+
+    def _look(self) -> None:
+        self._reads = Reads.of(*self._read())
+        self._use_graphs = self._reads is not None
+        if self._reads is None:
+            self._rest()
+
+    def _rest(self) -> None:
+        self._wait = self._backoff = min(1023, 2 * self._backoff + 1)
 
     def _single(self, entries: Sequence[StepEntry]) -> torch.Tensor:
         """A step of one-token rows whose logits are all wanted. Enqueued kernel by kernel it is bound by the host (28 layers of
@@ -203,16 +208,18 @@ class Runner:
         kernels do for their first launch must not be captured. Both run with the plan that serves every step of the kind, so a
         step's logits do not depend on how it was run."""
         step = self.context(entries, pad_rows=0)
-        if self._reads is None:
-            return self.model.forward(step)
-        key = (self._generation, len(entries), self.model.capture_plan(step, self.ctx.max_positions),
-               torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction)
+        kind = (len(entries), self.model.capture_plan(step, self.ctx.max_positions),
+                torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction)
+        key = (self._generation, *kind)
         found = self._recorded.get(key)
-        if found is None and key in self._seen:
-            del self._seen[key]
-            found = self._record(step)
+        if found is None and kind not in self._seen:
+            self._keep(self._seen, kind, None, self.SEEN)
         elif found is None:
-            self._keep(self._seen, key, None, self.SEEN)
+            if self._reads is None and not self._wait:
+                self._look()
+            if self._reads is not None:
+                del self._seen[kind]
+                found = self._record(step)
         if found is None:
             return self.model.forward(step)
         self._keep(self._recorded, key, found, self.GRAPHS)
